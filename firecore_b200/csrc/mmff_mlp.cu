@@ -7,24 +7,35 @@
 // learned component; the network is this project's addition, checked against
 // the FP64 restatement in oracle/mlp_oracle.py.
 //
-// Network kernel: one CTA of 256 threads per SM, persistent over 128-atom
-// tiles.  Warps w and w + 4 share TMEM lanes 32 (w % 4) .. + 31 (tile rows)
-// and split the columns of every epilogue in halves.  Per tile, all operands stay on chip:
-//   Z1 = X W1^T -> H1 = silu(Z1 + b1)                     (TMEM cols 0..127)
+// Network kernel: one CTA of 512 threads per SM, persistent over 128-atom
+// tiles.  The four warps w, w + 4, w + 8, w + 12 share TMEM lanes 32 (w % 4) ..
+// + 31 (tile rows) and split the columns of every epilogue in quarters.  Per
+// tile, all operands stay on chip:
+//   Z1 = X W1^T -> H1 = silu(Z1 + b1), S1 = silu'(.)      (TMEM cols 0..127)
 //   Z2 = H1 W2^T -> H2 = silu(.), S2 = silu'(.)           (cols 128..255)
 //   Y  = H2 W3^T -> dY = 2 (Y + b3 - T) / B
 //   dW3^T += H2^T dY ; dH2 = dY W3 -> dZ2 = dH2 * S2
-//   dW2 += dZ2^T H1 ; db2 += dZ2^T 1 ; dH1 = dZ2 W2 -> dZ1 = dH1 * silu'(Z1)
+//   dW2 += dZ2^T H1 ; db2 += dZ2^T 1 ; dH1 = dZ2 W2 -> dZ1 = dH1 * S1
 //   dW1 += dZ1^T X  ; db1 += dZ1^T 1
 // Weight gradients accumulate in TMEM columns 256..511 over all tiles of the
 // CTA and are stored once at the end as this CTA's partial sums; a second
 // kernel adds the partials of all CTAs in a fixed order (no atomics).  Shared-memory layout
 // and the descriptor of every product: mmff_umma.h.  Inference runs the first
 // three products only.
+// Bound: not the tensor cores (152.8 kflop per row: 6 us of a 65536-row step at
+// 1.6 PFLOP/s) but the serial chain of a tile, six products with an epilogue
+// over 128 x 128 values between each two; operands and accumulators of one tile
+// fill shared memory and TMEM, so tiles cannot overlap.  Hence short epilogues:
+// 16 warps with 32 columns each, one TMEM load per epilogue, silu' of the first
+// layer kept (S1) instead of recomputed, intrinsics for the sigmoid.  With the
+// reduction below (gradient slices summed over 8 threads each, AdamW in the same
+// launch, no memsets or copies between steps: two launches per step instead of
+// six) 200 steps of 65536 rows with their upload take 14.4 ms, before 28.3 ms.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -101,11 +112,25 @@ __device__ __forceinline__ void tm_ld16(uint32_t taddr, float* v) {
     for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
 }
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float dsilu_f(float z) {
-    const float s = 1.f / (1.f + expf(-z));
-    return s * fmaf(z, 1.f - s, 1.f);
+// 32 of them
+__device__ __forceinline__ void tm_ld32(uint32_t taddr, float* v) {
+    uint32_t r[32];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
 }
+
+// silu(z) = z s and silu'(z) = s (1 + z (1 - s)), s = 1 / (1 + exp(-z)).  The
+// intrinsics' few units in the last place of FP32 vanish in the bf16 rounding
+// that follows (2^-9); with the library's expf and divisions the three
+// epilogues took most of a tile's time.
+__device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.f, 1.f + __expf(-z)); }
 __device__ __forceinline__ uint32_t pack_bf2(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
@@ -164,7 +189,12 @@ struct NetArgs {
     int no_issue;            // wait test only: issue no product and no commit, so the first wait runs out
 };
 
-constexpr int NET_THREADS = 256;
+constexpr int NET_THREADS = 512;
+constexpr int NQ = NET_THREADS / 128;           // column parts of an epilogue
+constexpr int QC = HID / NQ;                    // columns of a part
+static_assert(QC == 32, "one 32-column TMEM load per part");
+constexpr int XV = TILE * K0 * 2 / 16;          // 16-byte words of an input tile
+constexpr int XPT = (XV + NET_THREADS - 1) / NET_THREADS;
 
 template <bool TRAIN>
 __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
@@ -173,7 +203,7 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
     const uint32_t sb = smem_u32(sm);
     const int tid = threadIdx.x, warp = tid >> 5;
     const int r = 32 * (warp & 3) + (tid & 31);   // tile row = TMEM lane of this thread
-    const int half = warp >> 2;                   // which half of the columns
+    const int part = warp >> 2;                   // which part of the columns
     float* sbias = reinterpret_cast<float*>(sm + SM_BIAS);
     const uint32_t bar = sb + SM_MISC;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + SM_MISC + 8);
@@ -199,7 +229,7 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
     tc_after();
     const uint32_t tbase = *tslot;
     const uint32_t trow = tbase + ((uint32_t)(32 * (warp & 3)) << 16);   // this warp's 32 TMEM lanes
-    const int c0 = half * (HID / 2), c1 = c0 + HID / 2;                   // this thread's epilogue columns
+    const int c0 = part * QC;                                             // this thread's epilogue columns
 
     uint32_t phase = 0;
     bool failed = false;
@@ -223,51 +253,73 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
         tc_after();
     };
 
-    float v[16], w[16];
+    // 32 values -> row r, columns c0 .. c0 + 31; and back
+    auto put = [&](int off, const float* x) { st_row16(sm + off, r, c0, HID, x); st_row16(sm + off, r, c0 + 16, HID, x + 16); };
+    auto get = [&](int off, float* x) { ld_row16(sm + off, r, c0, HID, x); ld_row16(sm + off, r, c0 + 16, HID, x + 16); };
+
+    float v[32], w[32];
+    // the next tile's input waits in registers: its buffer is an operand of the
+    // last products of this tile, its global latency passes behind them
+    uint4 xn[XPT];
+    auto fetch = [&](int tile) {
+        const uint4* src = A.X + (size_t)tile * XV;
+#pragma unroll
+        for (int k = 0; k < XPT; k++) if (tid + k * NET_THREADS < XV) xn[k] = src[tid + k * NET_THREADS];
+    };
+    if ((int)blockIdx.x < A.ntile) fetch(blockIdx.x);
     for (int tile = blockIdx.x; tile < A.ntile; tile += gridDim.x) {
         const bool acc = done > 0;
         const int row = tile * TILE + r;
         {
-            const uint4* src = A.X + (size_t)tile * (TILE * K0 * 2 / 16);
             uint4* dst = reinterpret_cast<uint4*>(sm + SM_X);
-            for (int i = tid; i < TILE * K0 * 2 / 16; i += NET_THREADS) dst[i] = src[i];
+#pragma unroll
+            for (int k = 0; k < XPT; k++) if (tid + k * NET_THREADS < XV) dst[tid + k * NET_THREADS] = xn[k];
         }
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (TRAIN && part == 0) t = A.T[row];
+        if (tile + (int)gridDim.x < A.ntile) fetch(tile + gridDim.x);
         sync_for_mma();
         if (tid == 0 && !A.no_issue) issue(sb, tbase, OP_L1, false);
         if (!complete()) { failed = true; break; }
-        for (int c = c0; c < c1; c += 16) {          // H1 = silu(Z1 + b1)
-            tm_ld16(trow + TM_Z1 + c, v);
+        // H1 = silu(Z1 + b1), S1 = silu'(Z1 + b1)
+        tm_ld32(trow + TM_Z1 + c0, v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] = silu_f(v[j] + sbias[c + j]);
-            st_row16(sm + SM_H1, r, c, HID, v);
+        for (int j = 0; j < QC; j++) {
+            const float z = v[j] + sbias[c0 + j], s = sigmoid_f(z);
+            v[j] = z * s;
+            if (TRAIN) w[j] = s * fmaf(z, 1.f - s, 1.f);
         }
+        put(SM_H1, v);
+        if (TRAIN) put(SM_S1, w);
         sync_for_mma();
         if (tid == 0 && !A.no_issue) issue(sb, tbase, OP_L2, false);
         if (!complete()) { failed = true; break; }
-        for (int c = c0; c < c1; c += 16) {          // H2 = silu(Z2 + b2), S2 = silu'(Z2 + b2)
-            tm_ld16(trow + TM_WORK + c, v);
+        // H2 = silu(Z2 + b2), S2 = silu'(Z2 + b2)
+        tm_ld32(trow + TM_WORK + c0, v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) { const float z = v[j] + sbias[HID + c + j]; v[j] = silu_f(z); w[j] = dsilu_f(z); }
-            st_row16(sm + SM_H2, r, c, HID, v);
-            if (TRAIN) st_row16(sm + SM_S2, r, c, HID, w);
+        for (int j = 0; j < QC; j++) {
+            const float z = v[j] + sbias[HID + c0 + j], s = sigmoid_f(z);
+            v[j] = z * s;
+            if (TRAIN) w[j] = s * fmaf(z, 1.f - s, 1.f);
         }
+        put(SM_H2, v);
+        if (TRAIN) put(SM_S2, w);
         sync_for_mma();
         if (tid == 0 && !A.no_issue) issue(sb, tbase, OP_L3, false);
         if (!complete()) { failed = true; break; }
-        if (half == 0) {
+        if (part == 0) {
             tm_ld16(trow + TM_WORK, v);
 #pragma unroll
             for (int j = 0; j < NOP; j++) v[j] += sbias[2 * HID + j];
         }
         if (!TRAIN) {
-            if (half == 0 && row < A.nrows)
+            if (part == 0 && row < A.nrows)
                 A.out[row] = make_float4(v[0] * A.out_scale, v[1] * A.out_scale, v[2] * A.out_scale, 0.f);
             done++;
             sync_for_mma();      // TMEM reads of this tile finish before the next tile's products
             continue;
         }
-        if (half == 0) {   // loss and dY = 2 (y - t) w / B (padding rows have w = 0)
-            const float4 t = A.T[row];
+        if (part == 0) {   // loss and dY = 2 (y - t) w / B (padding rows have w = 0)
             const float d0 = (v[0] - t.x) * t.w, d1 = (v[1] - t.y) * t.w, d2 = (v[2] - t.z) * t.w;
             lsum += d0 * d0 + d1 * d1 + d2 * d2;
             const float s = 2.f * A.inv_batch;
@@ -280,23 +332,21 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
         sync_for_mma();
         if (tid == 0 && !A.no_issue) { issue(sb, tbase, OP_DW3, acc); issue(sb, tbase, OP_DH2, false); }
         if (!complete()) { failed = true; break; }
-        for (int c = c0; c < c1; c += 16) {          // dZ2 = dH2 * S2 (in place of S2)
-            tm_ld16(trow + TM_WORK + c, v);
-            ld_row16(sm + SM_S2, r, c, HID, w);
+        // dZ2 = dH2 * S2 (in place of S2)
+        tm_ld32(trow + TM_WORK + c0, v);
+        get(SM_S2, w);
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] *= w[j];
-            st_row16(sm + SM_S2, r, c, HID, v);
-        }
+        for (int j = 0; j < QC; j++) v[j] *= w[j];
+        put(SM_S2, v);
         sync_for_mma();
         if (tid == 0 && !A.no_issue) { issue(sb, tbase, OP_DW2, acc); issue(sb, tbase, OP_DB2, acc); issue(sb, tbase, OP_DH1, false); }
         if (!complete()) { failed = true; break; }
-        for (int c = c0; c < c1; c += 16) {          // dZ1 = dH1 * silu'(Z1 + b1), into the H2 buffer
-            tm_ld16(trow + TM_WORK + c, v);
-            tm_ld16(trow + TM_Z1 + c, w);
+        // dZ1 = dH1 * S1, into the H2 buffer
+        tm_ld32(trow + TM_WORK + c0, v);
+        get(SM_S1, w);
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] *= bf_round(dsilu_f(w[j] + sbias[c + j]));
-            st_row16(sm + SM_H2, r, c, HID, v);
-        }
+        for (int j = 0; j < QC; j++) v[j] *= w[j];
+        put(SM_H2, v);
         sync_for_mma();
         if (tid == 0 && !A.no_issue) { issue(sb, tbase, OP_DW1, acc); issue(sb, tbase, OP_DB1, acc); }
         if (!complete()) { failed = true; break; }
@@ -307,23 +357,18 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
         // this CTA's gradient sums, plain stores into its own slice (reduced
         // over CTAs by reduce_grad_kernel: no atomics, deterministic order)
         float* g = A.gpart + (size_t)blockIdx.x * P_TOTAL;
-        float* red = reinterpret_cast<float*>(sm + SM_X);      // X tile no longer needed: 8 warps x 4 floats
+        float* red = reinterpret_cast<float*>(sm + SM_X);      // X tile no longer needed: 16 warps x 4 floats
         if (!failed && done > 0) {
             // 16-byte stores (every row start and chunk is 64-byte aligned)
-            for (int c = c0; c < c1; c += 16) {
-                tm_ld16(trow + TM_DW2 + c, v);
-                float4* d = reinterpret_cast<float4*>(g + P_W2 + r * HID + c);
+            auto out16 = [&](int tcol, float* dst) {
+                tm_ld16(trow + tcol, v);
 #pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            }
-            // dW1: 5 chunks of 16 columns, 3 in the first half, 2 in the second
-            for (int c = half ? 48 : 0; c < (half ? K0 : 48); c += 16) {
-                tm_ld16(trow + TM_DW1 + c, v);
-                float4* d = reinterpret_cast<float4*>(g + P_W1 + r * K0 + c);
-#pragma unroll
-                for (int j = 0; j < 4; j++) d[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            }
-            if (half == 0) {
+                for (int j = 0; j < 4; j++)
+                    reinterpret_cast<float4*>(dst)[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            };
+            for (int c = c0; c < c0 + QC; c += 16) out16(TM_DW2 + c, g + P_W2 + r * HID + c);
+            for (int c = 16 * part; c < K0; c += 16 * NQ) out16(TM_DW1 + c, g + P_W1 + r * K0 + c);   // 5 chunks
+            if (part == 0) {
                 tm_ld16(trow + TM_DW3, v);
 #pragma unroll
                 for (int j = 0; j < NOP; j++) g[P_W3 + j * HID + r] = v[j];
@@ -366,22 +411,6 @@ __global__ void __launch_bounds__(NET_THREADS, 1) mlp_kernel(NetArgs A) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TM_COLS) : "memory");
 }
 
-// sum of the per-CTA gradient slices (fixed order) and of the loss partials
-__global__ void reduce_grad_kernel(const float* __restrict__ gpart, const double* __restrict__ lpart, int nblk,
-                                   float* __restrict__ grad, double* __restrict__ loss) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < P_TOTAL) {
-        float acc = 0.f;
-        for (int b = 0; b < nblk; b++) acc += gpart[(size_t)b * P_TOTAL + i];
-        grad[i] = acc;
-    }
-    if (i == 0) {
-        double l = 0.0;
-        for (int b = 0; b < nblk; b++) l += lpart[b];
-        *loss = l;
-    }
-}
-
 // standardise raw features and pack them into bf16 core-matrix tiles
 __global__ void pack_input_kernel(const float* __restrict__ F, int n, int ntile, const float* __restrict__ mean,
                                   const float* __restrict__ istd, uint8_t* __restrict__ X) {
@@ -400,40 +429,81 @@ __global__ void pack_input_kernel(const float* __restrict__ F, int n, int ntile,
         make_uint4(pack_bf2(v[0], v[1]), pack_bf2(v[2], v[3]), pack_bf2(v[4], v[5]), pack_bf2(v[6], v[7]));
 }
 
-// AdamW on the flat FP32 parameters (step t >= 1; t == 0 packs only), then the
-// packed bf16 weight image.  Weight decay on W1, W2, W3, not on the biases.
-__global__ void adamw_pack_kernel(float* __restrict__ prm, const float* __restrict__ g, float* __restrict__ m,
-                                  float* __restrict__ vv, int t, float lr, float b1, float b2, float eps, float wd,
-                                  uint8_t* __restrict__ Wp) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P_TOTAL) return;
-    float p = prm[i];
+// AdamW of parameter i (step t >= 1; t == 0 packs only) on the flat FP32
+// parameters, then its place in the packed bf16 weight image.  Weight decay on
+// W1, W2, W3, not on the biases.
+struct AdamArgs {
+    float *prm, *m, *v;
+    uint8_t* Wp;
+    int t;
+    float lr, b1, b2, eps, wd, c1, c2;       // c1, c2: 1 - b1^t, 1 - b2^t
+};
+__device__ __forceinline__ void adamw_pack(const AdamArgs& a, int i, float gi) {
+    float p = a.prm[i];
     const bool isW = (i < P_B1) || (i >= P_W2 && i < P_B2) || (i >= P_W3 && i < P_B3);
-    if (t > 0) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * vv[i] + (1.f - b2) * gi * gi;
-        m[i] = mi; vv[i] = vi;
-        const float mh = mi / (1.f - powf(b1, (float)t));
-        const float vh = vi / (1.f - powf(b2, (float)t));
-        float upd = mh / (sqrtf(vh) + eps);
-        if (isW) upd += wd * p;
-        p -= lr * upd;
+    if (a.t > 0) {
+        const float mi = a.b1 * a.m[i] + (1.f - a.b1) * gi;
+        const float vi = a.b2 * a.v[i] + (1.f - a.b2) * gi * gi;
+        a.m[i] = mi; a.v[i] = vi;
+        float upd = (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+        if (isW) upd += a.wd * p;
+        p -= a.lr * upd;
         // padding: W1 inputs >= 68, W3 / b3 outputs >= 3 stay zero
         if ((i < P_B1 && (i % K0) >= NFEAT) || (i >= P_W3 && i < P_B3 && (i - P_W3) / HID >= NOUT) ||
             (i >= P_B3 && i - P_B3 >= NOUT))
             p = 0.f;
-        prm[i] = p;
+        a.prm[i] = p;
     }
     const __nv_bfloat16 h = __float2bfloat16_rn(p);
     if (i < P_B1) {
-        *reinterpret_cast<__nv_bfloat16*>(Wp + WP_W1 + cm_off(i / K0, i % K0, K0)) = h;
+        *reinterpret_cast<__nv_bfloat16*>(a.Wp + WP_W1 + cm_off(i / K0, i % K0, K0)) = h;
     } else if (i >= P_W2 && i < P_B2) {
         const int e = i - P_W2;
-        *reinterpret_cast<__nv_bfloat16*>(Wp + WP_W2 + cm_off(e / HID, e % HID, HID)) = h;
+        *reinterpret_cast<__nv_bfloat16*>(a.Wp + WP_W2 + cm_off(e / HID, e % HID, HID)) = h;
     } else if (i >= P_W3 && i < P_B3) {
         const int e = i - P_W3;
-        *reinterpret_cast<__nv_bfloat16*>(Wp + WP_W3 + cm_off(e / HID, e % HID, HID)) = h;
+        *reinterpret_cast<__nv_bfloat16*>(a.Wp + WP_W3 + cm_off(e / HID, e % HID, HID)) = h;
+    }
+}
+__global__ void adamw_pack_kernel(AdamArgs a, const float* __restrict__ g) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < P_TOTAL) adamw_pack(a, i, a.t > 0 ? g[i] : 0.f);
+}
+
+// Sum of the per-CTA gradient slices and of the loss partials (fixed order),
+// and with UPDATE the AdamW step of those parameters.  17 MB of slices for a
+// full grid: a block takes 32 float4 columns and splits the slices over RS
+// threads each, so that some 30 loads per SM partition are in flight instead
+// of one thread's chain of 148.
+constexpr int RS = 8;
+template <bool UPDATE>
+__global__ void __launch_bounds__(32 * RS) reduce_grad_kernel(const float* __restrict__ gpart, const double* __restrict__ lpart,
+                                                              int nblk, float* __restrict__ grad, double* __restrict__ loss,
+                                                              AdamArgs a) {
+    __shared__ float4 part[RS][32];
+    const int col = blockIdx.x * 32 + (threadIdx.x & 31), sl = threadIdx.x >> 5;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (col < P_TOTAL / 4) {
+#pragma unroll 4
+        for (int b = sl; b < nblk; b += RS) {
+            const float4 x = reinterpret_cast<const float4*>(gpart + (size_t)b * P_TOTAL)[col];
+            s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+        }
+    }
+    part[sl][threadIdx.x & 31] = s;
+    __syncthreads();
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (threadIdx.x < 128 && i < P_TOTAL) {
+        float g = 0.f;
+#pragma unroll
+        for (int k = 0; k < RS; k++) g += reinterpret_cast<const float*>(part[k])[threadIdx.x];
+        grad[i] = g;
+        if (UPDATE) adamw_pack(a, i, g);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 128) {
+        double l = 0.0;
+        for (int b = 0; b < nblk; b++) l += lpart[b];
+        *loss = l;
     }
 }
 
@@ -706,21 +776,33 @@ int pack_input(const float* d_feat, int n, int ntile, uint8_t* X, cudaStream_t s
     return 0;
 }
 
-int run_net(bool train, const uint8_t* X, const float4* T, int ntile, int nrows, float inv_batch, float4* out,
-            cudaStream_t st) {
+AdamArgs adam_args(int t, double lr, double wd) {
+    AdamArgs a;
+    a.prm = N.prm.p; a.m = N.m.p; a.v = N.v.p; a.Wp = N.Wp.p;
+    a.t = t; a.lr = (float)lr; a.b1 = 0.9f; a.b2 = 0.999f; a.eps = 1e-8f; a.wd = (float)wd;
+    a.c1 = (float)(1.0 - std::pow((double)a.b1, t)); a.c2 = (float)(1.0 - std::pow((double)a.b2, t));
+    return a;
+}
+
+// the network over packed tiles: inference (T null) into out, or one training
+// pass whose gradient sums go to N.grad and loss to loss; adam (nullable): the
+// AdamW step of the same launch
+int run_net(const uint8_t* X, const float4* T, int ntile, int nrows, float inv_batch, float4* out, double* loss,
+            const AdamArgs* adam, cudaStream_t st) {
     if (set_attr()) return -1;
     const int grid = std::max(1, std::min(ntile, num_sms()));
-    if (train && (N.gpart.ensure((size_t)grid * P_TOTAL) || N.lpart.ensure(grid))) return -1;
+    if (T && (N.gpart.ensure((size_t)grid * P_TOTAL) || N.lpart.ensure(grid))) return -1;
     NetArgs a;
     a.X = reinterpret_cast<const uint4*>(X); a.T = T; a.Wp = reinterpret_cast<const uint4*>(N.Wp.p);
     a.prm = N.prm.p; a.gpart = N.gpart.p; a.lpart = N.lpart.p; a.out = out; a.err = N.err.p;
     a.ntile = ntile; a.nrows = nrows; a.inv_batch = inv_batch; a.out_scale = N.out_scale;
     a.wait_limit = 1ll << 31; a.no_issue = 0;
-    if (train) {
+    if (T) {
         mlp_kernel<true><<<grid, NET_THREADS, SM_ALLOC, st>>>(a);
-        mmff_count_launches(1);
-        reduce_grad_kernel<<<(P_TOTAL + 255) / 256, 256, 0, st>>>(N.gpart.p, N.lpart.p, grid, N.grad.p, N.loss.p);
-        mmff_count_launches(1);
+        const int nb = (P_TOTAL / 4 + 31) / 32;
+        if (adam) reduce_grad_kernel<true><<<nb, 32 * RS, 0, st>>>(N.gpart.p, N.lpart.p, grid, N.grad.p, loss, *adam);
+        else reduce_grad_kernel<false><<<nb, 32 * RS, 0, st>>>(N.gpart.p, N.lpart.p, grid, N.grad.p, loss, AdamArgs());
+        mmff_count_launches(2);
     } else {
         mlp_kernel<false><<<grid, NET_THREADS, SM_ALLOC, st>>>(a);
         mmff_count_launches(1);
@@ -730,8 +812,7 @@ int run_net(bool train, const uint8_t* X, const float4* T, int ntile, int nrows,
 }
 
 int adamw(int t, double lr, double wd, cudaStream_t st) {
-    adamw_pack_kernel<<<(P_TOTAL + 255) / 256, 256, 0, st>>>(N.prm.p, N.grad.p, N.m.p, N.v.p, t, (float)lr, 0.9f,
-                                                             0.999f, 1e-8f, (float)wd, N.Wp.p);
+    adamw_pack_kernel<<<(P_TOTAL + 255) / 256, 256, 0, st>>>(adam_args(t, lr, wd), N.grad.p);
     mmff_count_launches(1);
     MCK(cudaGetLastError());
     return 0;
@@ -833,10 +914,8 @@ int mmff_mlp_grad(int n, const float* feat, const float* target, float* grad_out
     MCK(cudaMemcpyAsync(N.feat.p, feat, (size_t)n * NFEAT * sizeof(float), cudaMemcpyHostToDevice, st));
     MCK(cudaMemcpyAsync(N.outs.p, T.data(), T.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
     if (pack_input(N.feat.p, n, ntile, N.Xs.p, st)) return -1;
-    MCK(cudaMemsetAsync(N.grad.p, 0, P_TOTAL * sizeof(float), st));
-    MCK(cudaMemsetAsync(N.loss.p, 0, sizeof(double), st));
     MCK(cudaMemsetAsync(N.err.p, 0, sizeof(int), st));
-    if (run_net(true, N.Xs.p, N.outs.p, ntile, n, 1.f / n, nullptr, st)) return -1;
+    if (run_net(N.Xs.p, N.outs.p, ntile, n, 1.f / n, nullptr, N.loss.p, nullptr, st)) return -1;
     if (check_err(st, "mmff_mlp_grad")) return -1;
     if (grad_out) MCK(cudaMemcpyAsync(grad_out, N.grad.p, P_TOTAL * sizeof(float), cudaMemcpyDeviceToHost, st));
     if (loss_out) MCK(cudaMemcpyAsync(loss_out, N.loss.p, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -864,7 +943,7 @@ int mmff_mlp_infer(int n, const float* feat, float* out) {
     MCK(cudaMemcpyAsync(N.feat.p, feat, (size_t)n * NFEAT * sizeof(float), cudaMemcpyHostToDevice, st));
     MCK(cudaMemsetAsync(N.err.p, 0, sizeof(int), st));
     if (pack_input(N.feat.p, n, ntile, N.Xs.p, st)) return -1;
-    if (run_net(false, N.Xs.p, nullptr, ntile, n, 0.f, N.outs.p, st)) return -1;
+    if (run_net(N.Xs.p, nullptr, ntile, n, 0.f, N.outs.p, nullptr, nullptr, st)) return -1;
     if (check_err(st, "mmff_mlp_infer")) return -1;
     std::vector<float4> h(n);
     MCK(cudaMemcpyAsync(h.data(), N.outs.p, n * sizeof(float4), cudaMemcpyDeviceToHost, st));
@@ -901,14 +980,11 @@ int mmff_mlp_train(int nsteps, int batch_tiles, double lr, double wd, double* lo
     for (int k = 0; k < nsteps; k++) {
         if (t0 + batch_tiles > N.ntile_data) t0 = 0;
         const int rows = std::min(batch_tiles * TILE, N.ndata - t0 * TILE);
-        MCK(cudaMemsetAsync(N.grad.p, 0, P_TOTAL * sizeof(float), st));
-        MCK(cudaMemsetAsync(N.loss.p, 0, sizeof(double), st));
-        if (run_net(true, N.Xd.p + (size_t)t0 * TILE * K0 * 2, N.Td.p + (size_t)t0 * TILE, batch_tiles, rows,
-                    1.f / rows, nullptr, st))
-            return -1;
         N.t++;
-        if (adamw(N.t, lr, wd, st)) return -1;
-        MCK(cudaMemcpyAsync(N.losses.p + k, N.loss.p, sizeof(double), cudaMemcpyDeviceToDevice, st));
+        const AdamArgs a = adam_args(N.t, lr, wd);
+        if (run_net(N.Xd.p + (size_t)t0 * TILE * K0 * 2, N.Td.p + (size_t)t0 * TILE, batch_tiles, rows, 1.f / rows, nullptr,
+                    N.losses.p + k, &a, st))
+            return -1;
         t0 += batch_tiles;
     }
     if (check_err(st, "mmff_mlp_train")) return -1;
@@ -1026,7 +1102,7 @@ int mmff_mlp_warmstart(int nsteps, double z_top, int* accepted) {
     for (int k = 0; k < nsteps; k++) {
         if (features_device(V, z_top)) return -1;
         if (pack_input(N.feat.p, V.NA, ntile, N.Xs.p, V.stream)) return -1;
-        if (run_net(false, N.Xs.p, nullptr, ntile, V.NA, 0.f, N.outs.p, V.stream)) return -1;
+        if (run_net(N.Xs.p, nullptr, ntile, V.NA, 0.f, N.outs.p, nullptr, nullptr, V.stream)) return -1;
         save_kernel<<<ga, 256, 0, V.stream>>>(V.Y, N.atom_sys.p, V.NA, N.save.p);
         mmff_count_launches(1);
         if (N.projection == 1) {
