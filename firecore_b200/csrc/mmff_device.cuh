@@ -694,6 +694,9 @@ __device__ __forceinline__ float4 grid_atom(const Params& P, float3 u, float4 PL
 }
 
 
+// grid build: nodes per thread of the node-potential kernel (consecutive in x)
+constexpr int kGridNX = 4;
+
 // ---- shared-memory carve-up of one system (byte offsets)
 struct SmemLayout {
     int maxNA, maxNN, maxNV, nwarps, nimg, nwords;
