@@ -79,10 +79,10 @@ struct Params {
     float slv[9];                          // substrate lattice vectors a, b, c
     float sK, sR2damp;                     // -alphaMorse, Rdamp^2
     float sg0[3];                          // grid origin: world = local + gorg + sg0
-    // shifted-image pair lists of the CTA relax kernels (null: none): vstride
-    // 32-bit words per CTA, the first vcap of them list entries
-    uint32_t* vlist;
-    int vstride, vcap;
+    // shifted-image pair lists of the CTA relax kernels (null: none): vcap
+    // list entries per CTA
+    unsigned short* vlist;
+    int vcap;
     float vskin;                           // list skin [A]
 };
 
@@ -167,6 +167,20 @@ __device__ __forceinline__ float3 operator-(float3 a, float3 b) { return make_fl
 __device__ __forceinline__ float3 operator*(float3 a, float f) { return make_float3(a.x * f, a.y * f, a.z * f); }
 __device__ __forceinline__ float dot3(float3 a, float3 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, a.z * b.z)); }
 __device__ __forceinline__ float3 fma3(float3 a, float f, float3 c) { return make_float3(fmaf(a.x, f, c.x), fmaf(a.y, f, c.y), fmaf(a.z, f, c.z)); }
+
+// 1 / sqrt(x) of a positive normal number, without the denormal scaling that
+// rsqrtf() adds (three instructions of ten around the pair loops' roots)
+__device__ __forceinline__ float rsq(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// ... with one Newton step: the last-place error of the approximate root times
+// a bond stiffness of 30 eV/A^2 is most of the force noise near a minimum
+__device__ __forceinline__ float rsq_nr(float x) {
+    const float y = rsq(x), e = fmaf(-x * y, y, 1.f);
+    return fmaf(0.5f * y, e, y);
+}
 
 // image index c (NBFF.h:42 ordering: x fastest, then y, then z) -> shift
 // in lattice units.  Quotients by the small image counts go through a float
@@ -591,17 +605,25 @@ __device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int n
 // grid_slice with a per-atom cache of the 64 channel-combined coefficients
 // PLQ . C of the atom's stencil (PLQ is constant per atom).  An atom whose
 // stencil cell is the cached one reads its 16 numbers of slice a (4 float4,
-// 64 contiguous bytes) instead of gathering 16 float4 of the grid (256 B from
-// four columns); on a cell change the slice is gathered, combined and stored
-// as before.  The arithmetic is the same as grid_slice's, so results are
-// bit-identical.  All 32 lanes of the warp call it (a shuffle inside); the
-// four lanes of an atom are consecutive (lane a = lane & 3); ok = the lane
-// holds a real atom.  The cache of an atom is read and written only by the
-// block that owns its system in this launch; a block barrier separates steps.
-template <int UNROLL = 4>
+// 64 contiguous bytes at cs + 4 a) instead of gathering 16 float4 of the grid
+// (256 B from four columns); on a cell change the slice is gathered, combined
+// and stored as before.  The arithmetic is the same as grid_slice's, so
+// results are bit-identical.  The four cached rows are loaded before the key
+// is compared (latency: the loads do not wait for one another nor for the
+// key), and the key's copy in shared memory (skey) keeps a second dependent
+// global load off the path; gkey is its lasting copy.  All 32 lanes of the
+// warp call it; the four lanes of an atom are consecutive (lane a = lane & 3);
+// ok = the lane holds a real atom.  The cache of an atom is read and written
+// only by the block that owns its system in this launch, each slice always by
+// the same lane position; a block barrier separates steps.
 __device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G, int nx, int ny, int nz, float3 u,
-                                                    float4 PLQ, int a, bool ok, unsigned int* gkey, float4* gcs,
-                                                    int atom) {
+                                                    float4 PLQ, int a, bool ok, unsigned int* skey, unsigned int* gkey,
+                                                    float4* cs_atom) {
+    float4* mine = cs_atom + 4 * a;
+    float4 cs[4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) cs[b] = mine[b];
+    const unsigned old = *skey;
     u = grid_safe(u);
     int ix = (int)u.x, iy = (int)u.y, iz = (int)u.z;
     if (u.x < 0.f) ix--;
@@ -611,38 +633,37 @@ __device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G
     ix = wrap_index(ix - 1, nx);
     iy = wrap_index(iy - 1, ny);
     const unsigned key = ((unsigned)ix * 4096u + (unsigned)iy) * 256u + (unsigned)iz;
-    unsigned old = 0xffffffffu;
-    if (ok && a == 0) old = gkey[atom];
-    old = __shfl_sync(0xffffffffu, old, (threadIdx.x & 31) & ~3);
-    const bool hit = ok && old == key;
-    float4* mine = gcs + (size_t)atom * 16 + 4 * a;
-    int xa = ix + a; if (xa >= nx) xa -= nx;
-    const float4 bz = bs_basis(tz), dz = bs_dbasis(tz);
-    const float4 by = bs_basis(ty), dy = bs_dbasis(ty);
-    float ex = 0.f, ey = 0.f, ez = 0.f;
-#pragma unroll UNROLL
-    for (int b = 0; b < 4; b++) {
-        float4 cs;
-        if (hit) {
-            cs = mine[b];
-        } else {
+    __syncwarp();                        // the atom's four lanes have read the old key
+    if (ok && old != key) {
+        int xa = ix + a; if (xa >= nx) xa -= nx;
+#pragma unroll 1
+        for (int b = 0; b < 4; b++) {
             int yb = iy + b; if (yb >= ny) yb -= ny;
             const float4* col = G + ((size_t)(xa * ny + yb) * nz + (iz - 1));
             const float4 c0 = __ldg(col), c1 = __ldg(col + 1), c2 = __ldg(col + 2), c3 = __ldg(col + 3);
-            cs.x = fmaf(PLQ.x, c0.x, fmaf(PLQ.y, c0.y, PLQ.z * c0.z));
-            cs.y = fmaf(PLQ.x, c1.x, fmaf(PLQ.y, c1.y, PLQ.z * c1.z));
-            cs.z = fmaf(PLQ.x, c2.x, fmaf(PLQ.y, c2.y, PLQ.z * c2.z));
-            cs.w = fmaf(PLQ.x, c3.x, fmaf(PLQ.y, c3.y, PLQ.z * c3.z));
-            if (ok) mine[b] = cs;
+            float4 c;
+            c.x = fmaf(PLQ.x, c0.x, fmaf(PLQ.y, c0.y, PLQ.z * c0.z));
+            c.y = fmaf(PLQ.x, c1.x, fmaf(PLQ.y, c1.y, PLQ.z * c1.z));
+            c.z = fmaf(PLQ.x, c2.x, fmaf(PLQ.y, c2.y, PLQ.z * c2.z));
+            c.w = fmaf(PLQ.x, c3.x, fmaf(PLQ.y, c3.y, PLQ.z * c3.z));
+            mine[b] = c;
         }
-        const float v = fmaf(bz.x, cs.x, fmaf(bz.y, cs.y, fmaf(bz.z, cs.z, bz.w * cs.w)));
-        const float d = fmaf(dz.x, cs.x, fmaf(dz.y, cs.y, fmaf(dz.z, cs.z, dz.w * cs.w)));
+#pragma unroll
+        for (int b = 0; b < 4; b++) cs[b] = mine[b];
+        if (a == 0) { *skey = key; *gkey = key; }
+    }
+    const float4 bz = bs_basis(tz), dz = bs_dbasis(tz);
+    const float4 by = bs_basis(ty), dy = bs_dbasis(ty);
+    float ex = 0.f, ey = 0.f, ez = 0.f;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+        const float v = fmaf(bz.x, cs[b].x, fmaf(bz.y, cs[b].y, fmaf(bz.z, cs[b].z, bz.w * cs[b].w)));
+        const float d = fmaf(dz.x, cs[b].x, fmaf(dz.y, cs[b].y, fmaf(dz.z, cs[b].z, dz.w * cs[b].w)));
         const float byb = comp(by, b), dyb = comp(dy, b);
         ex = fmaf(v, dyb, ex);
         ey = fmaf(d, byb, ey);
         ez = fmaf(v, byb, ez);
     }
-    if (ok && !hit && a == 0) gkey[atom] = key;
     const float4 bx = bs_basis(tx), dx = bs_dbasis(tx);
     const float bxa = comp(bx, a), dxa = comp(dx, a);
     return make_float4(dxa * ez, bxa * ex, bxa * ey, bxa * ez);
@@ -702,9 +723,18 @@ struct SmemLayout {
     int maxNA, maxNN, maxNV, nwarps, nimg, nwords;
     // offsets in bytes
     int pos, vel, fasm, fnb, fgrid, REQ, PLQ, ng, ngC, bk, apar, bL, bK, ksp, kpp, fng, red;
+    int sysc;                           // lattice vectors and grid offset of the system
+    int key;                            // per atom: stencil cell of its GridFF cache
     int cwords, cpref, ccnt, clist;     // per-image candidate lists (cutoff + PBC only)
-    int facc, total;                    // fixed-point force sums of the central image [3 * maxNA] int64
-    int stage;                          // image tiles: per warp the 32 j of the current tile (pos, REQ), or -1
+    int facc, total;                    // fixed-point force sums [3 * maxNA] int64
+    // evaluation kernels only (-1 otherwise): pair forces fnb, and the staged
+    // j of an image tile (per warp 32 positions and parameters)
+    int stage;
+    // relaxation kernels only (-1 otherwise): positions and pair parameters as
+    // seven arrays of maxNA rounded up to whole warps (x, y, z, R0, sqrt E0,
+    // Q, H); with pair lists: the positions they were built at (3 arrays), the
+    // start of each atom's row, the listed pairs' forces, the images' shifts
+    int soa, vp, rst, flist, shf;
 };
 
 // number of shifted (non-central) PBC images of the pair term
@@ -731,19 +761,19 @@ constexpr int kImageTileMinThreads = 128;
 // shifted-image pair lists of the CTA relax kernels: shifted images handled
 // (2-D cells have 8) and the average list entries per atom a slot holds
 constexpr int kListMaxImages = 12;
-constexpr int kListEntriesPerAtom = 48;
+constexpr int kListEntriesPerAtom = 96;
 
-__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, bool compact) {
+__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, bool relax, int lvl) {
     SmemLayout L;
     L.maxNA = maxNA; L.maxNN = maxNN; L.maxNV = maxNA + maxNN; L.nwarps = T / 32;
     L.nimg = nimg; L.nwords = (maxNA + 31) / 32;
     int o = 0;
     auto take = [&](int bytes) { int r = o; o += (bytes + 15) & ~15; return r; };
-    auto opt = [&](int bytes) { return compact ? -1 : take(bytes); };
+    auto opt = [&](int bytes) { return lvl > 0 ? -1 : take(bytes); };
     L.pos = take(16 * L.maxNV);
-    L.vel = take(16 * L.maxNV);
+    L.vel = lvl < 2 ? take(16 * L.maxNV) : -1;
     L.fasm = take(16 * L.maxNV);
-    L.fnb = take(16 * maxNA);
+    L.fnb = relax ? -1 : take(16 * maxNA);
     L.fgrid = take(16 * maxNA);
     L.REQ = take(16 * maxNA);
     L.PLQ = opt(16 * maxNA);
@@ -755,26 +785,52 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
     L.bK = opt(16 * maxNN);
     L.ksp = opt(16 * maxNN);
     L.kpp = opt(16 * maxNN);
-    L.fng = take(16 * 8 * maxNN);
+    const int fng_bytes = 16 * 8 * maxNN;
+    L.fng = take(fng_bytes);
     L.red = take(128 * L.nwarps + 64);     // per warp: 4 doubles (32 B) at 0, bbox 6 floats at 64*nwarps
+    L.sysc = L.red + 96 * L.nwarps;        // the tail of red
+    L.key = relax ? take(4 * maxNA) : -1;
+    // candidate lists: built and used up before the recoil slots are written in
+    // the relaxation kernels, so there they share those slots' memory
+    const int o_keep = o;
+    if (relax) o = L.fng;
     L.cwords = take(4 * nimg * L.nwords);   // candidate bit words per image
     L.cpref = take(4 * nimg * L.nwords);    // exclusive prefix of their popcounts
     L.ccnt = take(4 * nimg);                // candidates per image
     L.clist = take(2 * nimg * maxNA);       // candidate atom indices per image, ascending
+    if (relax) {
+        const int need = o - L.fng;
+        o = o_keep;
+        if (need > fng_bytes) { L.cwords += o - L.fng; L.cpref += o - L.fng; L.ccnt += o - L.fng; L.clist += o - L.fng; take(need); }
+    }
     L.facc = take(8 * 3 * maxNA);
     // image tiles (blocks >= kImageTileMinThreads with candidate lists): the
     // positions and parameters of a tile's 32 candidates j, copied once per
     // tile so that the 32 rotation steps read them directly instead of through
     // the candidate list
-    L.stage = (nimg > 0 && T >= kImageTileMinThreads) ? take(2 * 16 * 32 * L.nwarps) : -1;
+    L.stage = (!relax && nimg > 0 && T >= kImageTileMinThreads) ? take(2 * 16 * 32 * L.nwarps) : -1;
+    L.soa = relax ? take(4 * 7 * 32 * L.nwords) : -1;
+    const bool lists = relax && nimg > 0 && nimg <= kListMaxImages;
+    L.vp = lists ? take(4 * 3 * maxNA) : -1;
+    L.rst = lists ? take(4 * (maxNA + 1)) : -1;
+    L.flist = lists ? take(16 * maxNA) : -1;
+    L.shf = lists ? take(16 * nimg) : -1;
     L.total = o;
     return L;
 }
 
-// nimg: shifted images that get candidate lists (0: none)
-__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg) {
-    const SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, false);
-    return (T >= kCompactMinThreads && L.total > kCompactAbove) ? smem_layout_(maxNA, maxNN, T, nimg, true) : L;
+// nimg: shifted images that get candidate lists (0: none).  Level 0: all in
+// shared memory; 1: topology and node parameters in global memory (above);
+// 2 (relaxation, when level 1 exceeds the CTA's limit): the velocities too,
+// which only the thread that owns a vector reads and writes.
+constexpr int kSmemMax = 227 * 1024;
+__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg, bool relax) {
+    SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, relax, 0);
+    if (T >= kCompactMinThreads && L.total > kCompactAbove) {
+        L = smem_layout_(maxNA, maxNN, T, nimg, relax, 1);
+        if (relax && L.total > kSmemMax) L = smem_layout_(maxNA, maxNN, T, nimg, relax, 2);
+    }
+    return L;
 }
 
 // ---- shared-memory carve-up of one warp-per-system region (byte offsets)

@@ -1,256 +1,31 @@
-// mmff_relax.cu -- system-resident relaxation kernels for sm_100a.
+// mmff_eval.cu -- one force (and energy) evaluation of every system, one CTA
+// per system (systems of more than 64 atoms, or any size with forced launch
+// shapes), and the grid sampler.
 //
-// One CTA owns one system at a time.  The system's whole state (positions,
-// velocities, topology, force-field parameters, recoil slots) is staged in
-// shared memory, and every FIRE step runs inside the CTA:
-//   phase 1  bonded terms (thread per node), non-bonded pairs (S threads per
-//            atom, j-split, warp-shuffle reduction) and the B-spline GridFF
-//            sample (4 lanes per atom, one x-slice of the 4x4x4 stencil each,
-//            float4 gathers that stay resident in L2)
-//   phase 2  recoil assembly (MMFFsp3_loc::assemble_atom), optional force clamp,
-//            FP64 block reduction of (f.v, v.v, f.f) and max|f|^2
-//   phase 3  FIRE_update_params in FP64 (every thread computes the same
-//            scalars), move_atom_FIRE, bounding box for PBC-image culling
-// The persistent variant claims systems from a device work queue (atomic
-// counter): a CTA that finishes a system (converged, failed or out of steps)
-// writes it back and claims the next one, so converged systems retire and
-// their slots refill without a host round trip.
-#include "mmff_device.cuh"
-#include <cfloat>
-
-// blocks of at least this many threads unroll the pair tiles and the GridFF
-// columns; smaller ones (four or eight per SM, instruction-fetch bound) do
-// not: measured +5-7 % at 64 threads, +1.7 % at 128 threads (C2 class of
-// 65-128 atoms), while the 256-thread blocks gain 5 % from unrolling
-#ifndef MMFF_UNROLL_MIN_T
-#define MMFF_UNROLL_MIN_T 256
-#endif
+//   phase 1  bonded terms (thread per node), non-bonded pairs (32 x 32 tiles,
+//            each unordered pair once) and the B-spline GridFF sample (4 lanes
+//            per atom, one x-slice of the 4x4x4 stencil each)
+//   phase 2  recoil assembly (MMFFsp3_loc::assemble_atom)
+#include "mmff_engine.cuh"
 
 namespace mmff {
 
-// warp-level sums / extrema
-__device__ __forceinline__ double wsum(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ float wmax(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ float wmin(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// Image shift for cell index (ix, iy, iz)
-__device__ __forceinline__ float3 image_shift(const float* lv, int ix, int iy, int iz) {
-    return make_float3(lv[0] * ix + lv[3] * iy + lv[6] * iz, lv[1] * ix + lv[4] * iy + lv[7] * iz,
-                       lv[2] * ix + lv[5] * iy + lv[8] * iz);
-}
-
 // ---------------------------------------------------------------------------
 // The per-system engine.  T threads, S threads per atom in the pair sum.
-template <int T, int S, bool ENERGY, bool COUNT = false>
-struct Engine {
-    static_assert(T % 32 == 0 && 32 % S == 0, "bad tile");
-    const Params& P;
-    const Systems& Y;
-    SmemLayout L;
-    char* sm;
-    int tid, lane, warp;
-    // current system
-    int isys, natoms, nnode, nvecs, aoff, noff, voff;
-    float lv[9];
-    float3 gorg;
-    // per-step image culling
-    float bbmin[3], bbmax[3];
-    bool hasH = false;          // any H-bond pseudo-charge in the system (block-uniform)
-    const uint32_t* xrow;       // central-image exclusion rows (ceil(natoms/32) words per atom)
-    int nbw;                    // words per row
-    bool pairbad = false;       // a non-finite pair force reached the fixed-point sums
+template <int T, int S, bool ENERGY>
+struct Engine : CtaSystem<T> {
+    static_assert(32 % S == 0, "bad tile");
+    using B = CtaSystem<T>;
+    using B::P; using B::Y; using B::L; using B::tid; using B::lane; using B::warp;
+    using B::isys; using B::natoms; using B::nnode; using B::nvecs; using B::aoff; using B::noff; using B::voff;
+    using B::lv; using B::hasH; using B::xrow; using B::nbw; using B::pairbad; using B::kFix;
+    using B::ngs; using B::ngc; using B::bks; using B::image_active; using B::build_candidates; using B::fix_add;
+    template <class X> __device__ __forceinline__ X* at(int off) { return B::template at<X>(off); }
     double e13 = 0.0;           // ENERGY: pair energies of the skipped 1-3 pairs (energy split)
-    // pair-images evaluated by this thread (COUNT builds only)
-    unsigned long long npair = 0;
-    // shifted-image pair lists of the current system (relax launches with
-    // P.vlist): entries (i | j << 12 | image << 24) in this CTA's slot of global
-    // scratch, then the positions at the last build.  Their state is
-    // block-uniform and sits in shared memory: [0] usable for this system (no
-    // overflow), [1] built and no atom moved more than half the skin since,
-    // [2] entries.
-    __device__ __forceinline__ uint32_t* vslot() const { return P.vlist + (size_t)blockIdx.x * P.vstride; }
-    __device__ __forceinline__ int* vstate() const {
-        __shared__ int st[3];
-        return st;
-    }
-
-    __device__ Engine(const Params& p, const Systems& y, char* smem, const SmemLayout& l)
-        : P(p), Y(y), L(l), sm(smem) {
-        tid = threadIdx.x; lane = tid & 31; warp = tid >> 5;
-    }
-    template <class X> __device__ __forceinline__ X* at(int off) { return reinterpret_cast<X*>(sm + off); }
-    // per-atom / per-node arrays that a compact layout leaves in global memory
-    static constexpr bool kMayCompact = T >= kCompactMinThreads;
-    __device__ __forceinline__ bool compact() const { return kMayCompact && L.ng < 0; }
-    __device__ __forceinline__ int4 ngs(int a) { return compact() ? __ldg(Y.neighs + aoff + a) : at<int4>(L.ng)[a]; }
-    __device__ __forceinline__ int4 ngc(int a) { return compact() ? __ldg(Y.neighCell + aoff + a) : at<int4>(L.ngC)[a]; }
-    __device__ __forceinline__ int4 bks(int a) { return compact() ? __ldg(Y.bkneighs + aoff + a) : at<int4>(L.bk)[a]; }
-    __device__ __forceinline__ float4 plq(int a) { return compact() ? __ldg(Y.PLQ + aoff + a) : at<float4>(L.PLQ)[a]; }
-    __device__ __forceinline__ float4 npar(int off, const float4* g, int n) {
-        return compact() ? __ldg(g + noff + n) : at<float4>(off)[n];
-    }
     // image tiles for long candidate lists (else ordered rows only)
     static constexpr bool kImgTiles = T >= kImageTileMinThreads;
 
-    __device__ void load(int s) {
-        isys = s;
-        const int4 d = Y.desc[s];
-        aoff = d.x; noff = d.y; voff = d.z; natoms = d.w;
-        nnode = Y.nnode[s];
-        nvecs = natoms + nnode;
-        xrow = Y.xmask + Y.moff[s];
-        nbw = (natoms + 31) >> 5;
-        pairbad = false;
-        if (tid == 0) { int* vs = vstate(); vs[0] = P.vlist != nullptr && natoms <= 4096; vs[1] = 0; vs[2] = 0; }
-#pragma unroll
-        for (int k = 0; k < 9; k++) lv[k] = Y.lvec[9 * s + k];
-        const float4 g = Y.gorg[s];
-        gorg = make_float3(g.x, g.y, g.z);
-        float4* spos = at<float4>(L.pos); float4* svel = at<float4>(L.vel);
-        for (int v = tid; v < nvecs; v += T) { spos[v] = Y.pos[voff + v]; svel[v] = Y.vel[voff + v]; }
-        float4* sREQ = at<float4>(L.REQ);
-        const bool full = !compact();         // else topology stays in global memory
-        int h = 0;
-        for (int a = tid; a < natoms; a += T) {
-            const float4 r = Y.REQ[aoff + a];
-            sREQ[a] = r; h |= (r.w != 0.f);
-            if (full) {
-                at<float4>(L.PLQ)[a] = Y.PLQ[aoff + a];
-                at<int4>(L.ng)[a] = Y.neighs[aoff + a];
-                at<int4>(L.ngC)[a] = Y.neighCell[aoff + a];
-                at<int4>(L.bk)[a] = Y.bkneighs[aoff + a];
-            }
-        }
-        hasH = __syncthreads_or(h) != 0;
-        if (full)
-            for (int n = tid; n < nnode; n += T) {
-                at<float4>(L.apar)[n] = Y.apars[noff + n]; at<float4>(L.bL)[n] = Y.bLs[noff + n];
-                at<float4>(L.bK)[n] = Y.bKs[noff + n]; at<float4>(L.ksp)[n] = Y.Ksp[noff + n];
-                at<float4>(L.kpp)[n] = Y.Kpp[noff + n];
-            }
-    }
-
-    // bounding box of the atoms (all threads end with the same box); needs a barrier inside
-    __device__ void bbox_from_smem() {
-        const float4* spos = at<float4>(L.pos);
-        float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (int a = tid; a < natoms; a += T) {
-            const float4 p = spos[a];
-            mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
-            mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
-        }
-        bbox_reduce(mn, mx);
-    }
-    // reduce per-thread boxes: warp shuffle, warp partials in smem, barrier, redundant final
-    __device__ void bbox_reduce(float* mn, float* mx) {
-        float* red = at<float>(L.red) + 8 * 2 * L.nwarps;   // after the 4 doubles per warp
-#pragma unroll
-        for (int k = 0; k < 3; k++) { mn[k] = wmin(mn[k]); mx[k] = wmax(mx[k]); }
-        if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) { red[6 * warp + k] = mn[k]; red[6 * warp + 3 + k] = mx[k]; }
-        }
-        __syncthreads();
-        float a[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, b[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-        for (int w = 0; w < L.nwarps; w++) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) { a[k] = fminf(a[k], red[6 * w + k]); b[k] = fmaxf(b[k], red[6 * w + 3 + k]); }
-        }
-#pragma unroll
-        for (int k = 0; k < 3; k++) { bbmin[k] = a[k]; bbmax[k] = b[k]; }
-    }
-
-    // is image (ix,iy,iz) within the cutoff of the molecule's own box?
-    __device__ __forceinline__ bool image_active(int ix, int iy, int iz) const { return image_within(ix, iy, iz, P.Rc2); }
-    // ... within sqrt(R2) (the cutoff, or the cutoff plus the list skin)
-    __device__ __forceinline__ bool image_within(int ix, int iy, int iz, float R2) const {
-        if (P.Rc2 <= 0.f) return true;
-        if (ix == 0 && iy == 0 && iz == 0) return true;
-        const float3 sh = image_shift(lv, ix, iy, iz);
-        // gap between [bbmin,bbmax] and [bbmin+sh, bbmax+sh] per axis
-        const float gx = fmaxf(0.f, fabsf(sh.x) - (bbmax[0] - bbmin[0]));
-        const float gy = fmaxf(0.f, fabsf(sh.y) - (bbmax[1] - bbmin[1]));
-        const float gz = fmaxf(0.f, fabsf(sh.z) - (bbmax[2] - bbmin[2]));
-        return gx * gx + gy * gy + gz * gz < R2;
-    }
-
-    // Candidate lists of the shifted images: atom j is a candidate of image
-    // (ix,iy,iz) when its shifted position lies within sqrt(R2) (the cutoff,
-    // or the cutoff plus the list skin) of this system's own bounding box (no
-    // atom i can reach the others).  Lists are
-    // ascending in j (ballot words, per-image prefix sums), so the pair sums
-    // keep a fixed order.  All threads; contains barriers.
-    __device__ void build_candidates(float R2) {
-        const float4* spos = at<float4>(L.pos);
-        uint32_t* words = at<uint32_t>(L.cwords);
-        int* pref = at<int>(L.cpref);
-        int* cnt = at<int>(L.ccnt);
-        unsigned short* list = at<unsigned short>(L.clist);
-        const int npx = P.npbc[0], npy = P.npbc[1], npz = P.npbc[2];
-        const int nw = L.nwords;
-        for (int base = warp * 32; base < natoms; base += T) {
-            const int j = base + lane;
-            const float4 p = (j < natoms) ? spos[j] : make_float4(0, 0, 0, 0);
-            int k = 0;
-            for (int iz = -npz; iz <= npz; iz++)
-                for (int iy = -npy; iy <= npy; iy++)
-                    for (int ix = -npx; ix <= npx; ix++) {
-                        if ((ix | iy | iz) == 0) continue;
-                        bool c = false;
-                        if (j < natoms && image_within(ix, iy, iz, R2)) {
-                            const float3 sh = image_shift(lv, ix, iy, iz);
-                            const float qx = p.x + sh.x, qy = p.y + sh.y, qz = p.z + sh.z;
-                            const float gx = fmaxf(0.f, fmaxf(bbmin[0] - qx, qx - bbmax[0]));
-                            const float gy = fmaxf(0.f, fmaxf(bbmin[1] - qy, qy - bbmax[1]));
-                            const float gz = fmaxf(0.f, fmaxf(bbmin[2] - qz, qz - bbmax[2]));
-                            c = gx * gx + gy * gy + gz * gz < R2;
-                        }
-                        const uint32_t bal = __ballot_sync(0xffffffffu, c);
-                        if (lane == 0) words[k * nw + (base >> 5)] = bal;
-                        k++;
-                    }
-        }
-        __syncthreads();
-        for (int k = warp; k < L.nimg; k += L.nwarps) {
-            int run = 0;
-            for (int w0 = 0; w0 < nw; w0 += 32) {
-                const int w = w0 + lane;
-                const uint32_t m = (w < nw && 32 * w < natoms) ? words[k * nw + w] : 0u;
-                const int c = __popc(m);
-                int incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                if (w < nw) pref[k * nw + w] = run + incl - c;
-                run += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            if (lane == 0) cnt[k] = run;
-        }
-        __syncthreads();
-        for (int j = tid; j < natoms; j += T) {
-            const int w = j >> 5;
-            const uint32_t below = (1u << (j & 31)) - 1u;
-            for (int k = 0; k < L.nimg; k++) {
-                const uint32_t m = words[k * nw + w];
-                if ((m >> (j & 31)) & 1u) list[k * L.maxNA + pref[k * nw + w] + __popc(m & below)] = (unsigned short)j;
-            }
-        }
-        __syncthreads();
-    }
+    __device__ Engine(const Params& p, const Systems& y, char* smem, const SmemLayout& l) : B(p, y, smem, l) {}
 
     // pair sum of one atom (already shifted by the image) over j = sub, sub+S, ...
     // Branch-free: excluded and out-of-range pairs get r^2 = 1e30, where every
@@ -274,7 +49,6 @@ struct Engine {
             float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             const bool ex = (j == e0) | (j == e1) | (j == e2) | (j == e3) | (j == e4);
             const bool ok = !ex && (r2 < Rc2);
-            if (COUNT && ok) npair++;
             r2 = ok ? r2 : 1e30f;
             const float ir = rsqrtf(r2);
             const float ir2 = ir * ir;
@@ -324,7 +98,6 @@ struct Engine {
     // sums reach the per-atom totals through 64-bit fixed-point shared-memory
     // adds (2^-32 eV/A resolution): integer addition is associative, so the
     // totals do not depend on which warp finishes first.
-    static constexpr float kFix = 4294967296.f;
 #ifndef MMFF_TILE_UNROLL_SMALL
 #define MMFF_TILE_UNROLL_SMALL 1
 #endif
@@ -336,20 +109,6 @@ struct Engine {
     // (unrolling by 4 measured -6 % at 64 threads), 4 in the larger blocks
     // (+4.7 %)
     static constexpr int kTileUnroll = T >= MMFF_UNROLL_MIN_T ? MMFF_TILE_UNROLL_LARGE : MMFF_TILE_UNROLL_SMALL;
-    // Each add is clamped to |f| <= 2^20 eV/A, so the 64-bit sums (2^31 units
-    // of range per eV/A) cannot wrap for any system that fits a block; a
-    // non-finite force (atoms on top of each other) would convert to an
-    // arbitrary integer, so it marks the system bad instead (assemble).
-    static constexpr float kFixMax = 1048576.f;
-    __device__ __forceinline__ void fix_add(long long* a, float3 f) {
-        pairbad |= !isfinite(f.x + f.y + f.z);
-        const float x = fminf(fmaxf(f.x, -kFixMax), kFixMax), y = fminf(fmaxf(f.y, -kFixMax), kFixMax);
-        const float z = fminf(fmaxf(f.z, -kFixMax), kFixMax);
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 0), (unsigned long long)__float2ll_rn(x * kFix));
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 1), (unsigned long long)__float2ll_rn(y * kFix));
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 2), (unsigned long long)__float2ll_rn(z * kFix));
-    }
-
     // own atom i of a tile: position and parameters; invalid slots exclude everything
     struct TileAtom { float4 p, R; int i; bool v; };
     __device__ __forceinline__ TileAtom tile_atom(int i, const float4* spos, const float4* sREQ) {
@@ -392,7 +151,6 @@ struct Engine {
             fi.x = fmaf(dx, F, fi.x); fi.y = fmaf(dy, F, fi.y); fi.z = fmaf(dz, F, fi.z);
             rj.x = fmaf(-dx, F, rj.x); rj.y = fmaf(-dy, F, rj.y); rj.z = fmaf(-dz, F, rj.z);
             if (ENERGY) ec += e;
-            if (COUNT && ok) npair += 2;
             const int nxt = (lane + 1) & 31;
             rj.x = __shfl_sync(0xffffffffu, rj.x, nxt);
             rj.y = __shfl_sync(0xffffffffu, rj.y, nxt);
@@ -425,7 +183,6 @@ struct Engine {
             const float F = pair_force<ENERGY, HB>(dx, dy, dz, a.R, Rj, excl, Rc2, kq, rc, CUT, ok, e);
             fi.x = fmaf(dx, F, fi.x); fi.y = fmaf(dy, F, fi.y); fi.z = fmaf(dz, F, fi.z);
             if (ENERGY) ec += e;
-            if (COUNT && ok) npair += 2;
             const int src = (lane - s) & 31;     // the lane whose partner this lane's atom was
             fi.x += __shfl_sync(0xffffffffu, -dx * F, src);
             fi.y += __shfl_sync(0xffffffffu, -dy * F, src);
@@ -511,7 +268,6 @@ struct Engine {
             fi.x = fmaf(dx, F, fi.x); fi.y = fmaf(dy, F, fi.y); fi.z = fmaf(dz, F, fi.z);
             rj.x = fmaf(-dx, F, rj.x); rj.y = fmaf(-dy, F, rj.y); rj.z = fmaf(-dz, F, rj.z);
             if (ENERGY) ec += e;
-            if (COUNT && ok) npair += 2;
             const int nxt = (lane + 1) & 31;
             rj.x = __shfl_sync(0xffffffffu, rj.x, nxt);
             rj.y = __shfl_sync(0xffffffffu, rj.y, nxt);
@@ -520,143 +276,6 @@ struct Engine {
         __syncwarp();                                         // staging slots free for the next tile
         if (vi) fix_add(facc + 3 * i, fi);
         if (j0 + lane < nJ) fix_add(facc + 3 * (int)Jl[j0 + lane], rj);
-    }
-
-    // ---- shifted-image pair lists (Verlet lists with a skin) ------------------
-    // (skin P.vskin, 1 A by default.)
-    // Of the pairs the candidate tiles of the shifted images evaluate, only a
-    // few percent lie inside the cutoff: for a large molecule the candidates
-    // of an image span its whole cross-section.  With lists, the ordered pairs
-    // (i, j + shift of image k) over every shifted image k closer than
-    // Rc + skin are collected once and evaluated every step (both orders of a
-    // pair are listed, so the force on i sums in registers and no reaction
-    // goes through the fixed-point atomics) until some atom has moved more
-    // than skin/2 since the build; then they are rebuilt.  The pairs inside
-    // the cutoff are the tiles' pairs, so forces differ from the tile path
-    // only in summation order.
-
-    // block-wide exclusive scan of one int per thread (total in every thread); tmp: nwarps ints
-    __device__ int block_scan(int x, int& total, int* tmp) {
-        int incl = x;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) tmp[warp] = incl;
-        __syncthreads();
-        int base = 0;
-        total = 0;
-        for (int w = 0; w < L.nwarps; w++) {
-            const int t = tmp[w];
-            if (w < warp) base += t;
-            total += t;
-        }
-        __syncthreads();
-        return base + incl - x;
-    }
-
-    // rebuild this system's lists from the current positions; false
-    // (block-uniform) when they do not fit in the slot.  All threads; barriers.
-    __device__ bool list_build(const float4* spos) {
-        const float Rv = sqrtf(P.Rc2) + P.vskin, Rv2 = Rv * Rv;
-        build_candidates(Rv2);
-        const int* ccnt = at<int>(L.ccnt);
-        const unsigned short* clist = at<unsigned short>(L.clist);
-        uint32_t* ent = vslot();
-        // rows: (shifted image k, candidate i of its mirror), k-major; thread tid takes rows [r0, r1)
-        int R = 0;
-        for (int k = 0; k < L.nimg; k++) R += ccnt[L.nimg - 1 - k];
-        const int r0 = (int)((long long)R * tid / T), r1 = (int)((long long)R * (tid + 1) / T);
-        int* tmp = reinterpret_cast<int*>(at<long long>(L.facc));   // unused until the pair sums start
-        int off = 0, total = 0;
-        for (int pass = 0; pass < 2; pass++) {           // count, then write at the scanned offset
-            int c = 0, k = 0, base = 0;
-            for (int r = r0; r < r1; r++) {
-                while (r >= base + ccnt[L.nimg - 1 - k]) { base += ccnt[L.nimg - 1 - k]; k++; }
-                const int i = clist[(L.nimg - 1 - k) * L.maxNA + (r - base)];
-                const int nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
-                const int ipbc = k < L.nimg / 2 ? k : k + 1;      // image index with the central one
-                const float3 sh = image_shift(lv, ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1],
-                                              ipbc / (nxi * nyi) - P.npbc[2]);
-                const float4 pi = spos[i];
-                const float qx = pi.x - sh.x, qy = pi.y - sh.y, qz = pi.z - sh.z;
-                const unsigned short* Jl = clist + k * L.maxNA;
-                const int nJ = ccnt[k];
-                for (int jj = 0; jj < nJ; jj++) {
-                    const int j = Jl[jj];
-                    const float4 pj = spos[j];
-                    const float dx = pj.x - qx, dy = pj.y - qy, dz = pj.z - qz;
-                    if (!(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < Rv2) || image_excluded(i, j, ipbc)) continue;
-                    if (pass == 1) ent[off + c] = (uint32_t)i | ((uint32_t)j << 12) | ((uint32_t)k << 24);
-                    c++;
-                }
-            }
-            if (pass == 0) {
-                off = block_scan(c, total, tmp);
-                if (total > P.vcap) return false;
-            }
-        }
-        float4* vp = reinterpret_cast<float4*>(ent + P.vcap);
-        for (int a = tid; a < natoms; a += T) vp[a] = spos[a];
-        if (tid == 0) vstate()[2] = total;
-        __syncthreads();
-        return true;
-    }
-
-    // excluded pair of the shifted image ipbc (NBFF::evalLJQs_ng4_PBC_atom,
-    // NBFF.h:590-607): i itself, and the bonded neighbours of i whose cell is this image
-    __device__ __forceinline__ bool image_excluded(int i, int j, int ipbc) {
-        if (j == i) return true;
-        const int4 ng = ngs(i), ngC = ngc(i);
-        return (ngC.x == ipbc && ng.x == j) || (ngC.y == ipbc && ng.y == j) || (ngC.z == ipbc && ng.z == j) ||
-               (ngC.w == ipbc && ng.w == j);
-    }
-
-    // the listed pairs of the shifted images into the fixed-point sums.  Each
-    // thread takes a contiguous run of entries (equal shares): consecutive
-    // entries mostly share atom i and image k, so the force on i adds up in
-    // registers and goes to the fixed-point sums once per run of i, the image
-    // shift is recomputed only when k changes, and the next entry's load
-    // overlaps the current pair.  Every pair is listed in both orders: half
-    // of its energy each time, no reaction.
-    template <bool HB>
-    __device__ void list_pairs(const float4* spos, const float4* sREQ, long long* facc, float& ec) {
-        const float Rc2 = P.Rc2, kq = P.kq_rc2, rc = sqrtf(1.f / kq);
-        const int nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
-        const uint32_t* ent = vslot();
-        const int n = vstate()[2];
-        const int q0 = (int)((long long)n * tid / T), q1 = (int)((long long)n * (tid + 1) / T);
-        if (q0 >= q1) return;
-        int ci = -1, ck = -1;
-        float3 sh = make_float3(0.f, 0.f, 0.f), fi = make_float3(0.f, 0.f, 0.f);
-        float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), Ri = pi;
-        uint32_t wn = __ldcg(ent + q0);
-        for (int q = q0; q < q1; q++) {
-            const uint32_t w = wn;
-            if (q + 1 < q1) wn = __ldcg(ent + q + 1);
-            const int i = (int)(w & 0xFFFu), j = (int)((w >> 12) & 0xFFFu), k = (int)(w >> 24);
-            if (i != ci) {
-                if (ci >= 0) fix_add(facc + 3 * ci, fi);
-                ci = i; fi = make_float3(0.f, 0.f, 0.f);
-                pi = spos[i]; Ri = sREQ[i];
-            }
-            if (k != ck) {
-                ck = k;
-                const int ipbc = k < L.nimg / 2 ? k : k + 1;
-                sh = image_shift(lv, ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1], ipbc / (nxi * nyi) - P.npbc[2]);
-            }
-            const float4 pj = spos[j];
-            const float dx = pj.x + sh.x - pi.x, dy = pj.y + sh.y - pi.y, dz = pj.z + sh.z - pi.z;
-            bool ok;
-            float e = 0.f;
-            const float F = pair_force<ENERGY, HB>(dx, dy, dz, Ri, sREQ[j], false, Rc2, kq, rc, true, ok, e);
-            if (ENERGY) ec += 0.5f * e;
-            if (!ok) continue;
-            if (COUNT) npair++;
-            fi.x = fmaf(dx, F, fi.x); fi.y = fmaf(dy, F, fi.y); fi.z = fmaf(dz, F, fi.z);
-        }
-        fix_add(facc + 3 * ci, fi);
     }
 
     // mirror pair (k, nimg-1-k): tiles (true) or ordered rows of both images.
@@ -752,48 +371,6 @@ struct Engine {
         }
     }
 
-    // GridFF B-spline of every atom, 4 lanes per atom (x-slices), by the
-    // threads t0 = 0 .. nt-1 of the caller (whole warps); zero without a grid
-    __device__ void grid_phase(int t0, int nt, float4* fgr, double& Eg) {
-        const float4* spos = at<float4>(L.pos);
-        if (!(P.flags & F_GRID)) {
-            for (int a = t0; a < natoms; a += nt) fgr[a] = make_float4(0, 0, 0, 0);
-            return;
-        }
-        const int nunits = natoms * 4;
-        const bool cached = Y.gkey != nullptr;      // launch-uniform
-        for (int u0 = 0; u0 < nunits; u0 += nt) {
-            const int u = u0 + t0;
-            const int i = u >> 2, a = u & 3;
-            float4 r = make_float4(0, 0, 0, 0);
-            if (cached) {
-                const bool ok = i < natoms;
-                const int ic = ok ? i : natoms - 1;
-                const float4 p = spos[ic];
-                const float3 uu = make_float3((p.x + gorg.x) * P.ginv[0], (p.y + gorg.y) * P.ginv[1],
-                                              (p.z + gorg.z) * P.ginv[2]);
-                r = grid_slice_cached<(T >= MMFF_UNROLL_MIN_T) ? 4 : 1>(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(ic),
-                                                                       a, ok, Y.gkey, Y.gcs, aoff + ic);
-            } else if (i < natoms) {
-                const float4 p = spos[i];
-                const float3 uu = make_float3((p.x + gorg.x) * P.ginv[0], (p.y + gorg.y) * P.ginv[1],
-                                              (p.z + gorg.z) * P.ginv[2]);
-                r = grid_slice<(T >= MMFF_UNROLL_MIN_T) ? 4 : 1>(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(i), a);
-            }
-#pragma unroll
-            for (int o = 2; o > 0; o >>= 1) {
-                r.x += __shfl_xor_sync(0xffffffffu, r.x, o);
-                r.y += __shfl_xor_sync(0xffffffffu, r.y, o);
-                r.z += __shfl_xor_sync(0xffffffffu, r.z, o);
-                r.w += __shfl_xor_sync(0xffffffffu, r.w, o);
-            }
-            if (i < natoms && a == 0) {
-                fgr[i] = make_float4(r.x * P.gmi[0], r.y * P.gmi[1], r.z * P.gmi[2], 0.f);
-                if (ENERGY) Eg += (double)r.w;
-            }
-        }
-    }
-
     // Threads given to the bonded terms when the GridFF runs beside them on
     // the remaining warps; T = no split.  Cost model in units of one grid
     // round (4 lanes x 16 float4 gathers per atom): one bonded pass (one node
@@ -814,37 +391,16 @@ struct Engine {
     __device__ void forces(double& Eb, double& Enb, double& Eg) {
         const int flags = P.flags;
         const float4* spos = at<float4>(L.pos);
-        float4* fasm = at<float4>(L.fasm);
         float4* fnb = at<float4>(L.fnb);
         float4* fgr = at<float4>(L.fgrid);
         const float4* sREQ = at<float4>(L.REQ);
-        float4* fng = at<float4>(L.fng);
         // Bonded terms and the GridFF stencil are independent: when the nodes
         // fill only part of the block, the other warps sample the grid at the
         // same time (block-uniform choice, see bonded_grid_split)
         const int Tb = bonded_grid_split();
         const bool split = Tb < T;
-        if (split && tid >= Tb) {
-            grid_phase(tid - Tb, T - Tb, fgr, Eg);
-        }
-        // --- bonded (nodes); caps get a zero own-force
-        if (tid < Tb)
-        for (int ia = tid; ia < natoms; ia += Tb) {
-            if (ia >= nnode) { fasm[ia] = make_float4(0, 0, 0, 0); continue; }
-            BondedOut o;
-            eval_atom<ENERGY>(ia, natoms, nnode, flags, P.Fmax2NB, spos, sREQ, ngs(ia), ngc(ia),
-                              npar(L.apar, Y.apars, ia), npar(L.bL, Y.bLs, ia), npar(L.bK, Y.bKs, ia),
-                              npar(L.ksp, Y.Ksp, ia), npar(L.kpp, Y.Kpp, ia), lv, P.npbc[0], P.npbc[1], P.npbc[2],
-                              __ldg(Y.a13 + noff + ia), Cut13(P), o);
-            fasm[ia] = make_float4(o.fa.x, o.fa.y, o.fa.z, 0.f);
-            fasm[natoms + ia] = make_float4(o.fpi.x, o.fpi.y, o.fpi.z, 0.f);
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                fng[ia * 4 + k] = make_float4(o.fbs[k].x, o.fbs[k].y, o.fbs[k].z, 0.f);
-                fng[4 * L.maxNN + ia * 4 + k] = make_float4(o.fps[k].x, o.fps[k].y, o.fps[k].z, 0.f);
-            }
-            if (ENERGY) { Eb += (double)o.E; e13 += (double)o.E13; }
-        }
+        if (split && tid >= Tb) B::template grid_phase<ENERGY, false>(tid - Tb, T - Tb, fgr, Eg);
+        B::template bonded_phase<ENERGY>(Tb, Eb, e13);
         // --- non-bonded pairs: S lanes per atom i, j strided by S
         if (flags & F_NONBONDED) {
             const bool pbc = (flags & F_PBC) != 0;
@@ -857,34 +413,7 @@ struct Engine {
                 for (int iy = -npy; iy <= npy; iy++)
                     for (int ix = -npx; ix <= npx; ix++)
                         if ((ix | iy | iz) != 0) any_shift |= image_active(ix, iy, iz);
-            // pair lists of the shifted images (relax kernels with a scratch slot):
-            // kept while no atom moved more than skin/2 since their build
-            bool vrows = false;
-            int* vs = vstate();
-            if (vs[0] && any_shift && P.Rc2 > 0.f && L.nimg > 0 && L.nimg <= kListMaxImages) {
-                bool need = !vs[1];
-                if (!need) {
-                    const float4* vp = reinterpret_cast<const float4*>(vslot() + P.vcap);
-                    const float lim2 = 0.25f * P.vskin * P.vskin;
-                    int moved = 0;
-                    for (int a = tid; a < natoms; a += T) {
-                        const float4 p = spos[a], q = vp[a];
-                        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-                        moved |= !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= lim2);
-                    }
-                    need = __syncthreads_or(moved) != 0;
-                }
-                if (need) {
-                    if (COUNT && tid == 0) atomicAdd(Y.counters + 3, 1ull);
-                    const bool built = list_build(spos);
-                    __syncthreads();                      // every thread has read the state
-                    if (tid == 0) { vs[0] = built; vs[1] = built; }
-                    __syncthreads();
-                }
-                vrows = vs[0] != 0;
-                if (COUNT && tid == 0 && vrows) atomicAdd(Y.counters + 4, (unsigned long long)vs[2]);
-            }
-            const bool lists = !vrows && L.nimg > 0 && any_shift;
+            const bool lists = L.nimg > 0 && any_shift;
             if (lists) build_candidates(P.Rc2);
             const int central = (npz * nyi + npy) * nxi + npx;
             // central image and (with candidate lists) the shifted images:
@@ -897,11 +426,9 @@ struct Engine {
                 if (hasH) {
                     if (lists) pair_tiles<true, true>(spos, sREQ, pbc, central, facc, ec);
                     else pair_tiles<true, false>(spos, sREQ, pbc, central, facc, ec);
-                    if (vrows) list_pairs<true>(spos, sREQ, facc, ec);
                 } else {
                     if (lists) pair_tiles<false, true>(spos, sREQ, pbc, central, facc, ec);
                     else pair_tiles<false, false>(spos, sREQ, pbc, central, facc, ec);
-                    if (vrows) list_pairs<false>(spos, sREQ, facc, ec);
                 }
                 if (ENERGY) Enb += (double)ec;
             }
@@ -911,7 +438,7 @@ struct Engine {
                                      (float)facc[3 * a + 2] * (1.f / kFix), 0.f);
             // without candidate lists: the other images of the bounding-box test,
             // ordered pairs (i, j + shift), S lanes per atom
-            if (!lists && !vrows && any_shift) {
+            if (!lists && any_shift) {
                 __syncthreads();
                 const int nunits = natoms * S;
                 for (int u0 = 0; u0 < nunits; u0 += T) {
@@ -950,14 +477,14 @@ struct Engine {
             for (int a = tid; a < natoms; a += T) fnb[a] = make_float4(0, 0, 0, 0);
         }
         // --- GridFF B-spline (unless it ran beside the bonded terms)
-        if (!split) grid_phase(tid, T, fgr, Eg);
+        if (!split) B::template grid_phase<ENERGY, false>(tid, T, fgr, Eg);
         // --- direct substrate term (getSurfMorse), one thread per atom
         if (flags & F_SURF) {
             __syncthreads();
             const float4* sR = at<float4>(L.REQ);
             for (int a = tid; a < natoms; a += T) {
                 const float4 p = spos[a];
-                const float4 r = surf_atom(P, make_float3(p.x + gorg.x, p.y + gorg.y, p.z + gorg.z), sR[a]);
+                const float4 r = surf_atom(P, make_float3(p.x + lv[9], p.y + lv[10], p.z + lv[11]), sR[a]);
                 const float4 g = fgr[a];
                 fgr[a] = make_float4(g.x + r.x, g.y + r.y, g.z + r.z, 0.f);
                 if (ENERGY) Eg += (double)r.w;
@@ -966,59 +493,36 @@ struct Engine {
     }
 
     // ------------------------------------------------------------------ phase 2
-    // assemble + clamp; FP64 partial sums of (vf, vv, ff) and max|f|^2 for this thread
-    __device__ void assemble(double& vf, double& vv, double& ff, float& fmax2, bool& bad) {
+    // assembled forces; this thread's max |f|^2
+    __device__ void assemble(float& fmax2) {
         float4* fasm = at<float4>(L.fasm);
         const float4* fnb = at<float4>(L.fnb);
         const float4* fgr = at<float4>(L.fgrid);
         const float4* fng = at<float4>(L.fng);
         const float4* spos = at<float4>(L.pos);
-        const float4* svel = at<float4>(L.vel);
-        const float Fl2 = P.Flim * P.Flim;
         for (int v = tid; v < nvecs; v += T) {
-            float3 f;
-            if (v < natoms) {
-                const float4 a = fasm[v], b = fnb[v], c = fgr[v];
-                f = make_float3(a.x + b.x + c.x, a.y + b.y + c.y, a.z + b.z + c.z);
-                const int4 bk = bks(v);
-                const int bks[4] = {bk.x, bk.y, bk.z, bk.w};
+            const bool pi = v >= natoms;
+            const int ia = pi ? v - natoms : v;
+            float3 f = f3(fasm[v]);
+            if (!pi) {
+                const float4 b = fnb[v], c = fgr[v];
+                f = make_float3(f.x + b.x + c.x, f.y + b.y + c.y, f.z + b.z + c.z);
+            }
+            const int4 bk = bks(ia);
+            const int bks[4] = {bk.x, bk.y, bk.z, bk.w};
+            const float4* slots = pi ? fng + 4 * L.maxNN : fng;
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (bks[k] < 0) break;
-                    f = f + f3(fng[bks[k]]);
-                }
-            } else {
-                const int ia = v - natoms;
-                f = f3(fasm[v]);
-                const int4 bk = bks(ia);
-                const int bks[4] = {bk.x, bk.y, bk.z, bk.w};
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (bks[k] < 0) break;
-                    f = f + f3(fng[4 * L.maxNN + bks[k]]);
-                }
+            for (int k = 0; k < 4; k++) {
+                if (bks[k] < 0) break;
+                f = f + f3(slots[bks[k]]);
+            }
+            if (pi) {
                 const float3 u = f3(spos[v]);
                 f = fma3(u, -dot3(f, u), f);      // Vec3::makeOrthoU
             }
-            if ((P.flags & F_BCONS) && v < natoms) f = bond_constraint_force(Y, isys, v, spos, lv, f);
-            if (P.Flim > 0.f) {
-                const float fr2 = dot3(f, f);
-                if (fr2 > Fl2) f = f * (P.Flim * rsqrtf(fr2));
-            }
-            if ((P.flags & F_CONSTR) && v < natoms) f = constraint_force(Y, aoff + v, f3(spos[v]), f);
-            // a system whose atoms left any sensible range (no force clamp,
-            // bad start) is retired like a non-finite one
-            if (v < natoms) { const float4 p = spos[v]; bad |= !(fabsf(p.x) + fabsf(p.y) + fabsf(p.z) < 1e5f); }
             fasm[v] = make_float4(f.x, f.y, f.z, 0.f);
-            const float4 vv4 = svel[v];
-            vf += (double)vv4.x * f.x + (double)vv4.y * f.y + (double)vv4.z * f.z;
-            vv += (double)vv4.x * vv4.x + (double)vv4.y * vv4.y + (double)vv4.z * vv4.z;
-            const double f2 = (double)f.x * f.x + (double)f.y * f.y + (double)f.z * f.z;
-            ff += f2;
-            fmax2 = fmaxf(fmax2, (float)f2);
-            bad |= !isfinite(f.x + f.y + f.z);
+            fmax2 = fmaxf(fmax2, dot3(f, f));
         }
-        bad |= pairbad;
     }
 
     // block reduction of 3 doubles + one float max (+flag); result in all threads
@@ -1040,213 +544,13 @@ struct Engine {
         }
         bad = nb != 0;
     }
-
-    // ------------------------------------------------------------------ phase 3
-    __device__ void move(double dt, double cv, double cfm, float* mn, float* mx) {
-        float4* spos = at<float4>(L.pos);
-        float4* svel = at<float4>(L.vel);
-        const float4* fasm = at<float4>(L.fasm);
-        const float dtf = (float)dt;
-        const float cvf = (float)cv;
-        const float kf = (float)((double)dtf + cfm);
-        for (int v = tid; v < nvecs; v += T) {
-            float3 f = f3(fasm[v]), ve = f3(svel[v]), p = f3(spos[v]);
-            const bool bPi = v >= natoms;
-            if (bPi) f = fma3(p, -dot3(p, f), f);
-            ve = ve * cvf;
-            ve = fma3(f, kf, ve);
-            if (bPi) ve = fma3(p, -dot3(p, ve), ve);
-            p = fma3(ve, dtf, p);
-            if (bPi) p = p * rsqrtf(dot3(p, p));
-            spos[v] = make_float4(p.x, p.y, p.z, 0.f);
-            svel[v] = make_float4(ve.x, ve.y, ve.z, 0.f);
-            if (!bPi) {
-                mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
-                mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
-            }
-        }
-    }
-
-    // Langevin step (MMFFsp3_loc::move_atom_Langevin, MMFFsp3_loc.h:1191-1216):
-    // f - gamma v + uniform(-1,1) * sqrt(2 kB T gamma / dt), then v += f dt,
-    // p += v dt; pi vectors keep unit length and stay orthogonal to their force
-    __device__ void move_md(int step, float* mn, float* mx) {
-        float4* spos = at<float4>(L.pos);
-        float4* svel = at<float4>(L.vel);
-        const float4* fasm = at<float4>(L.fasm);
-        const float dt = P.md_dt, g = P.md_gamma, nz = P.md_noise;
-        for (int v = tid; v < nvecs; v += T) {
-            float3 f = f3(fasm[v]), ve = f3(svel[v]), p = f3(spos[v]);
-            const bool bPi = v >= natoms;
-            if (bPi) f = fma3(p, -dot3(p, f), f);
-            f = fma3(ve, -g, f);
-            const long long gv = (long long)voff + v;
-            f.x = fmaf(langevin_rand(P.md_seed, gv, step, 0), nz, f.x);
-            f.y = fmaf(langevin_rand(P.md_seed, gv, step, 1), nz, f.y);
-            f.z = fmaf(langevin_rand(P.md_seed, gv, step, 2), nz, f.z);
-            ve = fma3(f, dt, ve);
-            if (bPi) ve = fma3(p, -dot3(p, ve), ve);
-            p = fma3(ve, dt, p);
-            if (bPi) p = p * rsqrtf(dot3(p, p));
-            spos[v] = make_float4(p.x, p.y, p.z, 0.f);
-            svel[v] = make_float4(ve.x, ve.y, ve.z, 0.f);
-            if (!bPi) {
-                mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
-                mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
-            }
-        }
-    }
-
-    // copy of the positions just moved (each thread its own vectors, as in move)
-    __device__ void snapshot() {
-        const float4* spos = at<float4>(L.pos);
-        for (int v = tid; v < nvecs; v += T) Y.minpos[voff + v] = spos[v];
-    }
-
-    __device__ void store_state(int status, int steps, float fconv, double dt, double damping, int lastNeg, double total) {
-        const float4* spos = at<float4>(L.pos);
-        const float4* svel = at<float4>(L.vel);
-        const float4* fasm = at<float4>(L.fasm);
-        for (int v = tid; v < nvecs; v += T) {
-            Y.pos[voff + v] = spos[v];
-            Y.vel[voff + v] = svel[v];
-            Y.force[voff + v] = fasm[v];
-        }
-        if (tid == 0) {
-            Y.fire[isys] = make_double4(dt, damping, (double)lastNeg, total);
-            Y.status[isys] = status;
-            Y.nsteps[isys] = steps;
-            Y.fconv[isys] = fconv;
-        }
-    }
 };
-
-// ---------------------------------------------------------------------------
-// Persistent relaxation: claims systems from queue[] via counter.
-// resident CTAs per SM the register allocation of the relax kernel targets,
-// per thread count (build options; without a target ptxas caps at 128
-// registers and spills)
-#ifndef MMFF_MINB_T64
-#define MMFF_MINB_T64 8
-#endif
-#ifndef MMFF_MINB_T128
-#define MMFF_MINB_T128 4
-#endif
-#ifndef MMFF_MINB_T256
-#define MMFF_MINB_T256 2
-#endif
-template <int T> constexpr int relax_min_blocks() {
-    return T == 64 ? MMFF_MINB_T64 : T == 128 ? MMFF_MINB_T128 : T == 256 ? MMFF_MINB_T256 : 1;
-}
-
-// P.vlist (null: none): scratch for the shifted-image pair lists, P.vstride
-// 32-bit words per CTA (P.vcap entries, then 4 * maxNA words of positions).
-// EXPL: the exploring cycle (P.md_mode 2) instead of plain FIRE or the drive.
-template <int T, int S, bool COUNT, bool EXPL = false>
-__global__ void __launch_bounds__(T, relax_min_blocks<T>()) relax_kernel(Params P, Systems Y, const int* __restrict__ queue, int nqueue,
-                                                  int* counter, int maxNA, int maxNN) {
-    extern __shared__ __align__(16) char smem[];
-    __shared__ int s_claim;
-    const SmemLayout L = smem_layout(maxNA, maxNN, T, P.Rc2 > 0.f ? shifted_images(P.flags, P.npbc) : 0);
-    Engine<T, S, false, COUNT> E(P, Y, smem, L);
-    while (true) {
-        if (threadIdx.x == 0) s_claim = atomicAdd(counter, 1);
-        __syncthreads();
-        const int q = s_claim;
-        if (q >= nqueue) break;
-        const int s = queue[q];
-        E.load(s);
-        const double4 fs = Y.fire[s];
-        double dt = fs.x, damping = fs.y, total = fs.w;
-        int lastNeg = (int)fs.z;
-        __syncthreads();
-        E.bbox_from_smem();
-        int status = ST_MAXSTEPS, itr = 0;
-        float meas = 0.f;
-        int ph = 0;                 // exploring cycle: 2 * (steps in the phase) + exploring
-        if constexpr (EXPL) { const int4 g = Y.gopt[s]; ph = 2 * g.y + (g.x != 0); }
-        for (itr = 0; itr < P.nstep_max; itr++) {
-            bool lang = false;      // an exploring step (Langevin instead of FIRE)
-            if constexpr (EXPL) {
-                const int ev = explore_step(ph, P.n_explore, P.n_relax);
-                lang = ev & 1;
-                if ((ev & 2) && threadIdx.x == 0) Y.gopt[s].w++;
-            }
-            double d0 = 0, d1 = 0, d2 = 0;
-            E.forces(d0, d1, d2);
-            __syncthreads();
-            double vf = 0, vv = 0, ff = 0;
-            float fmax2 = 0.f;
-            bool bad = false;
-            E.assemble(vf, vv, ff, fmax2, bad);
-            E.reduce4(vf, vv, ff, fmax2, bad);
-            if (bad) { status = ST_NAN; break; }
-            if (!EXPL && P.md_mode) {   // Langevin drive: fixed number of steps, no FIRE
-                float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-                E.move_md(P.md_step0 + itr, mn, mx);
-                total += 1.0;
-                meas = sqrtf(fmax2);
-                E.bbox_reduce(mn, mx);
-                continue;
-            }
-            // DynamicOpt::FIRE_update_params (FP64, identical in every thread); in the
-            // exploring cycle the FIRE scalars evolve in exploring steps too
-            // (MolWorld_sp3.h:2401-2424)
-            const double f_len = sqrt(ff), v_len = sqrt(vv);
-            const double cos_vf = vf / (f_len * v_len + 1e-32);
-            const double renorm_vf = v_len / (f_len + 1e-32);
-            double cv, cf;
-            if (cos_vf < 0.0) { cv = P.cv_kill; cf = 0.0; } else { cv = 1.0 - damping; cf = damping; }
-            cf = renorm_vf * cf;
-            if (cos_vf < 0.0) {
-                dt = fmax(dt * P.fdec, P.dt_min);
-                lastNeg = 0;
-                damping = P.damp_max;
-            } else {
-                if (lastNeg > P.minLastNeg) { dt = fmin(dt * P.finc, P.dt_max); damping = damping * P.falpha; }
-                lastNeg++;
-            }
-            float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-            if (EXPL && lang) E.move_md(P.md_step0 + itr, mn, mx);
-            else E.move(dt, cv, P.fire_variant == 1 ? cf : renorm_vf * cf, mn, mx);
-            total += 1.0;
-            const double m = (P.conv_mode == 0) ? ff : (double)fmax2;
-            meas = (float)sqrt(m);
-            if constexpr (EXPL) {
-                if (!lang && m < P.Fconv2) {
-                    // a minimum (MolWorld_sp3.h:2465-2473): keep it, start exploring
-                    E.snapshot();
-                    if (threadIdx.x == 0) Y.gopt[s].z++;
-                    ph = 1;
-                }
-            } else {
-                if (m < P.Fconv2) { status = ST_CONVERGED; itr++; E.bbox_reduce(mn, mx); break; }
-            }
-            E.bbox_reduce(mn, mx);   // contains the end-of-step barrier
-        }
-        // converged at step itr-1 (reference returns the loop index at break)
-        const int steps = (status == ST_CONVERGED) ? itr - 1 : itr;
-        __syncthreads();
-        E.store_state(status, steps, meas, dt, damping, lastNeg, total);
-        if (EXPL && threadIdx.x == 0) { Y.gopt[s].x = ph & 1; Y.gopt[s].y = ph >> 1; }
-        if (COUNT) {
-            // force evaluations done for this system: itr loop iterations
-            if (threadIdx.x == 0) {
-                atomicAdd(Y.counters + 1, (unsigned long long)itr * (unsigned long long)E.natoms);
-                atomicAdd(Y.counters + 2, (unsigned long long)itr);
-            }
-        }
-        __syncthreads();
-    }
-    if (COUNT) atomicAdd(Y.counters, E.npair);
-}
 
 // One force (and energy) evaluation per system; blockIdx.x indexes queue[].
 template <int T, int S, bool ENERGY>
 __global__ void __launch_bounds__(T) eval_kernel(Params P, Systems Y, const int* __restrict__ queue, int nqueue,
-                                                 int maxNA, int maxNN) {
+                                                 const __grid_constant__ SmemLayout L) {
     extern __shared__ __align__(16) char smem[];
-    const SmemLayout L = smem_layout(maxNA, maxNN, T, P.Rc2 > 0.f ? shifted_images(P.flags, P.npbc) : 0);
     Engine<T, S, ENERGY> E(P, Y, smem, L);
     const int q = blockIdx.x;
     if (q >= nqueue) return;
@@ -1258,10 +562,8 @@ __global__ void __launch_bounds__(T) eval_kernel(Params P, Systems Y, const int*
     E.forces(Eb, Enb, Eg);
     __syncthreads();
     // (the host passes Flim <= 0 here: eval reports unclamped forces)
-    double vf = 0, vv = 0, ff = 0;
     float fmax2 = 0.f;
-    bool bad = false;
-    E.assemble(vf, vv, ff, fmax2, bad);
+    E.assemble(fmax2);
     __syncthreads();
     const float4* fasm = E.template at<float4>(L.fasm);
     for (int v = threadIdx.x; v < E.nvecs; v += T) Y.force[E.voff + v] = fasm[v];
@@ -1325,20 +627,6 @@ __global__ void grid_sample_kernel(Params P, int n, const float4* __restrict__ p
         default: return nullptr;                                                              \
     }
 
-void* relax_fn(int T, int S, bool count) {
-    if (count) { MMFF_TS_SWITCH(T, S, return (void*)relax_kernel<T_, S_, true>) }
-    MMFF_TS_SWITCH(T, S, return (void*)relax_kernel<T_, S_, false>)
-}
-// the exploring cycle runs one pair lane per atom (S = 1) at any block size
-void* relax_explore_fn(int T) {
-    switch (T) {
-        case 64: return (void*)relax_kernel<64, 1, false, true>;
-        case 128: return (void*)relax_kernel<128, 1, false, true>;
-        case 256: return (void*)relax_kernel<256, 1, false, true>;
-        case 512: return (void*)relax_kernel<512, 1, false, true>;
-        default: return nullptr;
-    }
-}
 void* eval_fn(int T, int S, bool energy) {
     if (energy) { MMFF_TS_SWITCH(T, S, return (void*)eval_kernel<T_, S_, true>) }
     MMFF_TS_SWITCH(T, S, return (void*)eval_kernel<T_, S_, false>)

@@ -22,9 +22,7 @@
 #include "mmff_world.h"
 
 namespace mmff {
-// kernels (mmff_relax.cu, mmff_grid.cu)
-template <int T, int S, bool C> __global__ void relax_kernel(Params, Systems, const int*, int, int*, int, int);
-template <int T, int S, bool E> __global__ void eval_kernel(Params, Systems, const int*, int, int, int);
+// kernels (mmff_relax.cu, mmff_eval.cu, mmff_warp.cu, mmff_grid.cu)
 __global__ void grid_sample_kernel(Params, int, const float4*, const float4*, float4*);
 __global__ void grid_potential_kernel(int, int, int, double3, double3, int, const double4*, const double2*,
                                       const double3*, int, const double3*, int, double, int, const double*,
@@ -35,7 +33,7 @@ __global__ void far_contract_kernel(int, int, int, int, const double*, const dou
 __global__ void solve_open_kernel(double*, long, int, int, const double*, const double*);
 __global__ void solve_periodic_kernel(double*, long, int, long, long, long, const double*, const double*, const double*, double, double);
 __global__ void pack_grid_kernel(long, const double*, float4*);
-void* relax_fn(int T, int S, bool count);
+void* relax_fn(int T, bool count);
 void* eval_fn(int T, int S, bool energy);
 void* relax_warp_fn(int apl, bool count);
 void* relax_explore_fn(int T);
@@ -84,10 +82,13 @@ struct Bucket {
     DBuf<int> queue;
     int smem = 0, grid = 0;
     int cls = 0;                   // size class (see size_class)
+    // evaluation: eT threads and S lanes per atom per CTA, or (eapl > 0) a warp per system
+    int eT = 0, eapl = 0, esmem = 0;
+    SmemLayout lay, elay;          // CTA kernels: shared-memory layouts of relaxation and evaluation
     // CTA relax kernels with a cutoff and a 2-D cell: scratch for the shifted-image
-    // pair lists, vstride 32-bit words per resident CTA (0: none)
-    DBuf<uint32_t> vl;
-    int vstride = 0;
+    // pair lists, vcap entries per resident CTA (0: none)
+    DBuf<unsigned short> vl;
+    int vcap = 0;
 };
 
 // autotuned launch configuration of one size class (kind -1: heuristic)
@@ -98,7 +99,7 @@ struct Tune {
 
 struct World {
     bool ready = false;
-    int device = 0;
+    int device = 0, nsm = 148;
     cudaStream_t stream = nullptr;
     std::vector<cudaStream_t> bstreams;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evfork = nullptr;
@@ -182,6 +183,7 @@ int ensure_ready() {
     CK(cudaEventCreate(&W.ev0));
     CK(cudaEventCreate(&W.ev1));
     CK(cudaEventCreateWithFlags(&W.evfork, cudaEventDisableTiming));
+    CK(cudaDeviceGetAttribute(&W.nsm, cudaDevAttrMultiProcessorCount, W.device));
     W.ready = true;
     return 0;
 }
@@ -281,57 +283,74 @@ int set_smem_limit(void* fn, int bytes) {
 // engine (apl atoms per lane), kind 0 = CTA engine with T threads and S lanes
 // per atom in the pair sum.  Fills smem, grid; sets kernel attributes.
 int config_bucket(Bucket& B, int kind, int apl, int T, int S) {
-    int dev_smem = 0, nsm = 0;
+    int dev_smem = 0;
     CK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, W.device));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, W.device));
     B.maxNA = 0; B.maxNN = 0;
     for (int s : B.sys) { B.maxNA = std::max(B.maxNA, W.natoms[s]); B.maxNN = std::max(B.maxNN, W.nnode[s]); }
-    void* fns[2];
+    const int nimg = W.Rcut > 0 ? shifted_images(W.flags, W.npbc) : 0;
+    void* fns[3];
     if (kind == 1) {
         if (B.maxNA > 32 * apl) return fail("warp engine with %d atoms per lane cannot hold %d atoms", apl, B.maxNA);
         B.kind = 1; B.apl = apl; B.T = 128; B.S = 1;
         B.smem = 4 * warp_layout(B.maxNA, B.maxNN).per_warp;
-        fns[0] = relax_warp_fn(B.apl, false); fns[1] = relax_warp_fn(B.apl, true);
+        fns[0] = relax_warp_fn(B.apl, false); fns[1] = relax_warp_fn(B.apl, true); fns[2] = relax_warp_explore_fn(B.apl);
     } else {
         B.kind = 0; B.T = T; B.S = S;
-        B.smem = smem_layout(B.maxNA, B.maxNN, B.T, W.Rcut > 0 ? shifted_images(W.flags, W.npbc) : 0).total;
-        fns[0] = relax_fn(B.T, B.S, false); fns[1] = relax_fn(B.T, B.S, true);
+        B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
+        if (B.lay.total > dev_smem && B.T < kCompactMinThreads) {     // only the larger blocks leave arrays in global memory
+            B.T = kCompactMinThreads;
+            B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
+        }
+        B.smem = B.lay.total;
+        fns[0] = relax_fn(B.T, false); fns[1] = relax_fn(B.T, true); fns[2] = relax_explore_fn(B.T);
     }
-    if (B.smem > dev_smem) return fail("system too large for shared memory: %d B > %d B", B.smem, dev_smem);
-    if (!fns[0] || !fns[1]) return fail("no kernel for bucket (kind %d, T=%d, S=%d)", B.kind, B.T, B.S);
-    for (int f = 0; f < 2; f++) if (set_smem_limit(fns[f], B.smem)) return -1;
-    void* xf = B.kind ? relax_warp_explore_fn(B.apl) : relax_explore_fn(B.T);     // exploring cycle
-    if (!xf) return fail("no exploring-cycle kernel for bucket (kind %d, T=%d)", B.kind, B.T);
-    if (set_smem_limit(xf, B.smem)) return -1;
+    // evaluation: one pass over the system, a warp each up to 64 atoms
+    B.eapl = B.maxNA <= 32 ? 1 : B.maxNA <= 64 ? 2 : 0;
+    if (kind == 0 && W.force_T) B.eapl = 0;
+    B.eT = B.eapl ? 128 : T;
+    if (!B.eapl) B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, false);
+    B.esmem = B.eapl ? 4 * warp_layout(B.maxNA, B.maxNN).per_warp : B.elay.total;
+    if (B.smem > dev_smem || B.esmem > dev_smem)
+        return fail("system too large for shared memory: %d B > %d B", std::max(B.smem, B.esmem), dev_smem);
+    if (!fns[0] || !fns[1] || !fns[2]) return fail("no kernel for bucket (kind %d, T=%d, S=%d)", B.kind, B.T, B.S);
+    for (int f = 0; f < 3; f++) if (set_smem_limit(fns[f], B.smem)) return -1;
     for (int e = 0; e < 2; e++) {
-        void* ef = B.kind ? eval_warp_fn(B.apl, e) : eval_fn(B.T, B.S, e);
-        if (set_smem_limit(ef, B.smem)) return -1;
+        void* ef = B.eapl ? eval_warp_fn(B.eapl, e) : eval_fn(B.eT, B.S, e);
+        if (!ef) return fail("no evaluation kernel for bucket (T=%d, S=%d)", B.eT, B.S);
+        if (set_smem_limit(ef, B.esmem)) return -1;
     }
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[0], B.T, B.smem));
     if (occ < 1) return fail("kernel cannot be resident (T=%d smem=%d)", B.T, B.smem);
     const int per_block = B.kind ? 4 : 1;
     const int nblk = ((int)B.sys.size() + per_block - 1) / per_block;
-    B.grid = std::min(nblk, occ * nsm);
-    B.vstride = 0;
-    if (kind == 0 && W.Rcut > 0 && B.maxNA <= 4096) {
-        const int nimg = shifted_images(W.flags, W.npbc);
-        if (nimg > 0 && nimg <= kListMaxImages) {
-            B.vstride = B.maxNA * (kListEntriesPerAtom + 4);
-            if (B.vl.ensure((size_t)B.grid * B.vstride)) return -1;
-        }
+    B.grid = std::min(nblk, occ * W.nsm);
+    B.vcap = 0;
+    if (kind == 0 && nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
+        B.vcap = B.maxNA * kListEntriesPerAtom;
+        if (B.vl.ensure((size_t)B.grid * B.vcap)) return -1;
     }
     if (B.queue.ensure(B.sys.size())) return -1;
     CK(cudaMemcpy(B.queue.p, B.sys.data(), B.sys.size() * sizeof(int), cudaMemcpyHostToDevice));
     return 0;
 }
 
-// heuristic configuration of a size class: warp engine for <= 64 atoms, else
-// the class's thread count with pair lanes filling the block
-void default_config(int cls, int maxNA, int& kind, int& apl, int& T, int& S) {
-    if (cls <= 1) { kind = 1; apl = cls + 1; T = 128; S = 1; return; }
-    kind = 0; apl = 1; T = kClassT[cls - 2];
-    S = std::min(pow2_floor(std::max(1, T / std::max(1, maxNA))), 8);
+// Launch shape of a size class.  Base: the fewest threads that do not leave
+// lanes idle in the pair rows (32 up to 32 atoms, 64 up to 64, then the class's
+// bound, 256 above that), which is the fastest shape when there are systems
+// enough to fill the chip.  With fewer, the idle warp slots go to more threads
+// per system: about 16 warps per SM over the systems an SM holds, as far as a
+// system of that class still gains from them.
+void default_config(int cls, int maxNA, int nsys, int& kind, int& apl, int& T, int& S) {
+    kind = 0; apl = 1;
+    T = cls == 0 ? 32 : cls == 1 ? 64 : std::min(256, kClassT[cls - 2]);
+    S = cls <= 1 ? 1 : std::min(pow2_floor(std::max(1, kClassT[cls - 2] / std::max(1, maxNA))), 8);
+    if (W.force_T) T = W.force_T;
+    else {
+        const int cap = cls <= 1 ? 128 : cls == 3 ? 256 : 512;
+        const int per_sm = std::max(1, (nsys + W.nsm - 1) / W.nsm);
+        T = std::max(T, std::min(cap, pow2_floor(std::max(1, 512 / per_sm))));
+    }
     if (W.force_S) S = W.force_S;
 }
 
@@ -439,7 +458,7 @@ int build_buckets() {
         int maxNA = 0;
         for (int s : B.sys) maxNA = std::max(maxNA, W.natoms[s]);
         int kind, apl, T, S;
-        default_config(k, maxNA, kind, apl, T, S);
+        default_config(k, maxNA, (int)B.sys.size(), kind, apl, T, S);
         const Tune& tu = W.tune[k];
         if (tu.kind >= 0 && !W.force_T && !W.force_S) { kind = tu.kind; apl = tu.apl; T = tu.T; S = tu.S; }
         if (config_bucket(B, kind, apl, T, S)) return -1;
@@ -474,10 +493,9 @@ PinnedBuf g_stage_a, g_stage_b;
 
 // the bucket's pair-list scratch into the launch parameters (CTA relax kernels)
 void set_lists(Params& P, const Bucket& B) {
-    const bool on = W.pair_lists && B.kind == 0 && B.vstride > 4 * B.maxNA && B.vl.p;
+    const bool on = W.pair_lists && B.kind == 0 && B.vcap > 0 && B.vl.p;
     P.vlist = on ? B.vl.p : nullptr;
-    P.vstride = on ? B.vstride : 0;
-    P.vcap = on ? B.vstride - 4 * B.maxNA : 0;
+    P.vcap = on ? B.vcap : 0;
     P.vskin = (float)W.list_skin;
 }
 
@@ -494,13 +512,13 @@ int enqueue_relax(const Params& P) {
         cudaStream_t st = W.bstreams[b];
         CK(cudaStreamWaitEvent(st, W.evfork, 0));
         void* fn = P.md_mode == 2 ? (B.kind ? relax_warp_explore_fn(B.apl) : relax_explore_fn(B.T))
-                                  : (B.kind ? relax_warp_fn(B.apl, W.count) : relax_fn(B.T, B.S, W.count));
+                                  : (B.kind ? relax_warp_fn(B.apl, W.count) : relax_fn(B.T, W.count));
         const int* q = B.queue.p;
         int nq = (int)B.sys.size();
         int* ctr = W.d_counter.p + b;
         int mna = B.maxNA, mnn = B.maxNN;
         set_lists(Pc, B);
-        void* args[] = {&Pc, &Y, &q, &nq, &ctr, &mna, &mnn};
+        void* args[] = {&Pc, &Y, &q, &nq, &ctr, B.kind ? (void*)&mna : (void*)&B.lay, &mnn};
         CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
         if (!g_capturing) g_launches++;
     }
@@ -1038,13 +1056,13 @@ int mmff_eval(int with_energy) {
     Params P = make_params(true, 0, 0.0, 0);
     Systems Y = make_systems();
     for (auto& B : W.buckets) {
-        void* fn = B.kind ? eval_warp_fn(B.apl, with_energy != 0) : eval_fn(B.T, B.S, with_energy != 0);
+        void* fn = B.eapl ? eval_warp_fn(B.eapl, with_energy != 0) : eval_fn(B.eT, B.S, with_energy != 0);
         const int* q = B.queue.p;
         int nq = (int)B.sys.size();
         int mna = B.maxNA, mnn = B.maxNN;
-        void* args[] = {&P, &Y, &q, &nq, &mna, &mnn};
-        const int nblk = B.kind ? (nq + 3) / 4 : nq;
-        CK(cudaLaunchKernel(fn, dim3(nblk), dim3(B.T), args, B.smem, W.stream));
+        void* args[] = {&P, &Y, &q, &nq, B.eapl ? (void*)&mna : (void*)&B.elay, &mnn};
+        const int nblk = B.eapl ? (nq + 3) / 4 : nq;
+        CK(cudaLaunchKernel(fn, dim3(nblk), dim3(B.eT), args, B.esmem, W.stream));
         g_launches++;
     }
     CK(cudaGetLastError());
@@ -1277,12 +1295,12 @@ int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap
             B.sys = sample;
             float us = -1.f;
             if (config_bucket(B, c.kind, c.apl, c.T, c.S) == 0) {
-                void* fn = B.kind ? relax_warp_fn(B.apl, false) : relax_fn(B.T, B.S, false);
+                void* fn = B.kind ? relax_warp_fn(B.apl, false) : relax_fn(B.T, false);
                 const int* q = B.queue.p;
                 int nq = (int)B.sys.size(), mna = B.maxNA, mnn = B.maxNN;
                 int* ctr = W.d_counter.p + 32;
                 set_lists(P, B);
-                void* args[] = {&P, &Y, &q, &nq, &ctr, &mna, &mnn};
+                void* args[] = {&P, &Y, &q, &nq, &ctr, B.kind ? (void*)&mna : (void*)&B.lay, &mnn};
                 float ms = 0.f;
                 for (int rep = 0; rep < 2; rep++) {        // first launch warms caches and clocks
                     if (copy_state(false)) return -1;
@@ -1328,7 +1346,7 @@ int mmff_get_tuning(int cls, int* out) {
 int mmff_set_tuning(int cls, int kind, int apl, int T, int S) {
     if (cls < 0 || cls > 5) return fail("size class must be 0..5");
     if (kind == 1 && !((cls == 0 && apl == 1) || (cls == 1 && apl == 2))) return fail("warp engine only for classes 0/1 (apl = class + 1)");
-    if (kind == 0 && !relax_fn(T, S, false)) return fail("no CTA kernel with T=%d S=%d", T, S);
+    if (kind == 0 && (!relax_fn(T, false) || !(S == 1 || S == 2 || S == 4 || S == 8))) return fail("no CTA kernel with T=%d S=%d", T, S);
     if (kind != -1 && kind != 0 && kind != 1) return fail("kind must be -1, 0 or 1");
     W.tune[cls].kind = kind; W.tune[cls].apl = apl; W.tune[cls].T = T; W.tune[cls].S = S;
     W.buckets_dirty = true;
