@@ -733,8 +733,9 @@ struct SmemLayout {
     // relaxation kernels only (-1 otherwise): positions and pair parameters as
     // seven arrays of maxNA rounded up to whole warps (x, y, z, R0, sqrt E0,
     // Q, H); with pair lists: the positions they were built at (3 arrays), the
-    // start of each atom's row, the listed pairs' forces, the images' shifts
-    int soa, vp, rst, flist, shf;
+    // start of each atom's row, the listed pairs' forces, the images' shifts,
+    // the atoms by falling row length
+    int soa, vp, rst, flist, shf, perm;
 };
 
 // number of shifted (non-central) PBC images of the pair term
@@ -815,6 +816,7 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
     L.rst = lists ? take(4 * (maxNA + 1)) : -1;
     L.flist = lists ? take(16 * maxNA) : -1;
     L.shf = lists ? take(16 * nimg) : -1;
+    L.perm = lists ? take(2 * maxNA) : -1;
     L.total = o;
     return L;
 }

@@ -319,7 +319,7 @@ struct CtaSystem {
                 r.x += __shfl_xor_sync(0xffffffffu, r.x, o);
                 r.y += __shfl_xor_sync(0xffffffffu, r.y, o);
                 r.z += __shfl_xor_sync(0xffffffffu, r.z, o);
-                r.w += __shfl_xor_sync(0xffffffffu, r.w, o);
+                if (ENERGY) r.w += __shfl_xor_sync(0xffffffffu, r.w, o);
             }
             if (ok && a == 0) {
                 fgr[i] = make_float4(r.x * P.gmi[0], r.y * P.gmi[1], r.z * P.gmi[2], 0.f);

@@ -109,7 +109,7 @@ struct RelaxEngine : CtaSystem<T> {
     // shifted-image pair lists of the current system (block-uniform): usable
     // (a scratch slot, no overflow so far), built and valid, entries
     bool listok = false, listed = false;
-    int nlist = 0;
+    int nlist = 0, nrows = 0;
 
     __device__ RelaxEngine(const Params& p, const Systems& y, char* smem, const SmemLayout& l) : B(p, y, smem, l) {}
 
@@ -378,6 +378,21 @@ struct RelaxEngine : CtaSystem<T> {
         __syncthreads();
         const int total = rst[natoms];
         if (total > P.vcap) return false;
+        // rows by falling length: the four rows a warp evaluates at a time are
+        // alike (their longest sets the time), atoms without a row drop out
+        unsigned short* perm = at<unsigned short>(L.perm);
+        float4* flist = at<float4>(L.flist);
+        for (int a = tid; a < natoms; a += T) {
+            const int n = rst[a + 1] - rst[a];
+            flist[a] = make_float4(0.f, 0.f, 0.f, 0.f);
+            int rank = 0;
+            for (int o = 0, p0 = 0; o < natoms; o++) {
+                const int p1 = rst[o + 1], m = p1 - p0;
+                rank += (m > n) || (m == n && o < a);
+                p0 = p1;
+            }
+            perm[rank] = (unsigned short)a;
+        }
         unsigned short* ent = vslot();
         for (int i = warp; i < natoms; i += NW) {            // write
             int at0 = rst[i];
@@ -390,6 +405,12 @@ struct RelaxEngine : CtaSystem<T> {
         }
         nlist = total;
         __syncthreads();
+        int lo = 0, hi = natoms;                             // rows that are not empty
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1, a = perm[mid];
+            if (rst[a + 1] > rst[a]) lo = mid + 1; else hi = mid;
+        }
+        nrows = lo;
         return true;
     }
 
@@ -405,23 +426,26 @@ struct RelaxEngine : CtaSystem<T> {
         float4* flist = at<float4>(L.flist);
         const float4* shf = at<float4>(L.shf);
         const unsigned short* ent = vslot();
+        const unsigned short* perm = at<unsigned short>(L.perm);
         const int gl = lane & (G - 1);
         PairC C;
         C.Rc2 = P.Rc2;
         C.kq = pack2(P.kq_rc2, P.kq_rc2); C.one = pack2(1.f, 1.f); C.mone = pack2(-1.f, -1.f);
-        auto first = [&](int i, int& a, int& n, unsigned& w0, unsigned& w1) {
-            a = i < natoms ? rst[i] : 0;
-            n = i < natoms ? rst[i + 1] - a : 0;
+        auto first = [&](int row, int& i, int& a, int& n, unsigned& w0, unsigned& w1) {
+            i = row < nrows ? (int)perm[row] : 0;
+            a = rst[i];
+            n = row < nrows ? rst[i + 1] - a : 0;
             w0 = w1 = 0;
             if (2 * gl < n) { w0 = ent[a + 2 * gl]; w1 = ent[a + min(2 * gl + 1, n - 1)]; }
         };
-        int an, nn;
+        int in, an, nn;
         unsigned u0, u1;
-        first(tid / G, an, nn, u0, u1);
-        for (int i0 = 0; i0 < natoms; i0 += NG) {
-            const int i = i0 + tid / G, a = an, n = nn;
+        first(tid / G, in, an, nn, u0, u1);
+        for (int i0 = 0, k = 0; i0 < nrows; i0 += NG, k++) {
+            const int i = in, a = an, n = nn;
             unsigned w0 = u0, w1 = u1;
-            if (i0 + NG < natoms) first(i + NG, an, nn, u0, u1);
+            // every other round the warps take their rows in reverse order
+            if (i0 + NG < nrows) first(i0 + NG + ((k & 1) ? tid / G : (NG - 4) - 4 * warp + (lane / G)), in, an, nn, u0, u1);
             f32x2 fx = 0, fy = 0, fz = 0;
             if (2 * gl < n) {
                 const float4 pi = spos[i], Ri = sREQ[i];
@@ -449,7 +473,7 @@ struct RelaxEngine : CtaSystem<T> {
                 f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
                 f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
             }
-            if (gl == 0 && i < natoms) {
+            if (gl == 0 && n > 0) {
                 auto lim = [](float x) { return fminf(fmaxf(x, -B::kFixMax), B::kFixMax) + 0.f * x; };   // as fix_add; NaN stays
                 flist[i] = make_float4(lim(f.x), lim(f.y), lim(f.z), 0.f);
             }

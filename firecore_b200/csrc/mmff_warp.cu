@@ -1,18 +1,14 @@
-// mmff_warp.cu -- warp-per-system relaxation for systems of up to 64 atoms.
+// mmff_warp.cu -- one force (and energy) evaluation of systems of up to 64
+// atoms, one warp per system.
 //
-// One warp owns one system.  Lane l owns atoms {l, l+32} (APL = atoms per
-// lane, 1 or 2), the pi orbitals of nodes {l, l+32} and their velocities
-// (kept in registers across the whole relaxation).  Shared memory per warp
-// holds only what other lanes read: positions (atoms + pi), non-bonded
-// parameters and the node recoil slots.  A FIRE step is
-//   bonded (own nodes) -> pair sum (own atoms x all j, smem broadcast,
-//   64-bit exclusion masks) -> B-spline GridFF (own atoms, 64 float4 L2
-//   gathers each) -> __syncwarp -> recoil assembly -> FP64 warp reductions
-//   -> FIRE scalars (FP64, once per warp) -> move -> __syncwarp
-// with no block-level barrier, so the SM interleaves many independent
-// systems.  Physics is identical to mmff_relax.cu (same device functions,
-// same order of operations per term); see mmff_device.cuh for the reference
-// file:line of every term.
+// Lane l owns atoms {l, l+32} (APL = atoms per lane, 1 or 2) and the pi
+// orbitals of nodes {l, l+32}.  Shared memory per warp holds what other lanes
+// read: positions (atoms + pi), non-bonded parameters and the node recoil
+// slots.  Bonded terms (own nodes), pair sum (own atoms x all j, shared-memory
+// broadcasts, 64-bit exclusion masks), B-spline GridFF (own atoms, 64 float4
+// L2 gathers each), recoil assembly; no block-level barrier, so the SM
+// interleaves many independent systems.  Same physics as mmff_eval.cu; see
+// mmff_device.cuh for the reference file:line of every term.
 #include "mmff_device.cuh"
 #include <cfloat>
 
@@ -178,11 +174,11 @@ __device__ __forceinline__ float eval_atom_slots(int ia, int natoms, int nnode, 
 // Excluded and out-of-range pairs get r^2 = 1e30: every term then underflows
 // to zero except the shifted-force constant kq Q / r, below 1e-16 eV/A, so no
 // final select is needed.
-template <int APL, bool ENERGY, bool COUNT, bool HB>
+template <int APL, bool ENERGY, bool HB>
 __device__ __forceinline__ void pair_image(const Params& P, int N, const float4* __restrict__ sp,
                                            const float4* __restrict__ sR, float3 p0, float3 p1, float4 R0i,
                                            float4 R1i, uint32_t m0lo, uint32_t m0hi, uint32_t m1lo, uint32_t m1hi,
-                                           float3& f0, float3& f1, float& e0, float& e1, unsigned long long& np) {
+                                           float3& f0, float3& f1, float& e0, float& e1) {
     const bool CUT = P.Rc2 > 0.f;
     const float Rc2 = CUT ? P.Rc2 : 3.0e38f, kq = P.kq_rc2;
     const float rc = CUT ? sqrtf(1.f / kq) : 0.f;
@@ -214,7 +210,6 @@ __device__ __forceinline__ void pair_image(const Params& P, int N, const float4*
                 if (CUT) e += Q * kq * (r2 * ir - 2.f * rc);
                 e0 += e;
             }
-            if (COUNT && ok) np++;
         }
         if (APL == 2) {
             const float dx = pj.x - p1.x, dy = pj.y - p1.y, dz = pj.z - p1.z;
@@ -239,7 +234,6 @@ __device__ __forceinline__ void pair_image(const Params& P, int N, const float4*
                 if (CUT) e += Q * kq * (r2 * ir - 2.f * rc);
                 e1 += e;
             }
-            if (COUNT && ok) np++;
         }
     }
 }
@@ -253,11 +247,10 @@ __device__ __forceinline__ void pair_image(const Params& P, int N, const float4*
 // component.  Exclusions come from the own atom's mask (bonded neighbours in
 // the central cell are symmetric in MMFFsp3_loc topologies); slots >= N are
 // masked.  Energies are full pair energies (not halved).
-template <bool ENERGY, bool COUNT, bool HB>
+template <bool ENERGY, bool HB>
 __device__ __forceinline__ void central_pairs(const Params& P, int N, int lane, const float4* __restrict__ sp,
                                               const float4* __restrict__ sR, uint32_t m0lo, uint32_t m0hi,
-                                              uint32_t m1lo, uint32_t m1hi, float3& f0, float3& f1, float& ec,
-                                              unsigned long long& np) {
+                                              uint32_t m1lo, uint32_t m1hi, float3& f0, float3& f1, float& ec) {
     const bool CUT = P.Rc2 > 0.f;
     const float Rc2 = CUT ? P.Rc2 : 3.0e38f, kq = P.kq_rc2;
     const float rc = CUT ? sqrtf(1.f / kq) : 0.f;
@@ -278,7 +271,6 @@ __device__ __forceinline__ void central_pairs(const Params& P, int N, int lane, 
         f0.x = fmaf(dx, F, f0.x); f0.y = fmaf(dy, F, f0.y); f0.z = fmaf(dz, F, f0.z);
         f1.x = fmaf(-dx, F, f1.x); f1.y = fmaf(-dy, F, f1.y); f1.z = fmaf(-dz, F, f1.z);
         if (ENERGY) ec += e;
-        if (COUNT && ok) np += 2;
     }
 #ifndef MMFF_CENTRAL_UNROLL
 #define MMFF_CENTRAL_UNROLL 1
@@ -298,16 +290,14 @@ __device__ __forceinline__ void central_pairs(const Params& P, int N, int lane, 
                 f0.x = fmaf(dx, F, f0.x); f0.y = fmaf(dy, F, f0.y); f0.z = fmaf(dz, F, f0.z);
                 rA.x = -dx * F; rA.y = -dy * F; rA.z = -dz * F;
                 if (ENERGY) ec += e;
-                if (COUNT && ok) np += 2;
-            }
+                    }
             {   // s = 16: this is (A', B) of lane p, done there
                 const float dx = qA.x - q1.x, dy = qA.y - q1.y, dz = qA.z - q1.z;
                 const float F = pair_force<ENERGY, HB>(dx, dy, dz, R1, RA, ((m1lo >> p) & 1u) || (s == 16), Rc2, kq, rc, CUT, ok, e);
                 f1.x = fmaf(dx, F, f1.x); f1.y = fmaf(dy, F, f1.y); f1.z = fmaf(dz, F, f1.z);
                 rA.x = fmaf(-dx, F, rA.x); rA.y = fmaf(-dy, F, rA.y); rA.z = fmaf(-dz, F, rA.z);
                 if (ENERGY) ec += e;
-                if (COUNT && ok) np += 2;
-            }
+                    }
             f0.x += __shfl_sync(0xffffffffu, rA.x, src); f0.y += __shfl_sync(0xffffffffu, rA.y, src);
             f0.z += __shfl_sync(0xffffffffu, rA.z, src);
         }
@@ -320,16 +310,14 @@ __device__ __forceinline__ void central_pairs(const Params& P, int N, int lane, 
                 f1.x = fmaf(dx, F, f1.x); f1.y = fmaf(dy, F, f1.y); f1.z = fmaf(dz, F, f1.z);
                 rB.x = -dx * F; rB.y = -dy * F; rB.z = -dz * F;
                 if (ENERGY) ec += e;
-                if (COUNT && ok) np += 2;
-            }
+                    }
             {
                 const float dx = qB.x - q0.x, dy = qB.y - q0.y, dz = qB.z - q0.z;
                 const float F = pair_force<ENERGY, HB>(dx, dy, dz, R0, RB, (m0hi >> p) & 1u, Rc2, kq, rc, CUT, ok, e);
                 f0.x = fmaf(dx, F, f0.x); f0.y = fmaf(dy, F, f0.y); f0.z = fmaf(dz, F, f0.z);
                 rB.x = fmaf(-dx, F, rB.x); rB.y = fmaf(-dy, F, rB.y); rB.z = fmaf(-dz, F, rB.z);
                 if (ENERGY) ec += e;
-                if (COUNT && ok) np += 2;
-            }
+                    }
             f1.x += __shfl_sync(0xffffffffu, rB.x, src); f1.y += __shfl_sync(0xffffffffu, rB.y, src);
             f1.z += __shfl_sync(0xffffffffu, rB.z, src);
         }
@@ -349,7 +337,7 @@ __device__ __forceinline__ void excl_mask(int a, int4 ng, int4 ngC, int ipbc, bo
     if (!pbc || ngC.w == ipbc) setb(ng.w);
 }
 
-template <int APL, bool ENERGY, bool COUNT>
+template <int APL, bool ENERGY>
 struct WarpEngine {
     const Params& P;
     const Systems& Y;
@@ -366,13 +354,11 @@ struct WarpEngine {
     int isys, N, NN, NV, aoff, noff, voff;
     float* lv;       // [9] lattice vectors, then 3 floats grid offset, in the warp's region
     bool hasH;
-    // owned state (k = 0, 1): atom a_k = lane + 32k, node n_k = a_k if < NN
-    float3 va[APL], vp[APL];        // velocities of own atoms / own pi vectors
-    float3 fasm_a[APL], fasm_p[APL];// assembled forces of the current step
+    // own vectors (k = 0, 1): atom a_k = lane + 32k, node n_k = a_k if < NN
+    float3 fasm_a[APL], fasm_p[APL];// assembled forces
     const uint32_t* xrow;           // central-image exclusion rows of the system (ceil(N/32) words per atom)
     int nbw;                        // words per row
     double e13 = 0.0;               // ENERGY: pair energies of the skipped 1-3 pairs (energy split)
-    unsigned long long npair = 0;
 
     __device__ WarpEngine(const Params& p, const Systems& y, char* region, const WarpLayout& L, int maxNN_)
         : P(p), Y(y), maxNN(maxNN_) {
@@ -407,14 +393,6 @@ struct WarpEngine {
             spar[5 * n + 3] = Y.Ksp[noff + n]; spar[5 * n + 4] = Y.Kpp[noff + n];
         }
         hasH = __any_sync(0xffffffffu, h);
-#pragma unroll
-        for (int k = 0; k < APL; k++) {
-            const int a = lane + 32 * k;
-            const bool va_ok = a < N, vp_ok = a < NN;
-            const float4 v1 = va_ok ? Y.vel[voff + a] : make_float4(0, 0, 0, 0);
-            const float4 v2 = vp_ok ? Y.vel[voff + N + a] : make_float4(0, 0, 0, 0);
-            va[k] = f3(v1); vp[k] = f3(v2);
-        }
         __syncwarp();
     }
 
@@ -495,16 +473,16 @@ struct WarpEngine {
                             if (APL == 2 && a1 < N) excl_mask(a1, sng[a1], sngC[a1], ipbc, pbc, m1lo, m1hi); else { m1lo = m1hi = ~0u; }
                         }
                         if (APL == 2 && (ix | iy | iz) == 0) {      // central image: each pair once
-                            if (hasH) central_pairs<ENERGY, COUNT, true>(P, N, lane, sp, sR, m0lo, m0hi, m1lo, m1hi, f0, f1, ec, npair);
-                            else central_pairs<ENERGY, COUNT, false>(P, N, lane, sp, sR, m0lo, m0hi, m1lo, m1hi, f0, f1, ec, npair);
+                            if (hasH) central_pairs<ENERGY, true>(P, N, lane, sp, sR, m0lo, m0hi, m1lo, m1hi, f0, f1, ec);
+                            else central_pairs<ENERGY, false>(P, N, lane, sp, sR, m0lo, m0hi, m1lo, m1hi, f0, f1, ec);
                             continue;
                         }
                         const float3 p0 = make_float3(q0.x - shx, q0.y - shy, q0.z - shz);
                         const float3 p1 = make_float3(q1.x - shx, q1.y - shy, q1.z - shz);
                         if (hasH)
-                            pair_image<APL, ENERGY, COUNT, true>(P, N, sp, sR, p0, p1, Ri0, Ri1, m0lo, m0hi, m1lo, m1hi, f0, f1, e0, e1, npair);
+                            pair_image<APL, ENERGY, true>(P, N, sp, sR, p0, p1, Ri0, Ri1, m0lo, m0hi, m1lo, m1hi, f0, f1, e0, e1);
                         else
-                            pair_image<APL, ENERGY, COUNT, false>(P, N, sp, sR, p0, p1, Ri0, Ri1, m0lo, m0hi, m1lo, m1hi, f0, f1, e0, e1, npair);
+                            pair_image<APL, ENERGY, false>(P, N, sp, sR, p0, p1, Ri0, Ri1, m0lo, m0hi, m1lo, m1hi, f0, f1, e0, e1);
                     }
             if (ENERGY) Enb += 0.5 * ((double)e0 + (double)e1) + (double)ec;
         }
@@ -561,221 +539,7 @@ struct WarpEngine {
         }
     }
 
-    // clamp + FIRE sums of owned vectors, then warp totals (identical in all lanes)
-    __device__ void fire_sums(double& vf, double& vv, double& ff, float& fmax2, bool& bad) {
-        const float Fl = P.Flim;
-        vf = 0; vv = 0; ff = 0; fmax2 = 0.f; bool b = false;
-#pragma unroll
-        for (int k = 0; k < APL; k++) {
-            const int a = lane + 32 * k;
-#pragma unroll
-            for (int w = 0; w < 2; w++) {
-                const bool valid = (w == 0) ? (a < N) : (a < NN);
-                if (!valid) continue;
-                float3 f = (w == 0) ? fasm_a[k] : fasm_p[k];
-                const float3 v = (w == 0) ? va[k] : vp[k];
-                if ((P.flags & F_BCONS) && w == 0) f = bond_constraint_force(Y, isys, a, sp, lv, f);
-                if (Fl > 0.f) {
-                    const float fr2 = dot3(f, f);
-                    if (fr2 > Fl * Fl) f = f * (Fl * rsqrtf(fr2));
-                }
-                if ((P.flags & F_CONSTR) && w == 0) f = constraint_force(Y, aoff + a, f3(sp[a]), f);
-                // a system whose atoms left any sensible range is retired like a non-finite one
-                if (w == 0) { const float4 p = sp[a]; b |= !(fabsf(p.x) + fabsf(p.y) + fabsf(p.z) < 1e5f); }
-                if (w == 0) fasm_a[k] = f; else fasm_p[k] = f;
-                vf += (double)v.x * f.x + (double)v.y * f.y + (double)v.z * f.z;
-                vv += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z;
-                const double f2 = (double)f.x * f.x + (double)f.y * f.y + (double)f.z * f.z;
-                ff += f2;
-                fmax2 = fmaxf(fmax2, (float)f2);
-                b |= !isfinite(f.x + f.y + f.z);
-            }
-        }
-        vf = wsum_d(vf); vv = wsum_d(vv); ff = wsum_d(ff); fmax2 = wmax_f(fmax2);
-        bad = __any_sync(0xffffffffu, b);
-    }
-
-    __device__ void move(double dt, double cv, double cfm) {
-        const float dtf = (float)dt;
-        const float cvf = (float)cv;
-        const float kf = (float)((double)dtf + cfm);
-#pragma unroll
-        for (int k = 0; k < APL; k++) {
-            const int a = lane + 32 * k;
-            if (a < N) {
-                float3 v = va[k] * cvf;
-                v = fma3(fasm_a[k], kf, v);
-                float3 p = f3(sp[a]);
-                p = fma3(v, dtf, p);
-                sp[a] = make_float4(p.x, p.y, p.z, 0.f);
-                va[k] = v;
-            }
-            if (a < NN) {
-                float3 p = f3(sp[N + a]);
-                float3 f = fasm_p[k];
-                f = fma3(p, -dot3(p, f), f);
-                float3 v = vp[k] * cvf;
-                v = fma3(f, kf, v);
-                v = fma3(p, -dot3(p, v), v);
-                p = fma3(v, dtf, p);
-                p = p * rsqrtf(dot3(p, p));
-                sp[N + a] = make_float4(p.x, p.y, p.z, 0.f);
-                vp[k] = v;
-            }
-        }
-        __syncwarp();
-    }
-
-    // Langevin step (MMFFsp3_loc::move_atom_Langevin, MMFFsp3_loc.h:1191-1216)
-    __device__ void move_md(int step) {
-        const float dt = P.md_dt, g = P.md_gamma, nz = P.md_noise;
-#pragma unroll
-        for (int k = 0; k < APL; k++) {
-            const int a = lane + 32 * k;
-#pragma unroll
-            for (int w = 0; w < 2; w++) {
-                const bool valid = (w == 0) ? (a < N) : (a < NN);
-                if (!valid) continue;
-                const int v = (w == 0) ? a : N + a;
-                float3 p = f3(sp[v]);
-                float3 f = (w == 0) ? fasm_a[k] : fasm_p[k];
-                float3 ve = (w == 0) ? va[k] : vp[k];
-                if (w == 1) f = fma3(p, -dot3(p, f), f);
-                f = fma3(ve, -g, f);
-                const long long gv = (long long)voff + v;
-                f.x = fmaf(langevin_rand(P.md_seed, gv, step, 0), nz, f.x);
-                f.y = fmaf(langevin_rand(P.md_seed, gv, step, 1), nz, f.y);
-                f.z = fmaf(langevin_rand(P.md_seed, gv, step, 2), nz, f.z);
-                ve = fma3(f, dt, ve);
-                if (w == 1) ve = fma3(p, -dot3(p, ve), ve);
-                p = fma3(ve, dt, p);
-                if (w == 1) p = p * rsqrtf(dot3(p, p));
-                sp[v] = make_float4(p.x, p.y, p.z, 0.f);
-                if (w == 0) va[k] = ve; else vp[k] = ve;
-            }
-        }
-        __syncwarp();
-    }
-
-    // copy of the positions just moved (move ends with __syncwarp)
-    __device__ void snapshot() {
-        for (int v = lane; v < NV; v += 32) Y.minpos[voff + v] = sp[v];
-    }
-
-    __device__ void store(int status, int steps, float meas, double dt, double damping, int lastNeg, double total) {
-        for (int v = lane; v < NV; v += 32) Y.pos[voff + v] = sp[v];
-#pragma unroll
-        for (int k = 0; k < APL; k++) {
-            const int a = lane + 32 * k;
-            if (a < N) { Y.vel[voff + a] = make_float4(va[k].x, va[k].y, va[k].z, 0.f); Y.force[voff + a] = make_float4(fasm_a[k].x, fasm_a[k].y, fasm_a[k].z, 0.f); }
-            if (a < NN) { Y.vel[voff + N + a] = make_float4(vp[k].x, vp[k].y, vp[k].z, 0.f); Y.force[voff + N + a] = make_float4(fasm_p[k].x, fasm_p[k].y, fasm_p[k].z, 0.f); }
-        }
-        if (lane == 0) {
-            Y.fire[isys] = make_double4(dt, damping, (double)lastNeg, total);
-            Y.status[isys] = status;
-            Y.nsteps[isys] = steps;
-            Y.fconv[isys] = meas;
-        }
-    }
 };
-
-// Persistent: every warp claims systems from queue[] until it is empty.
-// minimum resident CTAs per SM the register allocation targets (build option)
-#ifndef MMFF_WARP_MINB
-#define MMFF_WARP_MINB 4
-#endif
-// EXPL: the exploring cycle (P.md_mode 2) instead of plain FIRE or the drive.
-template <int APL, bool COUNT, bool EXPL = false>
-__global__ void __launch_bounds__(128, MMFF_WARP_MINB) relax_warp_kernel(Params P, Systems Y, const int* __restrict__ queue, int nqueue,
-                                                         int* counter, int maxNA, int maxNN) {
-    extern __shared__ __align__(16) char smem[];
-    const WarpLayout L = warp_layout(maxNA, maxNN);
-    char* region = smem + (threadIdx.x >> 5) * L.per_warp;
-    WarpEngine<APL, false, COUNT> E(P, Y, region, L, maxNN);
-    const int lane = threadIdx.x & 31;
-    while (true) {
-        int q = 0;
-        if (lane == 0) q = atomicAdd(counter, 1);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= nqueue) break;
-        const int s = queue[q];
-        E.load(s);
-        const double4 fs = Y.fire[s];
-        double dt = fs.x, damping = fs.y, total = fs.w;
-        int lastNeg = (int)fs.z;
-        int status = ST_MAXSTEPS, itr = 0;
-        float meas = 0.f;
-        int ph = 0;                 // exploring cycle: 2 * (steps in the phase) + exploring
-        if constexpr (EXPL) { const int4 g = Y.gopt[s]; ph = 2 * g.y + (g.x != 0); }
-        for (itr = 0; itr < P.nstep_max; itr++) {
-            bool lang = false;      // an exploring step (Langevin instead of FIRE)
-            if constexpr (EXPL) {
-                const int ev = explore_step(ph, P.n_explore, P.n_relax);
-                lang = ev & 1;
-                if ((ev & 2) && lane == 0) Y.gopt[s].w++;
-            }
-            double d0 = 0, d1 = 0, d2 = 0;
-            E.forces(d0, d1, d2);
-            double vf, vv, ff;
-            float fmax2;
-            bool bad;
-            E.fire_sums(vf, vv, ff, fmax2, bad);
-            if (bad) { status = ST_NAN; break; }
-            if (!EXPL && P.md_mode) {   // Langevin drive: fixed number of steps, no FIRE
-                E.move_md(P.md_step0 + itr);
-                total += 1.0;
-                meas = sqrtf(fmax2);
-                continue;
-            }
-            // DynamicOpt::FIRE_update_params (DynamicOpt.cpp:250-267), FP64; in the
-            // exploring cycle the FIRE scalars evolve in exploring steps too
-            // (MolWorld_sp3.h:2401-2424)
-            const double f_len = sqrt(ff), v_len = sqrt(vv);
-            const double cos_vf = vf / (f_len * v_len + 1e-32);
-            const double renorm_vf = v_len / (f_len + 1e-32);
-            double cv, cf;
-            if (cos_vf < 0.0) { cv = P.cv_kill; cf = 0.0; } else { cv = 1.0 - damping; cf = damping; }
-            cf = renorm_vf * cf;
-            if (cos_vf < 0.0) {
-                dt = fmax(dt * P.fdec, P.dt_min);
-                lastNeg = 0;
-                damping = P.damp_max;
-            } else {
-                if (lastNeg > P.minLastNeg) { dt = fmin(dt * P.finc, P.dt_max); damping = damping * P.falpha; }
-                lastNeg++;
-            }
-            if (EXPL && lang) E.move_md(P.md_step0 + itr);
-            else E.move(dt, cv, P.fire_variant == 1 ? cf : renorm_vf * cf);
-            total += 1.0;
-            const double m = (P.conv_mode == 0) ? ff : (double)fmax2;
-            meas = (float)sqrt(m);
-            if constexpr (EXPL) {
-                if (!lang && m < P.Fconv2) {
-                    // a minimum (MolWorld_sp3.h:2465-2473): keep it, start exploring
-                    E.snapshot();
-                    if (lane == 0) Y.gopt[s].z++;
-                    ph = 1;
-                }
-            } else {
-                if (m < P.Fconv2) { status = ST_CONVERGED; itr++; break; }
-            }
-        }
-        const int steps = (status == ST_CONVERGED) ? itr - 1 : itr;
-        E.store(status, steps, meas, dt, damping, lastNeg, total);
-        if (EXPL && lane == 0) { Y.gopt[s].x = ph & 1; Y.gopt[s].y = ph >> 1; }
-        if (COUNT && lane == 0) {
-            atomicAdd(Y.counters + 1, (unsigned long long)itr * (unsigned long long)E.N);
-            atomicAdd(Y.counters + 2, (unsigned long long)itr);
-        }
-        __syncwarp();
-    }
-    if (COUNT) {
-        unsigned long long np = E.npair;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) np += __shfl_xor_sync(0xffffffffu, np, o);
-        if (lane == 0) atomicAdd(Y.counters, np);
-    }
-}
 
 // One force (and energy) evaluation; warp w of block b takes queue[b*4 + w].
 template <int APL, bool ENERGY>
@@ -786,7 +550,7 @@ __global__ void __launch_bounds__(128) eval_warp_kernel(Params P, Systems Y, con
     char* region = smem + (threadIdx.x >> 5) * L.per_warp;
     const int q = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (q >= nqueue) return;
-    WarpEngine<APL, ENERGY, false> E(P, Y, region, L, maxNN);
+    WarpEngine<APL, ENERGY> E(P, Y, region, L, maxNN);
     const int s = queue[q];
     E.load(s);
     double Eb = 0, Enb = 0, Eg = 0;
@@ -811,16 +575,6 @@ __global__ void __launch_bounds__(128) eval_warp_kernel(Params P, Systems Y, con
     if (lane == 0) Y.fconv[s] = sqrtf(fm);
 }
 
-void* relax_warp_fn(int apl, bool count) {
-    if (apl == 1) return count ? (void*)relax_warp_kernel<1, true> : (void*)relax_warp_kernel<1, false>;
-    if (apl == 2) return count ? (void*)relax_warp_kernel<2, true> : (void*)relax_warp_kernel<2, false>;
-    return nullptr;
-}
-void* relax_warp_explore_fn(int apl) {
-    if (apl == 1) return (void*)relax_warp_kernel<1, false, true>;
-    if (apl == 2) return (void*)relax_warp_kernel<2, false, true>;
-    return nullptr;
-}
 void* eval_warp_fn(int apl, bool energy) {
     if (apl == 1) return energy ? (void*)eval_warp_kernel<1, true> : (void*)eval_warp_kernel<1, false>;
     if (apl == 2) return energy ? (void*)eval_warp_kernel<2, true> : (void*)eval_warp_kernel<2, false>;

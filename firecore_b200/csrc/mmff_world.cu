@@ -35,9 +35,7 @@ __global__ void solve_periodic_kernel(double*, long, int, long, long, long, cons
 __global__ void pack_grid_kernel(long, const double*, float4*);
 void* relax_fn(int T, bool count);
 void* eval_fn(int T, int S, bool energy);
-void* relax_warp_fn(int apl, bool count);
 void* relax_explore_fn(int T);
-void* relax_warp_explore_fn(int apl);
 void* eval_warp_fn(int apl, bool energy);
 
 }  // namespace mmff
@@ -75,8 +73,6 @@ template <class X> struct DBuf {
 };
 
 struct Bucket {
-    int kind = 0;                  // 0: CTA per system (T threads, S lanes per atom); 1: warp per system
-    int apl = 1;                   // warp engine: atoms per lane (1: <=32 atoms, 2: <=64)
     int T = 64, S = 1, maxNA = 0, maxNN = 0;
     std::vector<int> sys;          // system indices, largest first
     DBuf<int> queue;
@@ -91,11 +87,14 @@ struct Bucket {
     int vcap = 0;
 };
 
-// autotuned launch configuration of one size class (kind -1: heuristic)
+// autotuned launch configuration of one size class (kind -1: default_config;
+// 1, from files saved when small systems had a warp of a shared block each: a
+// block of its own with as many lanes)
 struct Tune {
     int kind = -1, apl = 1, T = 0, S = 0;
     float us_per_sys_step = 0.f;
 };
+int tuned_threads(const Tune& t) { return t.kind == 1 ? 32 * t.apl : t.T; }
 
 struct World {
     bool ready = false;
@@ -279,40 +278,33 @@ int set_smem_limit(void* fn, int bytes) {
     return 0;
 }
 
-// launch configuration of a bucket whose systems are set: kind 1 = warp
-// engine (apl atoms per lane), kind 0 = CTA engine with T threads and S lanes
-// per atom in the pair sum.  Fills smem, grid; sets kernel attributes.
-int config_bucket(Bucket& B, int kind, int apl, int T, int S) {
+// launch configuration of a bucket whose systems are set: T threads per system,
+// S lanes per atom on the image rows of the evaluation.  Fills layouts, sizes
+// and grid; sets kernel attributes.
+int config_bucket(Bucket& B, int T, int S) {
     int dev_smem = 0;
     CK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, W.device));
     B.maxNA = 0; B.maxNN = 0;
     for (int s : B.sys) { B.maxNA = std::max(B.maxNA, W.natoms[s]); B.maxNN = std::max(B.maxNN, W.nnode[s]); }
     const int nimg = W.Rcut > 0 ? shifted_images(W.flags, W.npbc) : 0;
     void* fns[3];
-    if (kind == 1) {
-        if (B.maxNA > 32 * apl) return fail("warp engine with %d atoms per lane cannot hold %d atoms", apl, B.maxNA);
-        B.kind = 1; B.apl = apl; B.T = 128; B.S = 1;
-        B.smem = 4 * warp_layout(B.maxNA, B.maxNN).per_warp;
-        fns[0] = relax_warp_fn(B.apl, false); fns[1] = relax_warp_fn(B.apl, true); fns[2] = relax_warp_explore_fn(B.apl);
-    } else {
-        B.kind = 0; B.T = T; B.S = S;
+    B.T = T; B.S = S;
+    B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
+    if (B.lay.total > dev_smem && B.T < kCompactMinThreads) {     // only the larger blocks leave arrays in global memory
+        B.T = kCompactMinThreads;
         B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
-        if (B.lay.total > dev_smem && B.T < kCompactMinThreads) {     // only the larger blocks leave arrays in global memory
-            B.T = kCompactMinThreads;
-            B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
-        }
-        B.smem = B.lay.total;
-        fns[0] = relax_fn(B.T, false); fns[1] = relax_fn(B.T, true); fns[2] = relax_explore_fn(B.T);
     }
+    B.smem = B.lay.total;
+    fns[0] = relax_fn(B.T, false); fns[1] = relax_fn(B.T, true); fns[2] = relax_explore_fn(B.T);
     // evaluation: one pass over the system, a warp each up to 64 atoms
     B.eapl = B.maxNA <= 32 ? 1 : B.maxNA <= 64 ? 2 : 0;
-    if (kind == 0 && W.force_T) B.eapl = 0;
+    if (W.force_T) B.eapl = 0;
     B.eT = B.eapl ? 128 : T;
     if (!B.eapl) B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, false);
     B.esmem = B.eapl ? 4 * warp_layout(B.maxNA, B.maxNN).per_warp : B.elay.total;
     if (B.smem > dev_smem || B.esmem > dev_smem)
         return fail("system too large for shared memory: %d B > %d B", std::max(B.smem, B.esmem), dev_smem);
-    if (!fns[0] || !fns[1] || !fns[2]) return fail("no kernel for bucket (kind %d, T=%d, S=%d)", B.kind, B.T, B.S);
+    if (!fns[0] || !fns[1] || !fns[2]) return fail("no kernel for bucket (T=%d, S=%d)", B.T, B.S);
     for (int f = 0; f < 3; f++) if (set_smem_limit(fns[f], B.smem)) return -1;
     for (int e = 0; e < 2; e++) {
         void* ef = B.eapl ? eval_warp_fn(B.eapl, e) : eval_fn(B.eT, B.S, e);
@@ -322,11 +314,9 @@ int config_bucket(Bucket& B, int kind, int apl, int T, int S) {
     int occ = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[0], B.T, B.smem));
     if (occ < 1) return fail("kernel cannot be resident (T=%d smem=%d)", B.T, B.smem);
-    const int per_block = B.kind ? 4 : 1;
-    const int nblk = ((int)B.sys.size() + per_block - 1) / per_block;
-    B.grid = std::min(nblk, occ * W.nsm);
+    B.grid = std::min((int)B.sys.size(), occ * W.nsm);
     B.vcap = 0;
-    if (kind == 0 && nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
+    if (nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
         B.vcap = B.maxNA * kListEntriesPerAtom;
         if (B.vl.ensure((size_t)B.grid * B.vcap)) return -1;
     }
@@ -341,8 +331,7 @@ int config_bucket(Bucket& B, int kind, int apl, int T, int S) {
 // enough to fill the chip.  With fewer, the idle warp slots go to more threads
 // per system: about 16 warps per SM over the systems an SM holds, as far as a
 // system of that class still gains from them.
-void default_config(int cls, int maxNA, int nsys, int& kind, int& apl, int& T, int& S) {
-    kind = 0; apl = 1;
+void default_config(int cls, int maxNA, int nsys, int& T, int& S) {
     T = cls == 0 ? 32 : cls == 1 ? 64 : std::min(256, kClassT[cls - 2]);
     S = cls <= 1 ? 1 : std::min(pow2_floor(std::max(1, kClassT[cls - 2] / std::max(1, maxNA))), 8);
     if (W.force_T) T = W.force_T;
@@ -457,11 +446,11 @@ int build_buckets() {
         std::stable_sort(B.sys.begin(), B.sys.end(), [](int a, int b) { return W.natoms[a] > W.natoms[b]; });
         int maxNA = 0;
         for (int s : B.sys) maxNA = std::max(maxNA, W.natoms[s]);
-        int kind, apl, T, S;
-        default_config(k, maxNA, (int)B.sys.size(), kind, apl, T, S);
+        int T, S;
+        default_config(k, maxNA, (int)B.sys.size(), T, S);
         const Tune& tu = W.tune[k];
-        if (tu.kind >= 0 && !W.force_T && !W.force_S) { kind = tu.kind; apl = tu.apl; T = tu.T; S = tu.S; }
-        if (config_bucket(B, kind, apl, T, S)) return -1;
+        if (tu.kind >= 0 && !W.force_T && !W.force_S) { T = tuned_threads(tu); S = tu.S; }
+        if (config_bucket(B, T, S)) return -1;
         B.cls = k;
         W.buckets.push_back(std::move(B));
     }
@@ -493,7 +482,7 @@ PinnedBuf g_stage_a, g_stage_b;
 
 // the bucket's pair-list scratch into the launch parameters (CTA relax kernels)
 void set_lists(Params& P, const Bucket& B) {
-    const bool on = W.pair_lists && B.kind == 0 && B.vcap > 0 && B.vl.p;
+    const bool on = W.pair_lists && B.vcap > 0 && B.vl.p;
     P.vlist = on ? B.vl.p : nullptr;
     P.vcap = on ? B.vcap : 0;
     P.vskin = (float)W.list_skin;
@@ -511,14 +500,12 @@ int enqueue_relax(const Params& P) {
         Bucket& B = W.buckets[b];
         cudaStream_t st = W.bstreams[b];
         CK(cudaStreamWaitEvent(st, W.evfork, 0));
-        void* fn = P.md_mode == 2 ? (B.kind ? relax_warp_explore_fn(B.apl) : relax_explore_fn(B.T))
-                                  : (B.kind ? relax_warp_fn(B.apl, W.count) : relax_fn(B.T, W.count));
+        void* fn = P.md_mode == 2 ? relax_explore_fn(B.T) : relax_fn(B.T, W.count);
         const int* q = B.queue.p;
         int nq = (int)B.sys.size();
         int* ctr = W.d_counter.p + b;
-        int mna = B.maxNA, mnn = B.maxNN;
         set_lists(Pc, B);
-        void* args[] = {&Pc, &Y, &q, &nq, &ctr, B.kind ? (void*)&mna : (void*)&B.lay, &mnn};
+        void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
         CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
         if (!g_capturing) g_launches++;
     }
@@ -1235,14 +1222,15 @@ int mmff_set_graph(int on) {
 
 // ---------------------------------------------------------------- autotuner
 namespace {
-struct Cand { int kind, apl, T, S; };
+// threads per system tried for a size class, with the evaluation's lanes per atom
+struct Cand { int T, S; };
 std::vector<Cand> candidates(int cls) {
     switch (cls) {
-        case 0: return {{1, 1, 128, 1}, {0, 1, 64, 1}, {0, 1, 64, 2}, {0, 1, 64, 4}, {0, 1, 128, 2}, {0, 1, 128, 4}};
-        case 1: return {{1, 2, 128, 1}, {0, 1, 64, 1}, {0, 1, 64, 2}, {0, 1, 128, 1}, {0, 1, 128, 2}, {0, 1, 128, 4}};
-        case 3: return {{0, 1, 64, 1}, {0, 1, 64, 2}, {0, 1, 128, 1}, {0, 1, 128, 2}, {0, 1, 128, 4}, {0, 1, 256, 2}, {0, 1, 256, 4}};
-        case 4: return {{0, 1, 128, 1}, {0, 1, 128, 2}, {0, 1, 256, 1}, {0, 1, 256, 2}, {0, 1, 512, 1}, {0, 1, 512, 2}};
-        case 5: return {{0, 1, 256, 1}, {0, 1, 256, 2}, {0, 1, 512, 1}, {0, 1, 512, 2}, {0, 1, 512, 4}};
+        case 0: return {{32, 1}, {64, 1}, {128, 1}};
+        case 1: return {{32, 1}, {64, 1}, {128, 1}};
+        case 3: return {{64, 1}, {128, 1}, {256, 2}};
+        case 4: return {{128, 1}, {256, 1}, {512, 2}};
+        case 5: return {{256, 1}, {512, 1}};
         default: return {};
     }
 }
@@ -1294,13 +1282,13 @@ int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap
             Bucket B;
             B.sys = sample;
             float us = -1.f;
-            if (config_bucket(B, c.kind, c.apl, c.T, c.S) == 0) {
-                void* fn = B.kind ? relax_warp_fn(B.apl, false) : relax_fn(B.T, false);
+            if (config_bucket(B, c.T, c.S) == 0) {
+                void* fn = relax_fn(B.T, false);
                 const int* q = B.queue.p;
-                int nq = (int)B.sys.size(), mna = B.maxNA, mnn = B.maxNN;
+                int nq = (int)B.sys.size();
                 int* ctr = W.d_counter.p + 32;
                 set_lists(P, B);
-                void* args[] = {&P, &Y, &q, &nq, &ctr, B.kind ? (void*)&mna : (void*)&B.lay, &mnn};
+                void* args[] = {&P, &Y, &q, &nq, &ctr, &B.lay};
                 float ms = 0.f;
                 for (int rep = 0; rep < 2; rep++) {        // first launch warms caches and clocks
                     if (copy_state(false)) return -1;
@@ -1313,14 +1301,14 @@ int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap
                     CK(cudaEventElapsedTime(&ms, W.ev0, W.ev1));
                 }
                 us = 1e3f * ms / ((float)ns * (float)nstep_probe);
-                if (us < best) { best = us; bt.kind = c.kind; bt.apl = c.apl; bt.T = c.T; bt.S = c.S; bt.us_per_sys_step = us; }
+                if (us < best) { best = us; bt.kind = 0; bt.apl = 1; bt.T = c.T; bt.S = c.S; bt.us_per_sys_step = us; }
             } else {
                 cudaGetLastError();
             }
             B.queue.release();
             B.vl.release();
             if (report && nrep < report_cap) {
-                const float row[6] = {(float)cls, (float)c.kind, (float)c.apl, (float)c.T, (float)c.S, us};
+                const float row[6] = {(float)cls, 0.f, 1.f, (float)c.T, (float)c.S, us};
                 for (int j = 0; j < 6; j++) report[6 * nrep + j] = row[j];
             }
             nrep++;
@@ -1347,6 +1335,7 @@ int mmff_set_tuning(int cls, int kind, int apl, int T, int S) {
     if (cls < 0 || cls > 5) return fail("size class must be 0..5");
     if (kind == 1 && !((cls == 0 && apl == 1) || (cls == 1 && apl == 2))) return fail("warp engine only for classes 0/1 (apl = class + 1)");
     if (kind == 0 && (!relax_fn(T, false) || !(S == 1 || S == 2 || S == 4 || S == 8))) return fail("no CTA kernel with T=%d S=%d", T, S);
+    if (kind == 0 && T == 32 && cls > 1) return fail("32 threads per system only for classes 0/1");
     if (kind != -1 && kind != 0 && kind != 1) return fail("kind must be -1, 0 or 1");
     W.tune[cls].kind = kind; W.tune[cls].apl = apl; W.tune[cls].T = T; W.tune[cls].S = S;
     W.buckets_dirty = true;
@@ -1456,7 +1445,7 @@ int mmff_num_buckets(void) { return W.buckets_dirty ? -1 : (int)W.buckets.size()
 int mmff_bucket_info(int b, int* info) {
     if (b < 0 || b >= (int)W.buckets.size()) return fail("bad bucket");
     const Bucket& B = W.buckets[b];
-    info[0] = B.T; info[1] = B.kind ? -B.apl : B.S; info[2] = (int)B.sys.size(); info[3] = B.maxNA; info[4] = B.maxNN; info[5] = B.smem; info[6] = B.grid;
+    info[0] = B.T; info[1] = B.S; info[2] = (int)B.sys.size(); info[3] = B.maxNA; info[4] = B.maxNN; info[5] = B.smem; info[6] = B.grid;
     return 0;
 }
 

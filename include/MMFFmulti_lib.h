@@ -208,15 +208,16 @@ int mmff_explore(int nsteps, double Fconv, int conv_mode);
 int mmff_get_explore(int* gopt, double* minpos);
 /* Autotuner (no counterpart in the reference, which uses one fixed work-group
  * size): for each size class present (0: <= 32 atoms, 1: <= 64, 3: <= 128,
- * 4: <= 256, 5: larger), time every candidate launch configuration (warp per
- * system, or threads per CTA x lanes per atom in the pair sum) on up to
+ * 4: <= 256, 5: larger), time every candidate launch configuration (threads per
+ * system) on up to
  * max_sample of its systems for nstep_probe FIRE steps and keep the fastest.
  * State is restored.  report [6 per candidate] (nullable): class, kind,
  * atoms per lane, threads, pair lanes, us per system-step (< 0: not
  * launchable).  Returns the number of candidates tried. */
 int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap);
 /* Tuned configuration of size class cls: out[4] = (kind: -1 heuristic, 0 CTA
- * per system, 1 warp per system; atoms per lane; threads; pair lanes). */
+ * per system, 1 (files of earlier versions) 32 x atoms-per-lane threads per
+ * system; atoms per lane; threads; pair lanes of the evaluation). */
 int mmff_get_tuning(int cls, int* out);
 int mmff_set_tuning(int cls, int kind, int apl, int threads, int pair_split);
 
@@ -243,8 +244,7 @@ int mmff_get_counters(unsigned long long* out);
 double mmff_peak_fp32(void);
 double mmff_peak_l2(int mbytes);
 int mmff_num_buckets(void);
-/* info[7] = (threads, pair_split, nsys, maxNA, maxNN, smem bytes, CTAs);
- * pair_split < 0 marks a warp-per-system bucket with -pair_split atoms per lane */
+/* info[7] = (threads, pair_split, nsys, maxNA, maxNN, smem bytes, CTAs) */
 int mmff_bucket_info(int b, int* info);
 
 /* ------------------------------------------------------------ synthetic workloads */
