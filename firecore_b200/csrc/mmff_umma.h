@@ -46,9 +46,9 @@ constexpr int SM_X = SM_ONE + NOP * TILE * 2;     // X   [128 x 80]
 constexpr int SM_H1 = SM_X + TILE * K0 * 2;       // H1  [128 x 128]
 constexpr int SM_H2 = SM_H1 + TILE * HID * 2;     // H2, later dZ1
 constexpr int SM_S2 = SM_H2 + TILE * HID * 2;     // silu'(Z2), later dZ2
-constexpr int SM_S1 = SM_S2 + TILE * HID * 2;     // silu'(Z1)
-constexpr int SM_DY = SM_S1 + TILE * HID * 2;     // dY  [128 x 16]
-constexpr int SM_BIAS = SM_DY + TILE * NOP * 2;   // b1[128] b2[128] b3[16] (fp32)
+constexpr int SM_DY = SM_S2 + TILE * HID * 2;     // dY  [128 x 16]
+constexpr int SM_S1 = SM_DY + TILE * NOP * 2;     // silu'(Z1), no operand of a product
+constexpr int SM_BIAS = SM_S1 + TILE * HID * 2;   // b1[128] b2[128] b3[16] (fp32)
 constexpr int SM_MISC = SM_BIAS + (2 * HID + NOP) * 4;
 constexpr int SM_TOTAL = SM_MISC + 64;            // + mbarrier, TMEM base
 constexpr int SM_ALLOC = SM_TOTAL + 1024;         // slack for the 1024-B alignment
