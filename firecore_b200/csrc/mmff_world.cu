@@ -7,6 +7,7 @@
 // parameters to the FP32 layout the kernels read, groups systems into size
 // buckets and launches one persistent relaxation kernel per bucket.
 #include <cuda_runtime.h>
+#include <omp.h>
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -343,6 +344,64 @@ void default_config(int cls, int maxNA, int nsys, int& T, int& S) {
     if (W.force_S) S = W.force_S;
 }
 
+constexpr int kParallelAtoms = 8192;
+[[maybe_unused]] int host_threads(int atoms) { return std::max(1, std::min(std::min(16, omp_get_max_threads()), atoms / kParallelAtoms)); }
+
+// Page-locked host staging for the per-call state copies (positions and
+// velocities in, state, forces out), so the transfers run at full PCIe/C2C rate.
+// The FP64 <-> FP32 conversions between the caller's arrays and the staging run
+// on one host core per kParallelAtoms atoms, 16 at most (fewer atoms per core
+// and the threads' start costs more than they save): one core took 1.1 ms for the positions
+// of 2048 molecules (270k vectors) in and 2.0 ms for their forces out, longer
+// than the evaluation itself (0.4 ms).
+struct PinnedBuf {
+    float4* p = nullptr; size_t n = 0;
+    int ensure(size_t cnt) {
+        if (cnt <= n && p) return 0;
+        if (p) cudaFreeHost(p);
+        p = nullptr; n = 0;
+        if (cudaHostAlloc(reinterpret_cast<void**>(&p), cnt * sizeof(float4), cudaHostAllocDefault) != cudaSuccess)
+            return fail("cudaHostAlloc(%zu B) failed", cnt * sizeof(float4));
+        n = cnt;
+        return 0;
+    }
+};
+PinnedBuf g_stage_a, g_stage_b;
+
+// n doubles from the device into a caller's array.  From 32 MB on in pieces of
+// 16 MB through the two staging buffers: one is filled while the host cores copy
+// the other out (a fresh array's pages are first touched there, by all of them).
+// A whole grid build with its coefficients, plain copy / this: 15 MB 15.2 / 16.9
+// ms, 31 MB 20.7 / 20.9, 72 MB 43 / 33, 123 MB 82 / 47, 245 MB 130 / 91.
+constexpr size_t kStagedCopyBytes = (size_t)32 << 20;
+int copy_out(double* dst, const double* src, size_t n) {
+    if (n * sizeof(double) < kStagedCopyBytes) {
+        CK(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToHost, W.stream));
+        return 0;
+    }
+    const size_t piece = (size_t)2 << 20;
+    if (g_stage_a.ensure(piece / 2) || g_stage_b.ensure(piece / 2)) return -1;
+    double* st[2] = {reinterpret_cast<double*>(g_stage_a.p), reinterpret_cast<double*>(g_stage_b.p)};
+    auto start = [&](size_t o, int b) {
+        return cudaMemcpyAsync(st[b], src + o, std::min(piece, n - o) * sizeof(double), cudaMemcpyDeviceToHost, W.stream);
+    };
+    CK(start(0, 0));
+    int b = 0;
+    for (size_t o = 0; o < n; o += piece, b ^= 1) {
+        CK(cudaStreamSynchronize(W.stream));
+        if (o + piece < n) CK(start(o + piece, b ^ 1));
+        const size_t m = std::min(piece, n - o);
+        const double* s = st[b];
+        const long nb = (long)((m + 8191) / 8192);
+#pragma omp parallel for schedule(static) num_threads(host_threads((int)(m / 4)))
+        for (long k = 0; k < nb; k++) {
+            const size_t a = (size_t)k * 8192;
+            memcpy(dst + o + a, s + a, std::min((size_t)8192, m - a) * sizeof(double));
+        }
+    }
+    return 0;
+}
+
 template <class X> int upload(DBuf<X>& d, const std::vector<X>& h) {
     if (d.ensure(h.size())) return -1;
     if (!h.empty()) CK(cudaMemcpyAsync(d.p, h.data(), h.size() * sizeof(X), cudaMemcpyHostToDevice, W.stream));
@@ -405,6 +464,7 @@ int build_xmask() {
     for (int s = 0; s < W.nsys; s++) { moff[s] = (int)tot; tot += (size_t)W.natoms[s] * ((W.natoms[s] + 31) / 32); }
     if (tot > (size_t)INT32_MAX) return fail("exclusion rows too large (%zu words)", tot);
     std::vector<uint32_t> m(tot, 0u);
+#pragma omp parallel for schedule(dynamic, 16) num_threads(host_threads(W.NA))
     for (int s = 0; s < W.nsys; s++) {
         const int na = W.natoms[s], nn = W.nnode[s], a0 = W.desc[s].x, n0 = W.desc[s].y, nb = (na + 31) / 32;
         uint32_t* row = m.data() + moff[s];
@@ -433,8 +493,12 @@ int build_xmask() {
 }
 
 int build_buckets() {
-    for (auto& B : W.buckets) { B.queue.release(); B.vl.release(); }
-    W.buckets.clear();
+    // the queues and list scratch of the last buckets serve the new ones (every
+    // launch that uses them has ended), the rest is given back below
+    CK(cudaStreamSynchronize(W.stream));
+    std::vector<Bucket> old;
+    old.swap(W.buckets);
+    struct GiveBack { std::vector<Bucket>& v; ~GiveBack() { for (auto& B : v) { B.queue.release(); B.vl.release(); } } } give{old};
     W.graph_valid = false;
     std::vector<std::vector<int>> groups(6);
     for (int s = 0; s < W.nsys; s++) groups[size_class(W.natoms[s])].push_back(s);
@@ -446,11 +510,15 @@ int build_buckets() {
         std::stable_sort(B.sys.begin(), B.sys.end(), [](int a, int b) { return W.natoms[a] > W.natoms[b]; });
         int maxNA = 0;
         for (int s : B.sys) maxNA = std::max(maxNA, W.natoms[s]);
+        if (W.buckets.size() < old.size()) {
+            std::swap(B.queue, old[W.buckets.size()].queue);
+            std::swap(B.vl, old[W.buckets.size()].vl);
+        }
         int T, S;
         default_config(k, maxNA, (int)B.sys.size(), T, S);
         const Tune& tu = W.tune[k];
         if (tu.kind >= 0 && !W.force_T && !W.force_S) { T = tuned_threads(tu); S = tu.S; }
-        if (config_bucket(B, T, S)) return -1;
+        if (config_bucket(B, T, S)) { B.queue.release(); B.vl.release(); return -1; }
         B.cls = k;
         W.buckets.push_back(std::move(B));
     }
@@ -462,23 +530,6 @@ int build_buckets() {
     W.buckets_dirty = false;
     return 0;
 }
-
-// Page-locked host staging for the per-call state copies (positions and
-// velocities in, state out), so the transfers run at full PCIe/C2C rate.
-struct PinnedBuf {
-    float4* p = nullptr; size_t n = 0;
-    int ensure(size_t cnt) {
-        if (cnt <= n && p) return 0;
-        if (p) cudaFreeHost(p);
-        p = nullptr; n = 0;
-        if (cudaHostAlloc(reinterpret_cast<void**>(&p), cnt * sizeof(float4), cudaHostAllocDefault) != cudaSuccess)
-            return fail("cudaHostAlloc(%zu B) failed", cnt * sizeof(float4));
-        n = cnt;
-        return 0;
-    }
-};
-PinnedBuf g_stage_a, g_stage_b;
-
 
 // the bucket's pair-list scratch into the launch parameters (CTA relax kernels)
 void set_lists(Params& P, const Bucket& B) {
@@ -810,7 +861,7 @@ int mmff_grid_build(int nsub, const double* spos, const double* sREQ, const doub
     if (W.grid.ensure(ntot)) return -1;
     pack_grid_kernel<<<(unsigned)((ntot + 255) / 256), 256, 0, W.stream>>>(ntot, V.p, W.grid.p);
     CK(cudaGetLastError());
-    if (coefs_out) CK(cudaMemcpyAsync(coefs_out, V.p, 3 * ntot * sizeof(double), cudaMemcpyDeviceToHost, W.stream));
+    if (coefs_out && copy_out(coefs_out, V.p, 3 * ntot)) return -1;
     if (clear_grid_cache()) return -1;
     CK(cudaStreamSynchronize(W.stream));
     W.gn[0] = nx; W.gn[1] = ny; W.gn[2] = nz;
@@ -853,6 +904,7 @@ int mmff_systems_upload(int nsys, const int* natoms, const int* nnode, const dou
     std::vector<float> hlv(9 * nsys);
     std::vector<double4> hfire(nsys);
     const double sqk = std::sqrt(14.3996448915);
+#pragma omp parallel for schedule(dynamic, 16) num_threads(host_threads(NA))
     for (int s = 0; s < nsys; s++) {
         const int a0 = W.desc[s].x, n0 = W.desc[s].y, v0 = W.desc[s].z, na = natoms[s], nn = nnode[s];
         double c[3] = {0, 0, 0};
@@ -1012,9 +1064,10 @@ int mmff_systems_restore(void) {
 int mmff_systems_set_state(const double* pos, const double* vel, int reset_fire) {
     if (ensure_ready()) return -1;
     if (!W.nsys) return fail("no systems uploaded");
-    if (g_stage_a.ensure(W.NV) || g_stage_b.ensure(W.NV)) return -1;
+    if (g_stage_a.ensure(W.NV) || (vel && g_stage_b.ensure(W.NV))) return -1;
     float4* hpos = g_stage_a.p;
     float4* hvel = g_stage_b.p;
+#pragma omp parallel for schedule(static) num_threads(host_threads(W.NA))
     for (int s = 0; s < W.nsys; s++) {
         const int v0 = W.desc[s].z, na = W.natoms[s], nn = W.nnode[s];
         const double* c = W.orig.data() + 3 * s;
@@ -1022,12 +1075,15 @@ int mmff_systems_set_state(const double* pos, const double* vel, int reset_fire)
             const double* p = pos + 3 * (v0 + i);
             hpos[v0 + i] = (i < na) ? make_float4((float)(p[0] - c[0]), (float)(p[1] - c[1]), (float)(p[2] - c[2]), 0.f)
                                     : make_float4((float)p[0], (float)p[1], (float)p[2], 0.f);
-            const double* v = vel ? vel + 3 * (v0 + i) : nullptr;
-            hvel[v0 + i] = v ? make_float4((float)v[0], (float)v[1], (float)v[2], 0.f) : make_float4(0, 0, 0, 0);
+            if (vel) {
+                const double* v = vel + 3 * (v0 + i);
+                hvel[v0 + i] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.f);
+            }
         }
     }
     CK(cudaMemcpyAsync(W.d_pos.p, hpos, W.NV * sizeof(float4), cudaMemcpyHostToDevice, W.stream));
-    CK(cudaMemcpyAsync(W.d_vel.p, hvel, W.NV * sizeof(float4), cudaMemcpyHostToDevice, W.stream));
+    if (vel) CK(cudaMemcpyAsync(W.d_vel.p, hvel, W.NV * sizeof(float4), cudaMemcpyHostToDevice, W.stream));
+    else CK(cudaMemsetAsync(W.d_vel.p, 0, W.NV * sizeof(float4), W.stream));
     if (reset_fire) {
         std::vector<double4> hf(W.nsys, make_double4(W.fire[0], W.fire[2], 0.0, 0.0));
         CK(cudaMemcpyAsync(W.d_fire.p, hf.data(), W.nsys * sizeof(double4), cudaMemcpyHostToDevice, W.stream));
@@ -1344,8 +1400,11 @@ int mmff_set_tuning(int cls, int kind, int apl, int T, int S) {
 
 int mmff_get_forces(double* force) {
     if (mmff_sync()) return -1;
-    std::vector<float4> h(W.NV);
-    CK(cudaMemcpy(h.data(), W.d_force.p, W.NV * sizeof(float4), cudaMemcpyDeviceToHost));
+    if (g_stage_a.ensure(W.NV)) return -1;
+    CK(cudaMemcpyAsync(g_stage_a.p, W.d_force.p, W.NV * sizeof(float4), cudaMemcpyDeviceToHost, W.stream));
+    CK(cudaStreamSynchronize(W.stream));
+    const float4* h = g_stage_a.p;
+#pragma omp parallel for schedule(static) num_threads(host_threads(W.NA))
     for (int i = 0; i < W.NV; i++) { force[3 * i] = h[i].x; force[3 * i + 1] = h[i].y; force[3 * i + 2] = h[i].z; }
     return 0;
 }
@@ -1365,6 +1424,7 @@ int mmff_get_state(double* pos, double* vel, double* fire, int* status, int* nst
         CK(cudaMemcpyAsync(g_stage_a.p, W.d_pos.p, W.NV * sizeof(float4), cudaMemcpyDeviceToHost, W.stream));
         if (vel) CK(cudaMemcpyAsync(g_stage_b.p, W.d_vel.p, W.NV * sizeof(float4), cudaMemcpyDeviceToHost, W.stream));
         CK(cudaStreamSynchronize(W.stream));
+#pragma omp parallel for schedule(static) num_threads(host_threads(W.NA))
         for (int s = 0; s < W.nsys; s++) {
             const int v0 = W.desc[s].z, na = W.natoms[s], nn = W.nnode[s];
             const double* c = W.orig.data() + 3 * s;
