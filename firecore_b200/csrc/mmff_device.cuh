@@ -182,6 +182,14 @@ __device__ __forceinline__ float rsq_nr(float x) {
     return fmaf(0.5f * y, e, y);
 }
 
+// sqrt(x) from y ~ 1 / sqrt(x): Heron's step on x y, half a unit in the last
+// place.  Bond lengths and half-angle cosines enter as differences from their
+// rest values, times stiffnesses of some 30 eV/A^2.
+__device__ __forceinline__ float sqrt_from(float x, float y) {
+    const float s = x * y;
+    return fmaf(fmaf(-s, s, x), 0.5f * y, s);
+}
+
 // image index c (NBFF.h:42 ordering: x fastest, then y, then z) -> shift
 // in lattice units.  Quotients by the small image counts go through a float
 // reciprocal: (c + 1/2) / n stays >= 1/(2n) away from an integer, far beyond
@@ -203,7 +211,7 @@ __device__ __forceinline__ int wrap_index(int i, int n) {
 // Q = k_e*Qi*Qj.  Returns the scalar F with f = dp * F (the reference's -F).
 template <bool ENERGY>
 __device__ __forceinline__ float ljqh(float r2, float R0, float E0, float Q, float hw, float& E) {
-    const float ir = rsqrtf(r2);
+    const float ir = rsq(r2);
     const float ir2 = ir * ir;
     const float Eel = Q * ir;
     const float u2 = R0 * R0 * ir2;
@@ -229,7 +237,7 @@ __device__ __forceinline__ float pair13(float r2, float4 Ri, float4 Rj, bool x13
                                         float& e, float& ep) {
     const float R0 = Ri.x + Rj.x, E0 = Ri.y * Rj.y, Q = Ri.z * Rj.z, hw = fminf(Ri.w * Rj.w, 0.f);
     if (x13 && r2 < Rc2) {
-        const float ir = rsqrtf(r2);
+        const float ir = rsq(r2);
         if (ENERGY) {
             float eL;
             ljqh<true>(r2, R0, E0, Q, hw, eL);
@@ -255,7 +263,7 @@ __device__ __forceinline__ float pair_force(float dx, float dy, float dz, float4
     float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
     ok = !excl && (r2 < Rc2);
     r2 = ok ? r2 : 1e30f;
-    const float ir = rsqrtf(r2);
+    const float ir = rsq(r2);
     const float ir2 = ir * ir;
     const float R0 = Ri.x + Rj.x;
     const float E0 = Ri.y * Rj.y;
@@ -764,8 +772,9 @@ constexpr int kImageTileMinThreads = 128;
 constexpr int kListMaxImages = 12;
 constexpr int kListEntriesPerAtom = 96;
 
-__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, bool relax, int lvl) {
+__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, int mode, int lvl) {
     SmemLayout L;
+    const bool relax = mode > 0;
     L.maxNA = maxNA; L.maxNN = maxNN; L.maxNV = maxNA + maxNN; L.nwarps = T / 32;
     L.nimg = nimg; L.nwords = (maxNA + 31) / 32;
     int o = 0;
@@ -804,7 +813,7 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
         o = o_keep;
         if (need > fng_bytes) { L.cwords += o - L.fng; L.cpref += o - L.fng; L.ccnt += o - L.fng; L.clist += o - L.fng; take(need); }
     }
-    L.facc = take(8 * 3 * maxNA);
+    L.facc = take(8 * 3 * maxNA * (mode == 2 ? 2 : 1));
     // image tiles (blocks >= kImageTileMinThreads with candidate lists): the
     // positions and parameters of a tile's 32 candidates j, copied once per
     // tile so that the 32 rotation steps read them directly instead of through
@@ -821,16 +830,18 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
     return L;
 }
 
-// nimg: shifted images that get candidate lists (0: none).  Level 0: all in
+// nimg: shifted images that get candidate lists (0: none).  mode 0: evaluation,
+// 1: relaxation, 2: relaxation by a cluster of CTAs per system (two sets of
+// force sums).  Level 0: all in
 // shared memory; 1: topology and node parameters in global memory (above);
 // 2 (relaxation, when level 1 exceeds the CTA's limit): the velocities too,
 // which only the thread that owns a vector reads and writes.
 constexpr int kSmemMax = 227 * 1024;
-__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg, bool relax) {
-    SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, relax, 0);
+__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg, int mode) {
+    SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, mode, 0);
     if (T >= kCompactMinThreads && L.total > kCompactAbove) {
-        L = smem_layout_(maxNA, maxNN, T, nimg, relax, 1);
-        if (relax && L.total > kSmemMax) L = smem_layout_(maxNA, maxNN, T, nimg, relax, 2);
+        L = smem_layout_(maxNA, maxNN, T, nimg, mode, 1);
+        if (mode == 1 && L.total > kSmemMax) L = smem_layout_(maxNA, maxNN, T, nimg, mode, 2);
     }
     return L;
 }

@@ -50,7 +50,7 @@ struct Engine : CtaSystem<T> {
             const bool ex = (j == e0) | (j == e1) | (j == e2) | (j == e3) | (j == e4);
             const bool ok = !ex && (r2 < Rc2);
             r2 = ok ? r2 : 1e30f;
-            const float ir = rsqrtf(r2);
+            const float ir = rsq(r2);
             const float ir2 = ir * ir;
             const float R0 = Ri.x + Rj.x;
             const float E0 = Ri.y * Rj.y;

@@ -3,7 +3,7 @@
 // The system's whole state (positions, velocities, topology, force-field
 // parameters, recoil slots) is staged in shared memory, and every FIRE step
 // runs inside the CTA with three block barriers:
-//   forces   bonded terms (thread per node), GridFF samples (4 lanes per atom),
+//   forces   bonded terms (4 lanes per node), GridFF samples (4 lanes per atom),
 //            ordered pairs of the central image (and, without a cutoff, of
 //            every image), the listed pairs of the shifted images
 //   | barrier |
@@ -24,10 +24,12 @@
 // parameter (constant bank) instead of registers.  Time per system-step with
 // the chip full, the kernel before (ordered thread-per-node bonded terms,
 // 32 x 32 Newton-3 tiles with shuffled reactions, lists in runs per thread) and
-// this one: 60 atoms 0.0224 -> 0.0176 us, 100: 0.0566 -> 0.0337, 200: 0.136 ->
-// 0.102, 330: 0.286 -> 0.238; 127 atoms without a cutoff (9 images), 300
-// systems: 0.380 -> 0.266 us.
+// this one: 28 atoms 0.0087 -> 0.0059 us, 60: 0.0224 -> 0.0173, 100: 0.0566 ->
+// 0.0317, 200: 0.136 -> 0.094, 330: 0.286 -> 0.222; 127 atoms without a cutoff
+// (9 images), 300 systems: 0.380 -> 0.268 us.
 #include "mmff_engine.cuh"
+
+#include <cooperative_groups.h>
 
 namespace mmff {
 
@@ -44,12 +46,12 @@ __device__ __forceinline__ float hsum2(f32x2 v) { float a, b; unpack2(v, a, b); 
 struct PairJ { f32x2 x, y, z, R, E, Q, H; };
 // one atom i (shift - position, so that d = p_j + shift - p_i is one addition), in both halves
 struct PairI { f32x2 x, y, z, R, E, Q, H; };
-struct PairC { f32x2 kq, one, mone; float Rc2; };
+struct PairC { f32x2 kq, mone, p12, m12; float Rc2; };
 
 // Two ordered pairs: force on i into (fx, fy, fz).  getLJQH (Forces.h:341-360)
 // plus the shifted-force Coulomb part, as
 //   F = 12 E0 u6 (1 - u6 (1 + H)) / r^2 + Q (kq - 1/r^2) / r,  f_i += d F
-// (E of i holds 12 sqrt(E0)).  Excluded and out-of-range pairs are evaluated
+// Excluded and out-of-range pairs are evaluated
 // at r^2 = 1e30, where every term underflows to zero except kq Q / r
 // (< 1e-16 eV/A).  bits 0, 1 of m: pair excluded.
 template <bool HB, bool COUNT>
@@ -68,13 +70,13 @@ __device__ __forceinline__ void pair2(const PairJ& j, const PairI& i, const Pair
     const f32x2 w = mul2(add2(j.R, i.R), ir);
     const f32x2 u2 = mul2(w, w);
     const f32x2 u6 = mul2(mul2(u2, u2), u2);
-    f32x2 h = c.mone;
+    f32x2 h = c.m12;
     if (HB) {
         float h0, h1;
         unpack2(mul2(j.H, i.H), h0, h1);
-        h = pack2(-1.f - fminf(h0, 0.f), -1.f - fminf(h1, 0.f));
+        h = pack2(fmaf(-12.f, fminf(h0, 0.f), -12.f), fmaf(-12.f, fminf(h1, 0.f), -12.f));
     }
-    const f32x2 t = mul2(mul2(u6, fma2(u6, h, c.one)), ir2);
+    const f32x2 t = mul2(mul2(u6, fma2(u6, h, c.p12)), ir2);
     const f32x2 q = mul2(fma2(ir2, c.mone, c.kq), ir);
     const f32x2 F = fma2(t, mul2(i.E, j.E), mul2(q, mul2(i.Q, j.Q)));
     fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
@@ -95,7 +97,17 @@ __device__ __forceinline__ double length_ratio(double vv, double ff) {
     return vv > 0.0 ? sqrt(vv) / (sqrt(ff) + 1e-32) : 0.0;
 }
 
-template <int T, bool COUNT>
+// CL: a cluster of CTAs relaxes one system (batches with fewer systems than half
+// the SMs).  Every CTA holds the whole system and runs every step; each takes a
+// share of the pairs, list rows and GridFF samples into its own fixed-point
+// sums, and assemble adds the sums of all of them through distributed shared
+// memory.  Integer sums are exact, so all CTAs get the same bits, and with the
+// same code on the same bits they take every decision alike: the cluster barrier
+// after the forces is the only one of a step.  Two sets of sums alternate, so
+// that the next step's adds never meet a neighbour that still reads.  Whatever
+// one CTA alone could see (a non-finite pair force, a full list slot) is
+// exchanged before it decides anything.
+template <int T, bool COUNT, bool CL = false>
 struct RelaxEngine : CtaSystem<T> {
     using B = CtaSystem<T>;
     using B::P; using B::Y; using B::L; using B::tid; using B::lane; using B::warp;
@@ -110,8 +122,33 @@ struct RelaxEngine : CtaSystem<T> {
     // (a scratch slot, no overflow so far), built and valid, entries
     bool listok = false, listed = false;
     int nlist = 0, nrows = 0;
+    int cr = 0, cn = 1, par = 0;       // CL: rank in the cluster, its size, which set of sums this step uses
 
-    __device__ RelaxEngine(const Params& p, const Systems& y, char* smem, const SmemLayout& l) : B(p, y, smem, l) {}
+    __device__ RelaxEngine(const Params& p, const Systems& y, char* smem, const SmemLayout& l) : B(p, y, smem, l) {
+        if constexpr (CL) {
+            cr = (int)cooperative_groups::this_cluster().block_rank();
+            cn = (int)cooperative_groups::this_cluster().num_blocks();
+        }
+    }
+    // barrier of everything that works on the system
+    static __device__ __forceinline__ void csync() {
+        if constexpr (CL) cooperative_groups::this_cluster().sync();
+        else __syncthreads();
+    }
+    // this step's force sums
+    __device__ __forceinline__ long long* sums() { return at<long long>(L.facc) + (CL ? par * 3 * L.maxNA : 0); }
+    // flags of this CTA that the others read: [0, 1] non-finite pair force (per set of sums), [2] list slot full
+    __device__ __forceinline__ int* flags_cl() const {
+        __shared__ int f[4];
+        return f;
+    }
+    // some CTA of the cluster set flag k
+    __device__ __forceinline__ bool any_cl(int k) const {
+        int a = 0;
+        if constexpr (CL)
+            for (int c = 0; c < cn; c++) a |= cooperative_groups::this_cluster().map_shared_rank(flags_cl(), c)[k];
+        return a != 0;
+    }
 
     // arrays of the pair loops, NP atoms each
     __device__ __forceinline__ int np() const { return 32 * L.nwords; }
@@ -141,6 +178,11 @@ struct RelaxEngine : CtaSystem<T> {
         }
         long long* facc = at<long long>(L.facc);
         for (int a = tid; a < 3 * natoms; a += T) facc[a] = 0;
+        if constexpr (CL) {
+            par = 0;
+            for (int a = tid; a < 3 * natoms; a += T) facc[3 * L.maxNA + a] = 0;
+            if (tid < 4) flags_cl()[tid] = 0;
+        }
     }
 
     // ---- ordered pairs (i, j + shift), every atom i of the central image -----
@@ -160,8 +202,9 @@ struct RelaxEngine : CtaSystem<T> {
         const int nim = all_images ? (2 * P.npbc[0] + 1) * (2 * P.npbc[1] + 1) * (2 * P.npbc[2] + 1) : 1;
         const int c8 = (natoms + 7) >> 3, lg = last_lg(), cl = (c8 + (1 << lg) - 1) >> lg;
         const int total = ((nbw - 1) * c8 + cl) * nim;
-        const int q = (int)((long long)total * warp / NW);
-        plen = (int)((long long)total * (warp + 1) / NW) - q;
+        const int w = cr * NW + warp, nw = cn * NW;
+        const int q = (int)((long long)total * w / nw);
+        plen = (int)((long long)total * (w + 1) / nw) - q;
         pb0 = min(q / (c8 * nim), nbw - 1);
         pr0 = q - pb0 * c8 * nim;
     }
@@ -175,7 +218,7 @@ struct RelaxEngine : CtaSystem<T> {
         PairC C;
         const bool cut = P.Rc2 > 0.f;
         C.Rc2 = cut ? P.Rc2 : 3.0e38f;
-        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.one = pack2(1.f, 1.f); C.mone = pack2(-1.f, -1.f);
+        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.mone = pack2(-1.f, -1.f); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
         const float *X = soa(0), *Yy = soa(1), *Z = soa(2), *R = soa(3), *E = soa(4), *Q = soa(5), *H = soa(6);
         int b = pb0, r = pr0, left = plen;                   // r: position inside the block's images x chunks
         while (left > 0) {
@@ -188,8 +231,7 @@ struct RelaxEngine : CtaSystem<T> {
             const int ic = vi ? i : natoms - 1;
             const float ix = X[ic], iy = Yy[ic], iz = Z[ic];
             PairI I;
-            I.R = pack2(R[ic], R[ic]); I.Q = pack2(Q[ic], Q[ic]); I.H = HB ? pack2(H[ic], H[ic]) : 0;
-            { const float e = 12.f * E[ic]; I.E = pack2(e, e); }
+            I.R = pack2(R[ic], R[ic]); I.E = pack2(E[ic], E[ic]); I.Q = pack2(Q[ic], Q[ic]); I.H = HB ? pack2(H[ic], H[ic]) : 0;
             const uint8_t* row = reinterpret_cast<const uint8_t*>(xrow + ic * nbw);     // byte c: chunk c of 8 atoms j
             f32x2 fx = 0, fy = 0, fz = 0;
             while (r < rend) {
@@ -244,8 +286,8 @@ struct RelaxEngine : CtaSystem<T> {
                 f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
             }
             if (all_images) {
-                // atoms on top of an image (no force clamps of old here): scaled
-                // to the accumulators' range as a vector, its direction kept
+                // an atom on top of an image: the force is scaled to the
+                // accumulators' range as a vector, so that its direction stays
                 const float m = fmaxf(fabsf(f.x), fmaxf(fabsf(f.y), fabsf(f.z)));
                 if (m > B::kFixMax && isfinite(m)) f = f * (B::kFixMax / m);
             }
@@ -282,7 +324,7 @@ struct RelaxEngine : CtaSystem<T> {
         const unsigned short* clist = at<unsigned short>(L.clist);
         int nrows = 0;
         for (int k = 0; k < L.nimg; k++) nrows += ccnt[L.nimg - 1 - k];
-        for (int u = tid; u < nrows; u += T) {
+        for (int u = cr * T + tid; u < nrows; u += cn * T) {
             int c = u, k = 0;
             while (c >= ccnt[L.nimg - 1 - k]) { c -= ccnt[L.nimg - 1 - k]; k++; }
             const int i = clist[(L.nimg - 1 - k) * L.maxNA + c];
@@ -354,40 +396,48 @@ struct RelaxEngine : CtaSystem<T> {
         if (!any) return true;
         build_candidates(Rv2);
         int* rst = at<int>(L.rst);
-        for (int i = warp; i < natoms; i += NW) {            // count
+        for (int i = warp; i < natoms; i += NW) {            // count (CL: the rows of atoms i = cr mod cn)
             int c = 0;
-            row_pass(i, spos, Rv2, [&](bool in, int) { c += __popc(__ballot_sync(0xffffffffu, in)); });
+            if (!CL || i % cn == cr) row_pass(i, spos, Rv2, [&](bool in, int) { c += __popc(__ballot_sync(0xffffffffu, in)); });
             if (lane == 0) rst[i] = c;
         }
         __syncthreads();
         if (warp == 0) {                                     // row starts
             int run = 0;
             for (int a0 = 0; a0 < natoms; a0 += 32) {
-                const int a = a0 + lane, c = a < natoms ? rst[a] : 0;
+                const int a = a0 + lane, ce = a < natoms ? rst[a] : 0;
+                const int c = (ce + 1) & ~1;                 // rows start at whole words
                 int incl = c;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const int t = __shfl_up_sync(0xffffffffu, incl, o);
                     if (lane >= o) incl += t;
                 }
-                if (a < natoms) rst[a] = run + incl - c;
+                if (a < natoms) rst[a] = 2 * (run + incl - c) + (ce & 1);
                 run += __shfl_sync(0xffffffffu, incl, 31);
             }
-            if (lane == 0) rst[natoms] = run;
+            if (lane == 0) rst[natoms] = 2 * run;
         }
         __syncthreads();
-        const int total = rst[natoms];
-        if (total > P.vcap) return false;
-        // rows by falling length: the four rows a warp evaluates at a time are
+        const int total = rst[natoms] >> 1;
+        bool full = total > P.vcap;
+        if constexpr (CL) {
+            if (tid == 0) flags_cl()[2] = full;
+            csync();
+            full = any_cl(2);
+            csync();
+        }
+        if (full) return false;
+        // rows by falling length: the rows a warp evaluates at a time are
         // alike (their longest sets the time), atoms without a row drop out
         unsigned short* perm = at<unsigned short>(L.perm);
         float4* flist = at<float4>(L.flist);
         for (int a = tid; a < natoms; a += T) {
-            const int n = rst[a + 1] - rst[a];
+            const int n = (rst[a + 1] >> 2) - (rst[a] >> 2);
             flist[a] = make_float4(0.f, 0.f, 0.f, 0.f);
             int rank = 0;
             for (int o = 0, p0 = 0; o < natoms; o++) {
-                const int p1 = rst[o + 1], m = p1 - p0;
+                const int p1 = rst[o + 1] >> 2, m = p1 - p0;
                 rank += (m > n) || (m == n && o < a);
                 p0 = p1;
             }
@@ -395,8 +445,8 @@ struct RelaxEngine : CtaSystem<T> {
         }
         unsigned short* ent = vslot();
         for (int i = warp; i < natoms; i += NW) {            // write
-            int at0 = rst[i];
-            if (rst[i + 1] == at0) continue;
+            int at0 = rst[i] >> 1;
+            if ((rst[i + 1] >> 1) == at0) continue;
             row_pass(i, spos, Rv2, [&](bool in, int w) {
                 const uint32_t bal = __ballot_sync(0xffffffffu, in);
                 if (in) ent[at0 + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)w;
@@ -408,54 +458,62 @@ struct RelaxEngine : CtaSystem<T> {
         int lo = 0, hi = natoms;                             // rows that are not empty
         while (lo < hi) {
             const int mid = (lo + hi) >> 1, a = perm[mid];
-            if (rst[a + 1] > rst[a]) lo = mid + 1; else hi = mid;
+            if ((rst[a + 1] >> 2) > (rst[a] >> 2)) lo = mid + 1; else hi = mid;
         }
         nrows = lo;
         return true;
     }
 
-    // the listed pairs: kRowLanes lanes per atom, two entries per lane and
-    // packed instruction; each atom's sum goes to flist (no atomics: the row
-    // is all of the atom's listed pairs).  The first entries of a group's next
-    // row are in flight while a row is evaluated.
+    // the listed pairs: kRowLanes lanes per atom, two entries (one word) per lane
+    // and packed operation; each atom's sum goes to flist (no atomics: the row is
+    // all of the atom's listed pairs).  The entries come from L2, several hundred
+    // cycles away: four words per lane are in flight ahead of the one evaluated,
+    // and a group's next row is fetched before it evaluates this one.
     static constexpr int kRowLanes = 8;
     template <bool HB>
-    __device__ void list_pairs(const float4* spos, const float4* sREQ) {
-        constexpr int G = kRowLanes, NG = T / G;
+    __device__ void list_pairs(const float4* spos, const float4* sREQ, long long* facc) {
+        constexpr int G = kRowLanes, NG = T / G, RW = 32 / G;      // lanes per row, rows of the block, of a warp
         const int* rst = at<int>(L.rst);
         float4* flist = at<float4>(L.flist);
         const float4* shf = at<float4>(L.shf);
-        const unsigned short* ent = vslot();
+        const uint32_t* ent = reinterpret_cast<const uint32_t*>(vslot());       // two entries a word
         const unsigned short* perm = at<unsigned short>(L.perm);
         const int gl = lane & (G - 1);
         PairC C;
         C.Rc2 = P.Rc2;
-        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.one = pack2(1.f, 1.f); C.mone = pack2(-1.f, -1.f);
-        auto first = [&](int row, int& i, int& a, int& n, unsigned& w0, unsigned& w1) {
-            i = row < nrows ? (int)perm[row] : 0;
-            a = rst[i];
-            n = row < nrows ? rst[i + 1] - a : 0;
-            w0 = w1 = 0;
-            if (2 * gl < n) { w0 = ent[a + 2 * gl]; w1 = ent[a + min(2 * gl + 1, n - 1)]; }
+        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.mone = pack2(-1.f, -1.f); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
+        // row: atom, words, whether the last word holds one entry, first word, and
+        // this lane's first four words
+        struct Row { int i, nw, odd; const uint32_t* p; uint32_t u[4]; };
+        auto fetch = [&](int row, Row& x) {
+            x.i = row < nrows ? (int)perm[row] : 0;
+            const int a = rst[x.i];
+            x.odd = a & 1;
+            x.nw = row < nrows ? (rst[x.i + 1] >> 2) - (a >> 2) : 0;
+            x.p = ent + (a >> 2) + gl;
+#pragma unroll
+            for (int t = 0; t < 4; t++) x.u[t] = G * t + gl < x.nw ? x.p[G * t] : 0u;
         };
-        int in, an, nn;
-        unsigned u0, u1;
-        first(tid / G, in, an, nn, u0, u1);
+        Row nx;
+        fetch(tid / G, nx);
         for (int i0 = 0, k = 0; i0 < nrows; i0 += NG, k++) {
-            const int i = in, a = an, n = nn;
-            unsigned w0 = u0, w1 = u1;
+            Row w = nx;
             // every other round the warps take their rows in reverse order
-            if (i0 + NG < nrows) first(i0 + NG + ((k & 1) ? tid / G : (NG - 4) - 4 * warp + (lane / G)), in, an, nn, u0, u1);
+            if (i0 + NG < nrows) fetch(i0 + NG + ((k & 1) ? tid / G : (NG - RW) - RW * warp + (lane / G)), nx);
+            const int i = w.i, n = w.nw;
             f32x2 fx = 0, fy = 0, fz = 0;
-            if (2 * gl < n) {
+            if (gl < n) {
                 const float4 pi = spos[i], Ri = sREQ[i];
                 PairI I;
                 I.x = I.y = I.z = 0;
-                I.R = pack2(Ri.x, Ri.x); I.Q = pack2(Ri.z, Ri.z); I.H = HB ? pack2(Ri.w, Ri.w) : 0;
-                { const float e = 12.f * Ri.y; I.E = pack2(e, e); }
-                for (int q = 2 * gl; q < n; q += 2 * G) {
-                    const unsigned c0 = w0, c1 = w1;
-                    if (q + 2 * G < n) { w0 = ent[a + q + 2 * G]; w1 = ent[a + min(q + 2 * G + 1, n - 1)]; }
+                I.R = pack2(Ri.x, Ri.x); I.E = pack2(Ri.y, Ri.y); I.Q = pack2(Ri.z, Ri.z); I.H = HB ? pack2(Ri.w, Ri.w) : 0;
+#pragma unroll 1
+                for (int t = gl; t < n; t += G) {
+                    const bool one = w.odd && t + 1 == n;                  // the word's second half is no entry
+                    const unsigned c0 = w.u[0] & 0xFFFFu, c1 = one ? c0 : w.u[0] >> 16;
+                    w.u[0] = w.u[1]; w.u[1] = w.u[2]; w.u[2] = w.u[3];
+                    w.p += G;
+                    if (t + 4 * G < n) w.u[3] = w.p[3 * G];
                     const float4 s0 = shf[c0 >> 12], s1 = shf[c1 >> 12];
                     const float4 p0 = spos[c0 & 0xFFFu], p1 = spos[c1 & 0xFFFu], R0 = sREQ[c0 & 0xFFFu], R1 = sREQ[c1 & 0xFFFu];
                     PairJ J;
@@ -463,7 +521,7 @@ struct RelaxEngine : CtaSystem<T> {
                     J.y = pack2(p0.y + s0.y - pi.y, p1.y + s1.y - pi.y);
                     J.z = pack2(p0.z + s0.z - pi.z, p1.z + s1.z - pi.z);
                     J.R = pack2(R0.x, R1.x); J.E = pack2(R0.y, R1.y); J.Q = pack2(R0.z, R1.z); J.H = HB ? pack2(R0.w, R1.w) : 0;
-                    pair2<HB, COUNT>(J, I, C, false, q + 1 >= n, fx, fy, fz, npair);
+                    pair2<HB, COUNT>(J, I, C, false, one, fx, fy, fz, npair);
                 }
             }
             float3 f = make_float3(hsum2(fx), hsum2(fy), hsum2(fz));
@@ -473,7 +531,9 @@ struct RelaxEngine : CtaSystem<T> {
                 f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
                 f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
             }
-            if (gl == 0 && n > 0) {
+            if (CL) {
+                if (gl == 0 && n > 0) fix_add(facc + 3 * i, f);
+            } else if (gl == 0 && n > 0) {
                 auto lim = [](float x) { return fminf(fmaxf(x, -B::kFixMax), B::kFixMax) + 0.f * x; };   // as fix_add; NaN stays
                 flist[i] = make_float4(lim(f.x), lim(f.y), lim(f.z), 0.f);
             }
@@ -521,7 +581,7 @@ struct RelaxEngine : CtaSystem<T> {
             }
             const float l2 = dot3(h, h);
             il = rsq_nr(l2);
-            l = l2 * il;
+            l = sqrt_from(l2, il);
             h = h * il;
             if (ia < ing) {
                 if (flags & F_BONDS) {
@@ -562,9 +622,10 @@ struct RelaxEngine : CtaSystem<T> {
                 const int jng = __shfl_sync(0xffffffffu, ing, src), jcell = __shfl_sync(0xffffffffu, cell, src);
                 if (!v || p >= nbn) continue;
                 const float3 hs = h + hp;                                 // evalAngleCosHalf
-                const float c2 = dot3(hs, hs) * 0.25f;
-                const float c = sqrtf(c2), s = sqrtf(fmaxf(1.f - c2 + 1e-14f, 0.f));
-                const float fr = il * __fdividef(-apar.z * fmaf(apar.y, c, -apar.x * s), 4.f * c * s);
+                // cos and sin of the half angle with their reciprocals (no division)
+                const float c2 = dot3(hs, hs) * 0.25f, s2 = fmaxf(1.f - c2 + 1e-14f, 0.f);
+                const float rc = rsq(c2), rs = rsq(s2);
+                const float fr = il * (-0.25f * apar.z * fmaf(apar.y, sqrt_from(c2, rc), -apar.x * sqrt_from(s2, rs)) * (rc * rs));
                 fb = fb + hs * fr + h * (fr * (-2.f * c2));
                 if (flags & F_SUB_ANGLE_NB) {
                     const float3 dp = hp * lp - h * l;
@@ -599,7 +660,7 @@ struct RelaxEngine : CtaSystem<T> {
     template <bool HB>
     __device__ __forceinline__ void pairs(bool pbc, long long* facc) {
         ordered_pairs<HB>(pbc && !(P.Rc2 > 0.f), facc);
-        if (nlist > 0) list_pairs<HB>(at<float4>(L.pos), at<float4>(L.REQ));
+        if (nlist > 0) list_pairs<HB>(at<float4>(L.pos), at<float4>(L.REQ), facc);
     }
 
     // moved: some atom moved more than half the list skin since the lists were
@@ -608,7 +669,7 @@ struct RelaxEngine : CtaSystem<T> {
         const int flags = P.flags;
         const float4* spos = at<float4>(L.pos);
         const bool pbc = (flags & F_PBC) != 0;
-        long long* facc = at<long long>(L.facc);
+        long long* facc = sums();
         if ((flags & F_NONBONDED) && P.Rc2 > 0.f && L.nimg > 0) {
             if (listok && (!listed || moved)) {
                 if (COUNT && tid == 0) atomicAdd(Y.counters + 3, 1ull);
@@ -642,9 +703,19 @@ struct RelaxEngine : CtaSystem<T> {
             bonded_node(min(ia, nnode - 1), ia < nnode);
         }
         double d0 = 0.0;
+        if constexpr (CL) {
 #pragma unroll 1
-        for (int u = (warp + NW - nB % NW) % NW; u < nG; u += NW)
-            B::template grid_phase<false, true>(32 * u + lane, 1 << 30, fgr, d0);
+            for (int u = cr + cn * warp; u < nG; u += cn * NW) {
+                B::template grid_phase<false, true>(32 * u + lane, 1 << 30, fgr, d0);
+                __syncwarp();
+                const int a = 8 * u + lane;
+                if (lane < 8 && a < natoms) fix_add(facc + 3 * a, f3(fgr[a]));
+            }
+        } else {
+#pragma unroll 1
+            for (int u = (warp + NW - nB % NW) % NW; u < nG; u += NW)
+                B::template grid_phase<false, true>(32 * u + lane, 1 << 30, fgr, d0);
+        }
         if (flags & F_NONBONDED) {
             if (hasH) pairs<true>(pbc, facc);
             else pairs<false>(pbc, facc);
@@ -656,10 +727,11 @@ struct RelaxEngine : CtaSystem<T> {
             for (int a = tid; a < natoms; a += T) {
                 const float4 p = spos[a];
                 const float4 r = surf_atom(P, make_float3(p.x + lv[9], p.y + lv[10], p.z + lv[11]), sR[a]);
-                const float4 g = (flags & F_GRID) ? fgr[a] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 g = (!CL && (flags & F_GRID)) ? fgr[a] : make_float4(0.f, 0.f, 0.f, 0.f);
                 fgr[a] = make_float4(g.x + r.x, g.y + r.y, g.z + r.z, 0.f);
             }
         }
+        if (CL && pairbad) flags_cl()[par] = 1;
     }
 
     // ---------------------------------------------------------------- assemble
@@ -667,7 +739,7 @@ struct RelaxEngine : CtaSystem<T> {
     // thread; the pair sums are read and cleared for the next step
     __device__ void assemble(double& vf, double& vv, double& ff, float& fmax2, bool& bad) {
         float4* fasm = at<float4>(L.fasm);
-        long long* facc = at<long long>(L.facc);
+        long long* facc = sums();
         const float4* fgr = at<float4>(L.fgrid);
         const float4* flist = at<float4>(L.flist);
         const float4* fng = at<float4>(L.fng);
@@ -680,12 +752,23 @@ struct RelaxEngine : CtaSystem<T> {
             float3 f = make_float3(0.f, 0.f, 0.f);
             if (pi || v < nnode) f = f3(fasm[v]);
             if (!pi) {
-                if (P.flags & (F_GRID | F_SURF)) f = f + f3(fgr[v]);
-                if (nlist > 0) f = f + f3(flist[v]);
-                f.x += (float)facc[3 * v] * (1.f / kFix);
-                f.y += (float)facc[3 * v + 1] * (1.f / kFix);
-                f.z += (float)facc[3 * v + 2] * (1.f / kFix);
-                facc[3 * v] = 0; facc[3 * v + 1] = 0; facc[3 * v + 2] = 0;
+                if (P.flags & (CL ? F_SURF : F_GRID | F_SURF)) f = f + f3(fgr[v]);
+                if (!CL && nlist > 0) f = f + f3(flist[v]);
+                long long s[3] = {0, 0, 0};
+                if constexpr (CL) {
+                    for (int c = 0; c < cn; c++) {
+                        const long long* q = cooperative_groups::this_cluster().map_shared_rank(facc, c) + 3 * v;
+                        s[0] += q[0]; s[1] += q[1]; s[2] += q[2];
+                    }
+                    long long* z = at<long long>(L.facc) + (par ^ 1) * 3 * L.maxNA + 3 * v;
+                    z[0] = 0; z[1] = 0; z[2] = 0;
+                } else {
+                    s[0] = facc[3 * v]; s[1] = facc[3 * v + 1]; s[2] = facc[3 * v + 2];
+                    facc[3 * v] = 0; facc[3 * v + 1] = 0; facc[3 * v + 2] = 0;
+                }
+                f.x += (float)s[0] * (1.f / kFix);
+                f.y += (float)s[1] * (1.f / kFix);
+                f.z += (float)s[2] * (1.f / kFix);
             }
             const int4 bk = bks(ia);
             const int bks[4] = {bk.x, bk.y, bk.z, bk.w};
@@ -715,7 +798,13 @@ struct RelaxEngine : CtaSystem<T> {
             fmax2 = fmaxf(fmax2, (float)f2);
             bad |= !isfinite(f.x + f.y + f.z);
         }
-        bad |= pairbad;
+        if constexpr (CL) {
+            bad |= any_cl(par);
+            if (tid == 0) flags_cl()[par ^ 1] = 0;
+            par ^= 1;
+        } else {
+            bad |= pairbad;
+        }
     }
 
     // block reduction of 3 doubles + one float max (+flag); result in all threads
@@ -850,15 +939,23 @@ template <int T> constexpr int relax_min_blocks() {
 
 // P.vlist (null: none): scratch for the shifted-image pair lists, P.vcap entries per CTA.
 // EXPL: the exploring cycle (P.md_mode 2) instead of plain FIRE or the drive.
-template <int T, bool COUNT, bool EXPL>
+template <int T, bool COUNT, bool EXPL, bool CL = false>
 __global__ void __launch_bounds__(T, relax_min_blocks<T>()) relax_kernel(const __grid_constant__ Params P, const __grid_constant__ Systems Y, const int* __restrict__ queue, int nqueue,
                                                   int* counter, const __grid_constant__ SmemLayout L) {
     extern __shared__ __align__(16) char smem[];
     __shared__ int s_claim;
-    RelaxEngine<T, COUNT> E(P, Y, smem, L);
+    RelaxEngine<T, COUNT, CL> E(P, Y, smem, L);
+    if constexpr (CL) E.csync();        // the whole cluster runs before anyone writes to a neighbour
     while (true) {
-        if (threadIdx.x == 0) s_claim = atomicAdd(counter, 1);
-        __syncthreads();
+        if constexpr (CL) {
+            if (E.cr == 0 && threadIdx.x == 0) {
+                const int c = atomicAdd(counter, 1);
+                for (int k = 0; k < E.cn; k++) *cooperative_groups::this_cluster().map_shared_rank(&s_claim, k) = c;
+            }
+        } else if (threadIdx.x == 0) {
+            s_claim = atomicAdd(counter, 1);
+        }
+        E.csync();
         const int q = s_claim;
         if (q >= nqueue) break;
         const int s = queue[q];
@@ -880,7 +977,7 @@ __global__ void __launch_bounds__(T, relax_min_blocks<T>()) relax_kernel(const _
                 if ((ev & 2) && threadIdx.x == 0) Y.gopt[s].w++;
             }
             E.forces(far);
-            __syncthreads();
+            E.csync();
             double vf = 0, vv = 0, ff = 0;
             float fmax2 = 0.f;
             bool bad = false;
@@ -927,6 +1024,7 @@ __global__ void __launch_bounds__(T, relax_min_blocks<T>()) relax_kernel(const _
         // converged at step itr-1 (reference returns the loop index at break)
         const int steps = (status == ST_CONVERGED) ? itr - 1 : itr;
         __syncthreads();
+        if (CL && E.cr != 0) { E.csync(); continue; }      // every CTA has the same state: the first writes it
         // (a system retired as not finite had no move in its last step)
         E.store_state(status, steps, (float)sqrt(meas2), dt, damping, lastNeg, fs.w + (double)itr);
         if (EXPL && threadIdx.x == 0) { Y.gopt[s].x = ph & 1; Y.gopt[s].y = ph >> 1; }
@@ -937,7 +1035,7 @@ __global__ void __launch_bounds__(T, relax_min_blocks<T>()) relax_kernel(const _
                 atomicAdd(Y.counters + 2, (unsigned long long)itr);
             }
         }
-        __syncthreads();
+        E.csync();
     }
     if (COUNT) atomicAdd(Y.counters, E.npair);
 }
@@ -950,6 +1048,15 @@ template <bool COUNT, bool EXPL> static void* relax_of(int T) {
         case 128: return (void*)relax_kernel<128, COUNT, EXPL>;
         case 256: return (void*)relax_kernel<256, COUNT, EXPL>;
         case 512: return (void*)relax_kernel<512, COUNT, EXPL>;
+        default: return nullptr;
+    }
+}
+// ... by a cluster of CTAs per system
+void* relax_cluster_fn(int T) {
+    switch (T) {
+        case 128: return (void*)relax_kernel<128, false, false, true>;
+        case 256: return (void*)relax_kernel<256, false, false, true>;
+        case 512: return (void*)relax_kernel<512, false, false, true>;
         default: return nullptr;
     }
 }

@@ -192,7 +192,7 @@ __device__ __forceinline__ void pair_image(const Params& P, int N, const float4*
             float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             const bool ok = (((j < 32 ? m0lo : m0hi) & b) == 0) && (r2 < Rc2);
             r2 = ok ? r2 : 1e30f;
-            const float ir = rsqrtf(r2);
+            const float ir = rsq(r2);
             const float ir2 = ir * ir;
             const float R0 = R0i.x + Rj.x;
             const float E0 = R0i.y * Rj.y;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void pair_image(const Params& P, int N, const float4*
             float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
             const bool ok = (((j < 32 ? m1lo : m1hi) & b) == 0) && (r2 < Rc2);
             r2 = ok ? r2 : 1e30f;
-            const float ir = rsqrtf(r2);
+            const float ir = rsq(r2);
             const float ir2 = ir * ir;
             const float R0 = R1i.x + Rj.x;
             const float E0 = R1i.y * Rj.y;

@@ -37,6 +37,7 @@ __global__ void pack_grid_kernel(long, const double*, float4*);
 void* relax_fn(int T, bool count);
 void* eval_fn(int T, int S, bool energy);
 void* relax_explore_fn(int T);
+void* relax_cluster_fn(int T);
 void* eval_warp_fn(int apl, bool energy);
 
 }  // namespace mmff
@@ -82,6 +83,8 @@ struct Bucket {
     // evaluation: eT threads and S lanes per atom per CTA, or (eapl > 0) a warp per system
     int eT = 0, eapl = 0, esmem = 0;
     SmemLayout lay, elay;          // CTA kernels: shared-memory layouts of relaxation and evaluation
+    int cn = 1;                    // relaxation by clusters of cn CTAs per system (> 1), with layout clay
+    SmemLayout clay;
     // CTA relax kernels with a cutoff and a 2-D cell: scratch for the shifted-image
     // pair lists, vcap entries per resident CTA (0: none)
     DBuf<unsigned short> vl;
@@ -279,6 +282,42 @@ int set_smem_limit(void* fn, int bytes) {
     return 0;
 }
 
+// A launch of fn over grid CTAs in clusters of cn
+struct ClusterLaunch {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t c;
+    ClusterLaunch(int grid, int T, int smem, int cn, cudaStream_t st) {
+        memset(&c, 0, sizeof c);
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cn; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        c.gridDim = dim3(grid); c.blockDim = dim3(T); c.dynamicSmemBytes = smem; c.stream = st;
+        c.attrs = at; c.numAttrs = 1;
+    }
+};
+
+// Clusters per system for a bucket: the largest cluster of which one per system
+// is resident at once, for systems whose pair work is worth the exchange of the
+// force sums (kClusterMinAtoms; measured below that the cluster barrier and the
+// remote reads cost as much as the shared work saves).  Only plain relaxations
+// use it (not the counting and exploring kernels, whose shapes stay).
+constexpr int kClusterMinAtoms = 64;
+int cluster_size(Bucket& B, int nimg, int dev_smem) {
+    B.cn = 1;
+    const int n = (int)B.sys.size();
+    void* fn = relax_cluster_fn(B.T);
+    if (W.force_T || !fn || B.maxNA <= kClusterMinAtoms || 2 * W.nsys > W.nsm) return 0;
+    B.clay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 2);
+    if (B.clay.total > dev_smem || B.clay.vel < 0) return 0;
+    if (set_smem_limit(fn, B.clay.total)) return -1;
+    for (int c = std::min(8, W.nsm / W.nsys); c >= 2; c--) {
+        ClusterLaunch l(c, B.T, B.clay.total, c, W.stream);
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, fn, &l.c) != cudaSuccess) { cudaGetLastError(); continue; }
+        if (active >= n) { B.cn = c; break; }
+    }
+    return 0;
+}
+
 // launch configuration of a bucket whose systems are set: T threads per system,
 // S lanes per atom on the image rows of the evaluation.  Fills layouts, sizes
 // and grid; sets kernel attributes.
@@ -290,10 +329,10 @@ int config_bucket(Bucket& B, int T, int S) {
     const int nimg = W.Rcut > 0 ? shifted_images(W.flags, W.npbc) : 0;
     void* fns[3];
     B.T = T; B.S = S;
-    B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
+    B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 1);
     if (B.lay.total > dev_smem && B.T < kCompactMinThreads) {     // only the larger blocks leave arrays in global memory
         B.T = kCompactMinThreads;
-        B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, true);
+        B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 1);
     }
     B.smem = B.lay.total;
     fns[0] = relax_fn(B.T, false); fns[1] = relax_fn(B.T, true); fns[2] = relax_explore_fn(B.T);
@@ -316,10 +355,11 @@ int config_bucket(Bucket& B, int T, int S) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[0], B.T, B.smem));
     if (occ < 1) return fail("kernel cannot be resident (T=%d smem=%d)", B.T, B.smem);
     B.grid = std::min((int)B.sys.size(), occ * W.nsm);
+    if (cluster_size(B, nimg, dev_smem)) return -1;
     B.vcap = 0;
     if (nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
-        B.vcap = B.maxNA * kListEntriesPerAtom;
-        if (B.vl.ensure((size_t)B.grid * B.vcap)) return -1;
+        B.vcap = B.maxNA * kListEntriesPerAtom;      // even: rows are read by words
+        if (B.vl.ensure((size_t)std::max(B.grid, B.cn > 1 ? (int)B.sys.size() * B.cn : 0) * B.vcap)) return -1;
     }
     if (B.queue.ensure(B.sys.size())) return -1;
     CK(cudaMemcpy(B.queue.p, B.sys.data(), B.sys.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -337,7 +377,9 @@ void default_config(int cls, int maxNA, int nsys, int& T, int& S) {
     S = cls <= 1 ? 1 : std::min(pow2_floor(std::max(1, kClassT[cls - 2] / std::max(1, maxNA))), 8);
     if (W.force_T) T = W.force_T;
     else {
-        const int cap = cls <= 1 ? 128 : cls == 3 ? 256 : 512;
+        // without a cutoff every image's pairs are evaluated: enough for more threads
+        const bool all = W.Rcut <= 0 && shifted_images(W.flags, W.npbc) > 0;
+        const int cap = cls == 0 ? (all ? 256 : 128) : cls == 1 ? 256 : cls == 3 && !all ? 256 : 512;
         const int per_sm = std::max(1, (nsys + W.nsm - 1) / W.nsm);
         T = std::max(T, std::min(cap, pow2_floor(std::max(1, 512 / per_sm))));
     }
@@ -556,8 +598,14 @@ int enqueue_relax(const Params& P) {
         int nq = (int)B.sys.size();
         int* ctr = W.d_counter.p + b;
         set_lists(Pc, B);
-        void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
-        CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
+        if (B.cn > 1 && P.md_mode != 2 && !W.count) {
+            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.clay};
+            ClusterLaunch l(nq * B.cn, B.T, B.clay.total, B.cn, st);
+            CK(cudaLaunchKernelExC(&l.c, relax_cluster_fn(B.T), args));
+        } else {
+            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
+            CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
+        }
         if (!g_capturing) g_launches++;
     }
     for (size_t b = 0; b < W.buckets.size(); b++) {

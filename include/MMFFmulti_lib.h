@@ -58,8 +58,10 @@ int mmff_set_fire(double dt_max, double dt_min, double damp_max, double finc, do
                   int minLastNeg, double cv_kill, double Flim, int variant);
 /* Threads per CTA (64/128/256/512) and lanes per atom in the pair sum
  * (1/2/4/8) of the CTA-per-system kernels; 0 = chosen per size bucket
- * (systems of <= 64 atoms then run one per warp).  A non-zero thread count
- * forces every system onto the CTA-per-system kernels. */
+ * (evaluations of large batches then run systems of <= 64 atoms one per warp,
+ * relaxations of a few large systems a cluster of CTAs per system).  A non-zero
+ * thread count forces one CTA per system; the lanes per atom apply to the
+ * evaluation kernels. */
 int mmff_set_launch(int threads, int pair_split);
 
 /* ------------------------------------------------------------ substrate grid */
