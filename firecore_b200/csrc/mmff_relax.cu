@@ -25,7 +25,7 @@
 // the chip full, the kernel before (ordered thread-per-node bonded terms,
 // 32 x 32 Newton-3 tiles with shuffled reactions, lists in runs per thread) and
 // this one: 28 atoms 0.0087 -> 0.0059 us, 60: 0.0224 -> 0.0173, 100: 0.0566 ->
-// 0.0317, 200: 0.136 -> 0.094, 330: 0.286 -> 0.222; 127 atoms without a cutoff
+// 0.0299, 200: 0.136 -> 0.091, 330: 0.286 -> 0.216; 127 atoms without a cutoff
 // (9 images), 300 systems: 0.380 -> 0.268 us.
 #include "mmff_engine.cuh"
 
@@ -468,8 +468,13 @@ struct RelaxEngine : CtaSystem<T> {
     // and packed operation; each atom's sum goes to flist (no atomics: the row is
     // all of the atom's listed pairs).  The entries come from L2, several hundred
     // cycles away: four words per lane are in flight ahead of the one evaluated,
-    // and a group's next row is fetched before it evaluates this one.
-    static constexpr int kRowLanes = 8;
+    // and a group's next row is fetched before it evaluates this one.  Rows hold
+    // 5 to 30 entries: with four lanes fewer of them idle at the row's end and
+    // each warp closes eight rows at once (time per system-step, eight -> four
+    // lanes: 100 atoms 0.0317 -> 0.0299 us, 200: 0.0942 -> 0.0906, 330: 0.2223 ->
+    // 0.2163, 395: 0.3008 -> 0.2933); a cluster's CTA has too few rows for that
+    // (350 atoms x 37: 0.604 with eight, 0.634 with four).
+    static constexpr int kRowLanes = CL ? 8 : 4;
     template <bool HB>
     __device__ void list_pairs(const float4* spos, const float4* sREQ, long long* facc) {
         constexpr int G = kRowLanes, NG = T / G, RW = 32 / G;      // lanes per row, rows of the block, of a warp
