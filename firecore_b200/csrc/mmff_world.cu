@@ -340,7 +340,12 @@ int config_bucket(Bucket& B, int T, int S) {
     B.eapl = B.maxNA <= 32 ? 1 : B.maxNA <= 64 ? 2 : 0;
     if (W.force_T) B.eapl = 0;
     B.eT = B.eapl ? 128 : T;
-    if (!B.eapl) B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, false);
+    if (B.eapl && W.nsys <= W.nsm) {                      // too few for a warp each to hide anything: a block each
+        B.eT = 256;
+        B.S = B.eapl == 1 ? 8 : 4;
+        B.eapl = 0;
+    }
+    if (!B.eapl) B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, 0);
     B.esmem = B.eapl ? 4 * warp_layout(B.maxNA, B.maxNN).per_warp : B.elay.total;
     if (B.smem > dev_smem || B.esmem > dev_smem)
         return fail("system too large for shared memory: %d B > %d B", std::max(B.smem, B.esmem), dev_smem);
@@ -1146,15 +1151,26 @@ int mmff_eval(int with_energy) {
     if (W.buckets_dirty && build_buckets()) return -1;
     Params P = make_params(true, 0, 0.0, 0);
     Systems Y = make_systems();
-    for (auto& B : W.buckets) {
+    // the buckets side by side, each on its stream: one evaluation is too short
+    // to fill the chip to its end bucket by bucket
+    const bool fork = W.buckets.size() > 1;
+    if (fork) CK(cudaEventRecord(W.evfork, W.stream));
+    for (size_t b = 0; b < W.buckets.size(); b++) {
+        Bucket& B = W.buckets[b];
+        cudaStream_t st = fork ? W.bstreams[b] : W.stream;
+        if (fork) CK(cudaStreamWaitEvent(st, W.evfork, 0));
         void* fn = B.eapl ? eval_warp_fn(B.eapl, with_energy != 0) : eval_fn(B.eT, B.S, with_energy != 0);
         const int* q = B.queue.p;
         int nq = (int)B.sys.size();
         int mna = B.maxNA, mnn = B.maxNN;
         void* args[] = {&P, &Y, &q, &nq, B.eapl ? (void*)&mna : (void*)&B.elay, &mnn};
         const int nblk = B.eapl ? (nq + 3) / 4 : nq;
-        CK(cudaLaunchKernel(fn, dim3(nblk), dim3(B.eT), args, B.esmem, W.stream));
+        CK(cudaLaunchKernel(fn, dim3(nblk), dim3(B.eT), args, B.esmem, st));
         g_launches++;
+        if (fork) {
+            CK(cudaEventRecord(W.bev[b], st));
+            CK(cudaStreamWaitEvent(W.stream, W.bev[b], 0));
+        }
     }
     CK(cudaGetLastError());
     return 0;
