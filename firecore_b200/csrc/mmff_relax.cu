@@ -46,11 +46,14 @@ __device__ __forceinline__ float hsum2(f32x2 v) { float a, b; unpack2(v, a, b); 
 struct PairJ { f32x2 x, y, z, R, E, Q, H; };
 // one atom i (shift - position, so that d = p_j + shift - p_i is one addition), in both halves
 struct PairI { f32x2 x, y, z, R, E, Q, H; };
-struct PairC { f32x2 kq, mone, p12, m12; float Rc2; };
+struct PairC { f32x2 kq, p12, m12; float Rc2; };
 
 // Two ordered pairs: force on i into (fx, fy, fz).  getLJQH (Forces.h:341-360)
 // plus the shifted-force Coulomb part, as
 //   F = 12 E0 u6 (1 - u6 (1 + H)) / r^2 + Q (kq - 1/r^2) / r,  f_i += d F
+// taken as (12 E0 u6 (...) + g) / r^2 + (-kq) g with g = -Q / r (i.Q and c.kq hold
+// the negatives): 23 packed operations a pair instead of 24 and a shorter chain
+// (4096 x 60 atoms 159.9 -> 153.4 ms; errors against FP64 unchanged).
 // Excluded and out-of-range pairs are evaluated
 // at r^2 = 1e30, where every term underflows to zero except kq Q / r
 // (< 1e-16 eV/A).  bits 0, 1 of m: pair excluded.
@@ -76,9 +79,9 @@ __device__ __forceinline__ void pair2(const PairJ& j, const PairI& i, const Pair
         unpack2(mul2(j.H, i.H), h0, h1);
         h = pack2(fmaf(-12.f, fminf(h0, 0.f), -12.f), fmaf(-12.f, fminf(h1, 0.f), -12.f));
     }
-    const f32x2 t = mul2(mul2(u6, fma2(u6, h, c.p12)), ir2);
-    const f32x2 q = mul2(fma2(ir2, c.mone, c.kq), ir);
-    const f32x2 F = fma2(t, mul2(i.E, j.E), mul2(q, mul2(i.Q, j.Q)));
+    const f32x2 t = mul2(u6, fma2(u6, h, c.p12));
+    const f32x2 g = mul2(mul2(i.Q, j.Q), ir);
+    const f32x2 F = fma2(ir2, fma2(t, mul2(i.E, j.E), g), mul2(c.kq, g));
     fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
 }
 
@@ -218,7 +221,7 @@ struct RelaxEngine : CtaSystem<T> {
         PairC C;
         const bool cut = P.Rc2 > 0.f;
         C.Rc2 = cut ? P.Rc2 : 3.0e38f;
-        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.mone = pack2(-1.f, -1.f); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
+        C.kq = pack2(-P.kq_rc2, -P.kq_rc2); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
         const float *X = soa(0), *Yy = soa(1), *Z = soa(2), *R = soa(3), *E = soa(4), *Q = soa(5), *H = soa(6);
         int b = pb0, r = pr0, left = plen;                   // r: position inside the block's images x chunks
         while (left > 0) {
@@ -231,7 +234,7 @@ struct RelaxEngine : CtaSystem<T> {
             const int ic = vi ? i : natoms - 1;
             const float ix = X[ic], iy = Yy[ic], iz = Z[ic];
             PairI I;
-            I.R = pack2(R[ic], R[ic]); I.E = pack2(E[ic], E[ic]); I.Q = pack2(Q[ic], Q[ic]); I.H = HB ? pack2(H[ic], H[ic]) : 0;
+            I.R = pack2(R[ic], R[ic]); I.E = pack2(E[ic], E[ic]); I.Q = pack2(-Q[ic], -Q[ic]); I.H = HB ? pack2(H[ic], H[ic]) : 0;
             const uint8_t* row = reinterpret_cast<const uint8_t*>(xrow + ic * nbw);     // byte c: chunk c of 8 atoms j
             f32x2 fx = 0, fy = 0, fz = 0;
             while (r < rend) {
@@ -486,7 +489,7 @@ struct RelaxEngine : CtaSystem<T> {
         const int gl = lane & (G - 1);
         PairC C;
         C.Rc2 = P.Rc2;
-        C.kq = pack2(P.kq_rc2, P.kq_rc2); C.mone = pack2(-1.f, -1.f); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
+        C.kq = pack2(-P.kq_rc2, -P.kq_rc2); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
         // row: atom, words, whether the last word holds one entry, first word, and
         // this lane's first four words
         struct Row { int i, nw, odd; const uint32_t* p; uint32_t u[4]; };
@@ -511,7 +514,7 @@ struct RelaxEngine : CtaSystem<T> {
                 const float4 pi = spos[i], Ri = sREQ[i];
                 PairI I;
                 I.x = I.y = I.z = 0;
-                I.R = pack2(Ri.x, Ri.x); I.E = pack2(Ri.y, Ri.y); I.Q = pack2(Ri.z, Ri.z); I.H = HB ? pack2(Ri.w, Ri.w) : 0;
+                I.R = pack2(Ri.x, Ri.x); I.E = pack2(Ri.y, Ri.y); I.Q = pack2(-Ri.z, -Ri.z); I.H = HB ? pack2(Ri.w, Ri.w) : 0;
 #pragma unroll 1
                 for (int t = gl; t < n; t += G) {
                     const bool one = w.odd && t + 1 == n;                  // the word's second half is no entry
