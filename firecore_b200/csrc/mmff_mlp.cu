@@ -511,15 +511,65 @@ __global__ void __launch_bounds__(32 * RS) reduce_grad_kernel(const float* __res
 constexpr int DESC_WARPS = 8;
 constexpr int DESC_CAP = 192;           // candidates within 5 A kept per atom
 
+// box of each system's atoms (min, max), a warp per system
+__global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_box_kernel(Systems Y, int nsys, float4* __restrict__ box) {
+    const int lane = threadIdx.x & 31, s = blockIdx.x * DESC_WARPS + (threadIdx.x >> 5);
+    if (s >= nsys) return;
+    const int N = Y.desc[s].w, voff = Y.desc[s].z;
+    float mn[3] = {3e38f, 3e38f, 3e38f}, mx[3] = {-3e38f, -3e38f, -3e38f};
+    for (int j = lane; j < N; j += 32) {
+        const float4 p = Y.pos[voff + j];
+        mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
+        mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
+            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
+        }
+    if (lane == 0) {
+        box[2 * s] = make_float4(mn[0], mn[1], mn[2], 0.f);
+        box[2 * s + 1] = make_float4(mx[0], mx[1], mx[2], 0.f);
+    }
+}
+
+// height above the slab and GridFF force (the relaxer's sampler), a thread per
+// atom: one lane of the descriptors' warp took as many issue slots for it as
+// the rest of an atom's descriptors
+__global__ void __launch_bounds__(128) descriptor_site_kernel(Params P, Systems Y, const int* __restrict__ atom_sys, int NA,
+                                                              float zoff, float* __restrict__ feat) {
+    const int ga = blockIdx.x * 128 + threadIdx.x;
+    if (ga >= NA) return;
+    const int s = atom_sys[ga];
+    const int4 d = Y.desc[s];
+    const float4 pi = Y.pos[d.z + ga - d.x], go = Y.gorg[s];
+    float* out = feat + (size_t)ga * NFEAT;
+    out[64] = pi.z + go.z + zoff;
+    float4 fg = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (P.flags & F_GRID) {
+        const float3 u = make_float3((pi.x + go.x) * P.ginv[0], (pi.y + go.y) * P.ginv[1], (pi.z + go.z) * P.ginv[2]);
+        fg = grid_atom(P, u, Y.PLQ[ga]);
+    }
+    out[65] = fg.x; out[66] = fg.y; out[67] = fg.z;
+}
+
 // one warp per atom: candidates within 5 A over the pair-term image set, the
-// 32 nearest by (r, image, j), Gaussian radial bins per element channel,
-// height above the slab, GridFF force (the relaxer's sampler)
+// 32 nearest by (r, image, j), Gaussian radial bins per element channel.
+// Bound: instruction issue.  Most of it was distances to all atoms of all nine
+// images (100 rounds of 32 for a 330-atom molecule): images whose shifted
+// bounding box is out of reach of the atom are skipped, square roots taken of
+// near atoms only; the element channel is kept with a candidate, and the bins
+// run over the selected ones alone.
 __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, Systems Y, const int* __restrict__ atom_sys,
-                                                                    const int* __restrict__ elem, int NA, float zoff,
-                                                                    float* __restrict__ feat, int* __restrict__ err) {
+                                                                    const float4* __restrict__ box, const int* __restrict__ elem,
+                                                                    int NA, float* __restrict__ feat, int* __restrict__ err) {
     __shared__ float cr[DESC_WARPS][DESC_CAP];
     __shared__ int ck[DESC_WARPS][DESC_CAP];
-    __shared__ unsigned char csel[DESC_WARPS][DESC_CAP];
+    __shared__ unsigned char cch[DESC_WARPS][DESC_CAP];
+    __shared__ float sr[DESC_WARPS][32];
+    __shared__ unsigned char sch[DESC_WARPS][32];
     const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ga = blockIdx.x * DESC_WARPS + wib;
     if (ga >= NA) return;
@@ -531,6 +581,7 @@ __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, S
     const bool pbc = (P.flags & F_PBC) != 0;
     const int npx = pbc ? P.npbc[0] : 0, npy = pbc ? P.npbc[1] : 0, npz = pbc ? P.npbc[2] : 0;
     const float RC = 5.0f;
+    const float4 mn = box[2 * s], mx = box[2 * s + 1];           // the molecule's box
     int count = 0, k = 0;
     for (int iz = -npz; iz <= npz; iz++)
         for (int iy = -npy; iy <= npy; iy++)
@@ -539,6 +590,10 @@ __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, S
                 const float shy = lv[1] * ix + lv[4] * iy + lv[7] * iz;
                 const float shz = lv[2] * ix + lv[5] * iy + lv[8] * iz;
                 const bool central = (ix | iy | iz) == 0;
+                const float gx = fmaxf(0.f, fmaxf(mn.x + shx - pi.x, pi.x - mx.x - shx));
+                const float gy = fmaxf(0.f, fmaxf(mn.y + shy - pi.y, pi.y - mx.y - shy));
+                const float gz = fmaxf(0.f, fmaxf(mn.z + shz - pi.z, pi.z - mx.z - shz));
+                if (gx * gx + gy * gy + gz * gz > 1.001f * RC * RC) continue;      // with room for the rounding of r
                 for (int j0 = 0; j0 < N; j0 += 32) {
                     const int j = j0 + lane;
                     bool ok = false;
@@ -546,38 +601,90 @@ __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, S
                     if (j < N) {
                         const float4 pj = Y.pos[voff + j];
                         const float dx = pj.x + shx - pi.x, dy = pj.y + shy - pi.y, dz = pj.z + shz - pi.z;
-                        r = sqrtf(dx * dx + dy * dy + dz * dz);
-                        ok = (r < RC) && !(central && j == i);
+                        const float r2 = dx * dx + dy * dy + dz * dz;
+                        if (r2 < 1.001f * RC * RC) {
+                            r = sqrtf(r2);
+                            ok = (r < RC) && !(central && j == i);
+                        }
                     }
                     const unsigned bal = __ballot_sync(0xffffffffu, ok);
                     const int slot = count + __popc(bal & ((1u << lane) - 1u));
-                    if (ok && slot < DESC_CAP) { cr[wib][slot] = r; ck[wib][slot] = k * N + j; }
+                    if (ok && slot < DESC_CAP) {
+                        cr[wib][slot] = r; ck[wib][slot] = k * N + j;
+                        const int el = elem[aoff + j];
+                        cch[wib][slot] = (unsigned char)(el < 0 ? 255 : min(el, 3));       // a negative element has no channel
+                    }
                     count += __popc(bal);
                 }
             }
     if (count > DESC_CAP && lane == 0) atomicExch(err, 2);
     const int C = min(count, DESC_CAP);
     __syncwarp();
-    for (int c = lane; c < C; c += 32) {
-        const float r = cr[wib][c];
-        const int key = ck[wib][c];
-        int rank = 0;
-        for (int q = 0; q < C; q++) {
-            const float rq = cr[wib][q];
-            rank += (rq < r) || (rq == r && ck[wib][q] < key);
+    // The 32 nearest, in candidate order.  A distance with exactly 32 candidates
+    // below it, by bisection of (0, 5 A) (every lane counts its own candidates,
+    // one warp sum per try; 32nd and 33rd differ by some 0.05 A, so a few tries);
+    // where there is none within 12 (equal distances), the 32nd smallest by
+    // bisection over the bits of r (positive floats order as integers), then all
+    // nearer ones and, of those exactly there, the smallest (image, j) that fit.
+    constexpr int OWN = DESC_CAP / 32;
+    unsigned rb[OWN];
+#pragma unroll
+    for (int q = 0; q < OWN; q++) rb[q] = 32 * q + lane < C ? __float_as_uint(cr[wib][32 * q + lane]) : 0x7F800000u;
+    auto below = [&](unsigned t) {
+        int n = 0;
+#pragma unroll
+        for (int q = 0; q < OWN; q++) n += rb[q] < t;
+        return __reduce_add_sync(0xffffffffu, n);
+    };
+    unsigned thr = 0x7F800000u;                  // C <= 32: all
+    int room = 0;                                // how many at thr fit
+    if (C > 32) {
+        float lo = 0.f, hi = RC;
+        bool found = false;
+#pragma unroll 1
+        for (int it = 0; it < 12 && !found; it++) {
+            const float mid = 0.5f * (lo + hi);
+            thr = __float_as_uint(mid);
+            const int n = below(thr);
+            found = n == 32;
+            if (n < 32) lo = mid; else hi = mid;
         }
-        csel[wib][c] = rank < 32;
+        if (!found) {
+            thr = 0;                             // largest value with fewer than 32 below it
+#pragma unroll 1
+            for (int bit = 30; bit >= 0; bit--)
+                if (below(thr | (1u << bit)) < 32) thr |= 1u << bit;
+            room = 32 - below(thr);
+        }
+    }
+    int nsel = 0;
+    for (int c0 = 0; c0 < C; c0 += 32) {
+        const int c = c0 + lane;
+        bool in = false;
+        if (c < C) {
+            const unsigned r = __float_as_uint(cr[wib][c]);
+            in = r < thr;
+            if (r == thr && room > 0) {
+                int before = 0;
+                for (int p = 0; p < C; p++) before += __float_as_uint(cr[wib][p]) == thr && ck[wib][p] < ck[wib][c];
+                in = before < room;
+            }
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            const int o = nsel + __popc(bal & ((1u << lane) - 1u));
+            sr[wib][o] = cr[wib][c]; sch[wib][o] = cch[wib][c];
+        }
+        nsel += __popc(bal);
     }
     __syncwarp();
     const int ch0 = lane >> 4, ch1 = 2 + (lane >> 4);
     const float mu = (float)(lane & 15) * (5.0f / 15.0f);
     const float ig = 1.f / (2.f * 0.3f * 0.3f);
     float f0 = 0.f, f1 = 0.f;
-    for (int c = 0; c < C; c++) {
-        if (!csel[wib][c]) continue;
-        const int j = ck[wib][c] % N;
-        const int ch = min(elem[aoff + j], 3);
-        const float t = cr[wib][c] - mu;
+    for (int c = 0; c < nsel; c++) {
+        const int ch = sch[wib][c];
+        const float t = sr[wib][c] - mu;
         const float e = expf(-t * t * ig);
         if (ch == ch0) f0 += e;
         if (ch == ch1) f1 += e;
@@ -585,16 +692,6 @@ __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, S
     float* out = feat + (size_t)ga * NFEAT;
     out[lane] = f0;
     out[32 + lane] = f1;
-    if (lane == 0) {
-        const float4 go = Y.gorg[s];
-        out[64] = pi.z + go.z + zoff;
-        float4 fg = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (P.flags & F_GRID) {
-            const float3 u = make_float3((pi.x + go.x) * P.ginv[0], (pi.y + go.y) * P.ginv[1], (pi.z + go.z) * P.ginv[2]);
-            fg = grid_atom(P, u, Y.PLQ[aoff + i]);
-        }
-        out[65] = fg.x; out[66] = fg.y; out[67] = fg.z;
-    }
 }
 
 // ------------------------------------------------------------ warm start
@@ -733,7 +830,7 @@ struct Net {
     int t = 0;                              // AdamW step count
     Buf<float> prm, grad, m, v, mean, istd, feat, gpart;
     Buf<uint8_t> Wp, Xs, Xd;
-    Buf<float4> Td, outs, save;
+    Buf<float4> box, Td, outs, save;
     Buf<double> loss, losses, lpart;
     Buf<double4> E0;
     Buf<int> err, atom_sys, elem, accepted, keep;
@@ -834,11 +931,13 @@ std::vector<float4> make_targets(int n, int ntile, const float* target) {
 
 int features_device(const WorldView& V, double z_top) {
     if (!N.elem.p || N.na_elem != V.NA) return fail("element channels not set for these systems (mmff_mlp_set_elements)");
-    if (N.feat.ensure((size_t)V.NA * NFEAT) || N.err.ensure(1)) return -1;
+    if (N.feat.ensure((size_t)V.NA * NFEAT) || N.err.ensure(1) || N.box.ensure((size_t)2 * V.nsys)) return -1;
     const float zoff = (float)(V.gpos0[2] - z_top);
+    descriptor_box_kernel<<<(V.nsys + DESC_WARPS - 1) / DESC_WARPS, DESC_WARPS * 32, 0, V.stream>>>(V.Y, V.nsys, N.box.p);
     descriptor_kernel<<<(V.NA + DESC_WARPS - 1) / DESC_WARPS, DESC_WARPS * 32, 0, V.stream>>>(
-        V.P, V.Y, N.atom_sys.p, N.elem.p, V.NA, zoff, N.feat.p, N.err.p);
-    mmff_count_launches(1);
+        V.P, V.Y, N.atom_sys.p, N.box.p, N.elem.p, V.NA, N.feat.p, N.err.p);
+    descriptor_site_kernel<<<(V.NA + 127) / 128, 128, 0, V.stream>>>(V.P, V.Y, N.atom_sys.p, V.NA, zoff, N.feat.p);
+    mmff_count_launches(3);
     MCK(cudaGetLastError());
     return 0;
 }
