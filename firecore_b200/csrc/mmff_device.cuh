@@ -190,6 +190,18 @@ __device__ __forceinline__ float sqrt_from(float x, float y) {
     return fmaf(fmaf(-s, s, x), 0.5f * y, s);
 }
 
+// 1 / sqrt(x) in FP64 from the hardware's approximate reciprocal root y by one
+// step of the binomial series of (1 - e)^(-1/2), e = 1 - x y^2 (|e| < 2^-18:
+// the first term left out, 35/128 e^4, is below 2^-73).  Two roundings of at most
+// half a unit in the last place are left, of x y in e and of the result: within one
+// unit of the exact value.  For arguments far from overflow and underflow.
+__device__ __forceinline__ double inv_sqrt64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(e, fma(e, 0.3125, 0.375), 0.5), y);
+}
+
 // image index c (NBFF.h:42 ordering: x fastest, then y, then z) -> shift
 // in lattice units.  Quotients by the small image counts go through a float
 // reciprocal: (c + 1/2) / n stays >= 1/(2n) away from an integer, far beyond

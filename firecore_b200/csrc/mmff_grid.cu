@@ -25,17 +25,8 @@ namespace mmff {
 
 #define MMFF_COULOMB_D 14.3996448915
 
-// 1 / sqrt(x) in FP64 from the hardware's approximate reciprocal root by one
-// step of the binomial series of (1 - e)^(-1/2), e = 1 - x y^2 (|e| < 2^-18:
-// the first term left out, 35/128 e^4, is below 2^-73).  The rounding of the
-// last multiplication-addition is all that is left; arguments here are sums of
-// squares in A^2, far from overflow and underflow.
-__device__ __forceinline__ double inv_sqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(e, fma(e, 0.3125, 0.375), 0.5), y);
-}
+// (x, y, z, k_e Q) of a substrate atom
+__device__ __forceinline__ double4 charge_scaled(double4 s) { return make_double4(s.x, s.y, s.z, MMFF_COULOMB_D * s.w); }
 
 // Node potentials: Morse sums and the near Coulomb images directly, the far
 // ones as sum_c Lz[iz][c] far[ix][iy][c].  One thread takes kGridNX nodes that
@@ -63,7 +54,7 @@ __global__ void __launch_bounds__(128) grid_potential_kernel(int nx, int ny, int
     for (int m = 0; m < kGridNX; m++) { vp[m] = 0; vl[m] = 0; vc[m] = 0; }
     for (int t0 = 0; t0 < nsub; t0 += 128) {
         __syncthreads();
-        if (t0 + (int)threadIdx.x < nsub) { sa[threadIdx.x] = sposq[t0 + threadIdx.x]; sr[threadIdx.x] = sRE[t0 + threadIdx.x]; }
+        if (t0 + (int)threadIdx.x < nsub) { sa[threadIdx.x] = charge_scaled(sposq[t0 + threadIdx.x]); sr[threadIdx.x] = sRE[t0 + threadIdx.x]; }
         __syncthreads();
         const int nt = min(128, nsub - t0);
         if (!valid) continue;
@@ -78,28 +69,31 @@ __global__ void __launch_bounds__(128) grid_potential_kernel(int nx, int ny, int
 #pragma unroll
                 for (int m = 0; m < kGridNX; m++) {
                     const double x = dx + m * step.x, r2 = fma(x, x, yz);
-                    const double rr = r2 * inv_sqrt(r2);
+                    const double rr = r2 * inv_sqrt64(r2);
                     const double e = exp(-alpha * (rr - r.x));
                     const double eM = e * r.y;
                     vp[m] += eM * e;
                     vl[m] += eM * -2.0;
                 }
             }
-            double qsum[kGridNX];
-#pragma unroll
-            for (int m = 0; m < kGridNX; m++) qsum[m] = 0.0;
-            for (int k = 0; k < nc; k++) {
-                const double3 sh = shc[k];
-                const double dx = dx0 + sh.x, dy = dy0 + sh.y, dz = dz0 + sh.z;
+        }
+        // Coulomb: the atoms of one image after another, so that the partial sums
+        // stay near the neutral cell's.  (The images of one charge first add up to
+        // 10^2 eV, whose last place, 10^-11 eV over the sum, is as large as the last
+        // FP32 place of the coefficients some Angstrom above the slab.)
+        for (int k = 0; k < nc; k++) {
+            const double3 sh = shc[k];
+            const double bx = px + sh.x, by = py + sh.y, bz = pz0 + sh.z;
+            for (int a = 0; a < nt; a++) {
+                const double4 s = sa[a];
+                const double dx = bx - s.x, dy = by - s.y, dz = bz - s.z;
                 const double yz = dy * dy + (dz * dz + 1e-32);
 #pragma unroll
                 for (int m = 0; m < kGridNX; m++) {
                     const double x = dx + m * step.x;
-                    qsum[m] += inv_sqrt(fma(x, x, yz));
+                    vc[m] = fma(s.w, inv_sqrt64(fma(x, x, yz)), vc[m]);
                 }
             }
-#pragma unroll
-            for (int m = 0; m < kGridNX; m++) vc[m] += MMFF_COULOMB_D * s.w * qsum[m];
         }
     }
     if (!valid) return;
@@ -128,19 +122,17 @@ __global__ void __launch_bounds__(128) far_potential_kernel(int p, const double*
     double v = 0.0;
     for (int t0 = 0; t0 < nsub; t0 += 128) {
         __syncthreads();
-        if (t0 + (int)threadIdx.x < nsub) sa[threadIdx.x] = sposq[t0 + threadIdx.x];
+        if (t0 + (int)threadIdx.x < nsub) sa[threadIdx.x] = charge_scaled(sposq[t0 + threadIdx.x]);
         __syncthreads();
         const int nt = min(128, nsub - t0);
-        for (int a = 0; a < nt; a++) {
-            const double4 s = sa[a];
-            const double dx0 = px - s.x, dy0 = py - s.y, dz0 = pz - s.z;
-            double q = 0.0;
-            for (int k = k0; k < k1; k++) {
-                const double3 sh = shc[k];
-                const double dx = dx0 + sh.x, dy = dy0 + sh.y, dz = dz0 + sh.z;
-                q += inv_sqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
+        for (int k = k0; k < k1; k++) {          // (order: see grid_potential_kernel)
+            const double3 sh = shc[k];
+            const double bx = px + sh.x, by = py + sh.y, bz = pz + sh.z;
+            for (int a = 0; a < nt; a++) {
+                const double4 s = sa[a];
+                const double dx = bx - s.x, dy = by - s.y, dz = bz - s.z;
+                v = fma(s.w, inv_sqrt64(fma(dx, dx, fma(dy, dy, dz * dz))), v);
             }
-            v = fma(MMFF_COULOMB_D * s.w, q, v);
         }
     }
     if (valid) partial[(long)blockIdx.y * n3 + node] = v;

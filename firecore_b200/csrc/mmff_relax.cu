@@ -85,18 +85,11 @@ __device__ __forceinline__ void pair2(const PairJ& j, const PairI& i, const Pair
     fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
 }
 
-// sqrt(vv) / (sqrt(ff) + 1e-32) in FP64: from approximate reciprocal roots and
-// one step of the binomial series (error below the last place), where both
-// arguments are in range and the 1e-32 is below it; the library's roots and
-// division, four times the instructions for every thread of a step, otherwise
-__device__ __forceinline__ double rsqrt_series(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y * e, fma(e, fma(e, 0.3125, 0.375), 0.5), y);
-}
+// sqrt(vv) / (sqrt(ff) + 1e-32) in FP64 without the library's roots and division (four
+// times the instructions, for every thread of a step) where both arguments are in
+// range and the 1e-32 is below the last place
 __device__ __forceinline__ double length_ratio(double vv, double ff) {
-    if (vv > 1e-30 && ff > 1e-30 && vv < 1e30 && ff < 1e30) return vv * rsqrt_series(vv) * rsqrt_series(ff);
+    if (vv > 1e-30 && ff > 1e-30 && vv < 1e30 && ff < 1e30) return vv * inv_sqrt64(vv) * inv_sqrt64(ff);
     return vv > 0.0 ? sqrt(vv) / (sqrt(ff) + 1e-32) : 0.0;
 }
 

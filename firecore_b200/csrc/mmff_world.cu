@@ -868,7 +868,7 @@ int mmff_grid_build(int nsub, const double* spos, const double* sREQ, const doub
     const int p = F.p, n3 = p * p * p;
     const double *dfar = nullptr, *dLz = nullptr;
     if (p) {
-        const int parts = std::max(1, std::min((int)F.far.size(), 148 * 16 * 128 / std::max(128, n3)));
+        const int parts = std::max(1, std::min((int)F.far.size(), W.nsm * 16 * 128 / std::max(128, n3)));
         const size_t nt1 = (size_t)nx * p * p, nt2 = (size_t)nx * ny * p;
         std::vector<double> h(3 * p + (size_t)(nx + ny + nz) * p);
         double* hL = h.data() + 3 * p;
