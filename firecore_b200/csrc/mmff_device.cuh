@@ -79,10 +79,10 @@ struct Params {
     float slv[9];                          // substrate lattice vectors a, b, c
     float sK, sR2damp;                     // -alphaMorse, Rdamp^2
     float sg0[3];                          // grid origin: world = local + gorg + sg0
-    // shifted-image pair lists of the CTA relax kernels (null: none): vcap
-    // list entries per CTA
-    unsigned short* vlist;
-    int vcap;
+    // shifted-image pair lists of the relax kernels (null: none): vstride words per
+    // CTA for at most vcap list entries
+    uint32_t* vlist;
+    int vstride, vcap;
     float vskin;                           // list skin [A]
 };
 
@@ -579,15 +579,16 @@ __device__ __forceinline__ float3 grid_safe(float3 u) {
 }
 
 // One x-slice (a = 0..3) of the 4x4x4 stencil of Bspline::fe3d_pbc_comb3 for
-// grid coordinate u (already in voxel units).  Returns the slice's partial
-// (dE/dx*bx', E-channel combos) as (Fx, Fy, Fz, E) *before* the -1/step scale.
+// grid coordinate u (already in voxel units): its sums over y and z (d/dy, d/dz,
+// value), and the basis bx and its derivative dx along x, whose component a weighs
+// them (slice_force).
 // UNROLL: y-columns of the slice unrolled (their 16 loads in flight together).
 // In the fused relax step of small blocks (four or eight per SM) the step's
 // code, not its loads, is the limit: there no unrolling measured 5-7 % faster;
 // the 256-thread blocks keep all four (5 % faster there).
 template <int UNROLL = 4>
-__device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int nx, int ny, int nz, float3 u,
-                                             float4 PLQ, int a) {
+__device__ __forceinline__ float3 grid_slice(const float4* __restrict__ G, int nx, int ny, int nz, float3 u,
+                                             float4 PLQ, int a, float4& bx, float4& dx) {
     u = grid_safe(u);
     int ix = (int)u.x, iy = (int)u.y, iz = (int)u.z;
     if (u.x < 0.f) ix--;
@@ -617,9 +618,13 @@ __device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int n
         ey = fmaf(d, byb, ey);
         ez = fmaf(v, byb, ez);
     }
-    const float4 bx = bs_basis(tx), dx = bs_dbasis(tx);
+    bx = bs_basis(tx); dx = bs_dbasis(tx);
+    return make_float3(ex, ey, ez);
+}
+// slice a's part of (Fx, Fy, Fz, E), before the -1/step scale
+__device__ __forceinline__ float4 slice_force(float3 e, float4 bx, float4 dx, int a) {
     const float bxa = comp(bx, a), dxa = comp(dx, a);
-    return make_float4(dxa * ez, bxa * ex, bxa * ey, bxa * ez);
+    return make_float4(dxa * e.z, bxa * e.x, bxa * e.y, bxa * e.z);
 }
 
 // grid_slice with a per-atom cache of the 64 channel-combined coefficients
@@ -640,9 +645,9 @@ __device__ __forceinline__ float4 grid_slice(const float4* __restrict__ G, int n
 // ok = the lane holds a real atom.  The cache of an atom is read and written
 // only by the block that owns its system in this launch, each slice always by
 // the same lane position; a block barrier separates steps.
-__device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G, int nx, int ny, int nz, float3 u,
+__device__ __forceinline__ float3 grid_slice_cached(const float4* __restrict__ G, int nx, int ny, int nz, float3 u,
                                                     float4 PLQ, int a, bool ok, unsigned int* skey, unsigned int* gkey,
-                                                    float4* cs_atom) {
+                                                    float4* cs_atom, float4& bx, float4& dx) {
     float4* mine = cs_atom + 4 * a;
     float4 cs[4];
 #pragma unroll
@@ -686,9 +691,8 @@ __device__ __forceinline__ float4 grid_slice_cached(const float4* __restrict__ G
         ey = fmaf(d, byb, ey);
         ez = fmaf(v, byb, ez);
     }
-    const float4 bx = bs_basis(tx), dx = bs_dbasis(tx);
-    const float bxa = comp(bx, a), dxa = comp(dx, a);
-    return make_float4(dxa * ez, bxa * ex, bxa * ey, bxa * ez);
+    bx = bs_basis(tx); dx = bs_dbasis(tx);
+    return make_float3(ex, ey, ez);
 }
 
 // B-spline GridFF force + energy of one atom, the whole 4x4x4 stencil in this
@@ -752,12 +756,12 @@ struct SmemLayout {
     // evaluation kernels only (-1 otherwise): pair forces fnb, and the staged
     // j of an image tile (per warp 32 positions and parameters)
     int stage;
-    // relaxation kernels only (-1 otherwise): positions and pair parameters as
-    // seven arrays of maxNA rounded up to whole warps (x, y, z, R0, sqrt E0,
-    // Q, H); with pair lists: the positions they were built at (3 arrays), the
-    // start of each atom's row, the listed pairs' forces, the images' shifts,
-    // the atoms by falling row length
-    int soa, vp, rst, flist, shf, perm;
+    // relaxation kernels only (-1 otherwise): pair forces that are no fixed-point
+    // sums (flist); with pair lists: the positions they were built at (3 arrays) and
+    // the images' shifts
+    int flist, vp, shf;
+    int small;                          // relaxation: pair sums and grid in the order of the small systems (mmff_relax.cu)
+    int runs;                           // relaxation: runs that the pair lists are cut into
 };
 
 // number of shifted (non-central) PBC images of the pair term
@@ -776,15 +780,15 @@ __host__ __device__ inline int shifted_images(int flags, const int* npbc) {
 constexpr int kCompactAbove = 112 * 1024;
 constexpr int kCompactMinThreads = 256;
 
-// Image tiles are compiled into blocks of >= 128 threads only: the 64-thread
-// blocks serve molecules of <= 64 atoms, whose images reach a few edge atoms
-// (short candidate lists, ordered rows), and without the tile code there the
-// code of their central tiles stays as it is.
+// Evaluation: image tiles are compiled into blocks of >= 128 threads only: the
+// 64-thread blocks serve molecules of <= 64 atoms, whose images reach a few edge
+// atoms (short candidate lists, ordered rows), and without the tile code there
+// the code of their central tiles stays as it is.
 constexpr int kImageTileMinThreads = 128;
 // shifted-image pair lists of the CTA relax kernels: shifted images handled
 // (2-D cells have 8) and the average list entries per atom a slot holds
 constexpr int kListMaxImages = 12;
-constexpr int kListEntriesPerAtom = 96;
+constexpr int kListEntriesPerAtom = 48;
 
 __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, int mode, int lvl) {
     SmemLayout L;
@@ -798,7 +802,7 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
     L.vel = lvl < 2 ? take(16 * L.maxNV) : -1;
     L.fasm = take(16 * L.maxNV);
     L.fnb = relax ? -1 : take(16 * maxNA);
-    L.fgrid = take(16 * maxNA);
+    L.fgrid = take(16 * maxNA * (mode == 2 ? 2 : 1));
     L.REQ = take(16 * maxNA);
     L.PLQ = opt(16 * maxNA);
     L.ng = opt(16 * maxNA);
@@ -822,24 +826,26 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
     L.cpref = take(4 * nimg * L.nwords);    // exclusive prefix of their popcounts
     L.ccnt = take(4 * nimg);                // candidates per image
     L.clist = take(2 * nimg * maxNA);       // candidate atom indices per image, ascending
+    // image tiles: the positions and parameters of a tile's 32 candidates j, copied
+    // once per tile so that the 32 rotation steps read them directly instead of
+    // through the candidate list (evaluation: blocks >= kImageTileMinThreads)
+    L.stage = nimg > 0 && (relax || T >= kImageTileMinThreads) ? take(2 * 16 * 32 * L.nwarps) : -1;
     if (relax) {
         const int need = o - L.fng;
         o = o_keep;
-        if (need > fng_bytes) { L.cwords += o - L.fng; L.cpref += o - L.fng; L.ccnt += o - L.fng; L.clist += o - L.fng; take(need); }
+        if (need > fng_bytes) {
+            const int up = o - L.fng;
+            L.cwords += up; L.cpref += up; L.ccnt += up; L.clist += up;
+            if (L.stage >= 0) L.stage += up;
+            take(need);
+        }
     }
     L.facc = take(8 * 3 * maxNA * (mode == 2 ? 2 : 1));
-    // image tiles (blocks >= kImageTileMinThreads with candidate lists): the
-    // positions and parameters of a tile's 32 candidates j, copied once per
-    // tile so that the 32 rotation steps read them directly instead of through
-    // the candidate list
-    L.stage = (!relax && nimg > 0 && T >= kImageTileMinThreads) ? take(2 * 16 * 32 * L.nwarps) : -1;
-    L.soa = relax ? take(4 * 7 * 32 * L.nwords) : -1;
+    L.flist = relax ? take(16 * maxNA * (mode == 2 ? 2 : 1)) : -1;
     const bool lists = relax && nimg > 0 && nimg <= kListMaxImages;
     L.vp = lists ? take(4 * 3 * maxNA) : -1;
-    L.rst = lists ? take(4 * (maxNA + 1)) : -1;
-    L.flist = lists ? take(16 * maxNA) : -1;
     L.shf = lists ? take(16 * nimg) : -1;
-    L.perm = lists ? take(2 * maxNA) : -1;
+    L.small = 0; L.runs = 0;
     L.total = o;
     return L;
 }

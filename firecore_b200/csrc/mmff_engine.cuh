@@ -288,8 +288,7 @@ struct CtaSystem {
 
     // GridFF B-spline of every atom, 4 lanes per atom (x-slices), by the
     // threads t0 = 0 .. nt-1 of the caller (whole warps); zero without a grid
-    // (RELAX: the cache keys have a copy in shared memory)
-    template <bool ENERGY, bool RELAX>
+    template <bool ENERGY>
     __device__ void grid_phase(int t0, int nt, float4* fgr, double& Eg) {
         const float4* spos = at<float4>(L.pos);
         if (!(P.flags & F_GRID)) {
@@ -306,14 +305,14 @@ struct CtaSystem {
             const float4 p = spos[ic];
             const float3 uu = make_float3((p.x + lv[9]) * P.ginv[0], (p.y + lv[10]) * P.ginv[1],
                                           (p.z + lv[11]) * P.ginv[2]);
-            float4 r = make_float4(0, 0, 0, 0);
-            if (cached) {
-                r = grid_slice_cached(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(ic), a, ok,
-                                      RELAX ? at<unsigned>(L.key) + ic : Y.gkey + aoff + ic, Y.gkey + aoff + ic,
-                                      Y.gcs + (size_t)(aoff + ic) * 16);
-            } else if (ok) {
-                r = grid_slice<(T >= MMFF_UNROLL_MIN_T) ? 4 : 1>(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(ic), a);
-            }
+            float3 e = make_float3(0, 0, 0);
+            float4 bx = make_float4(0, 0, 0, 0), dx = bx;
+            if (cached)
+                e = grid_slice_cached(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(ic), a, ok, Y.gkey + aoff + ic,
+                                      Y.gkey + aoff + ic, Y.gcs + (size_t)(aoff + ic) * 16, bx, dx);
+            else if (ok)
+                e = grid_slice<(T >= MMFF_UNROLL_MIN_T) ? 4 : 1>(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, plq(ic), a, bx, dx);
+            float4 r = slice_force(e, bx, dx, a);
 #pragma unroll
             for (int o = 2; o > 0; o >>= 1) {
                 r.x += __shfl_xor_sync(0xffffffffu, r.x, o);

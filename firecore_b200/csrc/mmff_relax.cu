@@ -3,9 +3,8 @@
 // The system's whole state (positions, velocities, topology, force-field
 // parameters, recoil slots) is staged in shared memory, and every FIRE step
 // runs inside the CTA with three block barriers:
-//   forces   bonded terms (4 lanes per node), GridFF samples (4 lanes per atom),
-//            ordered pairs of the central image (and, without a cutoff, of
-//            every image), the listed pairs of the shifted images
+//   forces   units of one warp, claimed in turn: bonded terms (a node per lane),
+//            pair tiles, runs of the pair lists, GridFF samples (4 lanes per atom)
 //   | barrier |
 //   assemble recoil slots, clamp, FP64 sums of (f.v, v.v, f.f) and max |f|^2
 //   | barrier |
@@ -17,17 +16,14 @@
 // claims the next one, so converged systems retire and their slots refill
 // without a host round trip.
 //
-// Bound: FP32 issue, with 16 warps per SM (128 registers, shared memory) and, in
-// the small blocks, instruction fetch.  Hence few instructions per pair (two
-// pairs per packed operation), loops instead of straight-line code (bonded
-// terms by neighbour), three barriers, and shared-memory offsets as a kernel
-// parameter (constant bank) instead of registers.  Time per system-step with
-// the chip full, the kernel before (ordered thread-per-node bonded terms,
-// 32 x 32 Newton-3 tiles with shuffled reactions, lists in runs per thread) and
-// this one: 28 atoms 0.0087 -> 0.0056 us, 60: 0.0224 -> 0.0155, 100: 0.0566 ->
-// 0.0291, 200: 0.136 -> 0.088, 330: 0.286 -> 0.212; 127 atoms without a cutoff
-// (9 images), 300 systems: 0.380 -> 0.278 us.
-#include "mmff_engine.cuh"
+// A relaxation amplifies the last bit of a force: two or three molecules of a few
+// hundred part after some hundred steps, and the largest differences reach the
+// size of a bond.  So every FP32 sum here has a fixed order that depends on the
+// system alone, not on the block size, the cluster or which warp takes a unit:
+// partial sums over a tile or a run of list entries go to 64-bit integer totals,
+// everything else is summed by one lane.  The packed instructions below take two
+// independent sums side by side, never two terms of one sum.
+#include "mmff_pairs.cuh"
 
 #include <cooperative_groups.h>
 
@@ -40,49 +36,58 @@ __device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 d; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ float hsum2(f32x2 v) { float a, b; unpack2(v, a, b); return a + b; }
+__device__ __forceinline__ float lo2(f32x2 v) { float a, b; unpack2(v, a, b); return a; }
+__device__ __forceinline__ float hi2(f32x2 v) { float a, b; unpack2(v, a, b); return b; }
+__device__ __forceinline__ f32x2 neg2(f32x2 v) { return v ^ 0x8000000080000000ull; }
 
-// two atoms j at a time, as the arrays of SmemLayout::soa hold them
-struct PairJ { f32x2 x, y, z, R, E, Q, H; };
-// one atom i (shift - position, so that d = p_j + shift - p_i is one addition), in both halves
-struct PairI { f32x2 x, y, z, R, E, Q, H; };
-struct PairC { f32x2 kq, p12, m12; float Rc2; };
+// two atoms side by side.  x, y, z of an own atom are the negatives, so that
+// d = p_j - p_i is one addition; its Q is the negative too (see force2)
+struct Atom2 { f32x2 x, y, z, R, E, Q, H; };
+struct PairC { f32x2 nkq, m12, m1; float Rc2; };
 
-// Two ordered pairs: force on i into (fx, fy, fz).  getLJQH (Forces.h:341-360)
-// plus the shifted-force Coulomb part, as
-//   F = 12 E0 u6 (1 - u6 (1 + H)) / r^2 + Q (kq - 1/r^2) / r,  f_i += d F
-// taken as (12 E0 u6 (...) + g) / r^2 + (-kq) g with g = -Q / r (i.Q and c.kq hold
-// the negatives): 23 packed operations a pair instead of 24 and a shorter chain
-// (4096 x 60 atoms 159.9 -> 153.4 ms; errors against FP64 unchanged).
-// Excluded and out-of-range pairs are evaluated
-// at r^2 = 1e30, where every term underflows to zero except kq Q / r
-// (< 1e-16 eV/A).  bits 0, 1 of m: pair excluded.
-template <bool HB, bool COUNT>
-__device__ __forceinline__ void pair2(const PairJ& j, const PairI& i, const PairC& c, bool ex0, bool ex1, f32x2& fx,
-                                      f32x2& fy, f32x2& fz, unsigned long long& np) {
-    const f32x2 dx = add2(j.x, i.x), dy = add2(j.y, i.y), dz = add2(j.z, i.z);
+__device__ __forceinline__ Atom2 atom2(float4 p0, float4 R0, float4 p1, float4 R1) {
+    Atom2 a;
+    a.x = pack2(p0.x, p1.x); a.y = pack2(p0.y, p1.y); a.z = pack2(p0.z, p1.z);
+    a.R = pack2(R0.x, R1.x); a.E = pack2(R0.y, R1.y); a.Q = pack2(R0.z, R1.z); a.H = pack2(R0.w, R1.w);
+    return a;
+}
+__device__ __forceinline__ Atom2 own2(float4 p0, float4 R0, float4 p1, float4 R1) {
+    Atom2 a = atom2(p0, R0, p1, R1);
+    a.x = neg2(a.x); a.y = neg2(a.y); a.z = neg2(a.z); a.Q = neg2(a.Q);
+    return a;
+}
+
+// Two pairs: d = p_j - p_i and the scalar F of pair_force (mmff_device.cuh), operation
+// for operation in both halves (signs moved between factors do not round).
+// ex0, ex1: pair excluded.
+template <bool HB>
+__device__ __forceinline__ f32x2 force2(const Atom2& j, const Atom2& i, const PairC& c, bool ex0, bool ex1, f32x2& dx,
+                                        f32x2& dy, f32x2& dz, bool& ok0, bool& ok1) {
+    dx = add2(j.x, i.x); dy = add2(j.y, i.y); dz = add2(j.z, i.z);
     const f32x2 r2 = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
     float a, b;
     unpack2(r2, a, b);
-    const bool ok0 = !ex0 && a < c.Rc2, ok1 = !ex1 && b < c.Rc2;
-    if (COUNT) np += (ok0 ? 1 : 0) + (ok1 ? 1 : 0);
+    ok0 = !ex0 && a < c.Rc2;
+    ok1 = !ex1 && b < c.Rc2;
     a = ok0 ? a : 1e30f;
     b = ok1 ? b : 1e30f;
     const f32x2 ir = pack2(rsq(a), rsq(b));
     const f32x2 ir2 = mul2(ir, ir);
-    const f32x2 w = mul2(add2(j.R, i.R), ir);
-    const f32x2 u2 = mul2(w, w);
+    const f32x2 R0 = add2(i.R, j.R);
+    const f32x2 nQ = mul2(i.Q, j.Q);
+    const f32x2 u2 = mul2(mul2(R0, R0), ir2);
     const f32x2 u6 = mul2(mul2(u2, u2), u2);
-    f32x2 h = c.m12;
+    const f32x2 vdW = mul2(u6, mul2(i.E, j.E));
+    f32x2 X;
     if (HB) {
         float h0, h1;
-        unpack2(mul2(j.H, i.H), h0, h1);
-        h = pack2(fmaf(-12.f, fminf(h0, 0.f), -12.f), fmaf(-12.f, fminf(h1, 0.f), -12.f));
+        unpack2(mul2(i.H, j.H), h0, h1);
+        X = fma2(add2(u6, c.m1), vdW, mul2(mul2(u6, vdW), pack2(fminf(h0, 0.f), fminf(h1, 0.f))));
+    } else {
+        X = mul2(add2(u6, c.m1), vdW);
     }
-    const f32x2 t = mul2(u6, fma2(u6, h, c.p12));
-    const f32x2 g = mul2(mul2(i.Q, j.Q), ir);
-    const f32x2 F = fma2(ir2, fma2(t, mul2(i.E, j.E), g), mul2(c.kq, g));
-    fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+    const f32x2 F = fma2(mul2(c.m12, ir2), X, mul2(mul2(nQ, ir), ir2));
+    return fma2(mul2(nQ, c.nkq), ir, F);
 }
 
 // sqrt(vv) / (sqrt(ff) + 1e-32) in FP64 without the library's roots and division (four
@@ -95,30 +100,31 @@ __device__ __forceinline__ double length_ratio(double vv, double ff) {
 
 // CL: a cluster of CTAs relaxes one system (batches with fewer systems than half
 // the SMs).  Every CTA holds the whole system and runs every step; each takes a
-// share of the pairs, list rows and GridFF samples into its own fixed-point
-// sums, and assemble adds the sums of all of them through distributed shared
-// memory.  Integer sums are exact, so all CTAs get the same bits, and with the
-// same code on the same bits they take every decision alike: the cluster barrier
-// after the forces is the only one of a step.  Two sets of sums alternate, so
-// that the next step's adds never meet a neighbour that still reads.  Whatever
-// one CTA alone could see (a non-finite pair force, a full list slot) is
-// exchanged before it decides anything.
+// share of the tiles, list runs, image rows and GridFF samples.  Fixed-point sums
+// are added over all CTAs in assemble, through distributed shared memory; what one
+// lane summed (an atom's grid force, its image rows) is read from the CTA that has
+// it.  So all CTAs get the same bits, and with the same code on the same bits they
+// take every decision alike: the cluster barrier after the forces is the only one
+// of a step.  Two sets of sums alternate, so that the next step's writes never meet
+// a neighbour that still reads.  A non-finite pair force, which one CTA alone sees,
+// is exchanged before it decides anything.
 template <int T, bool COUNT, bool CL = false>
-struct RelaxEngine : CtaSystem<T> {
-    using B = CtaSystem<T>;
+struct RelaxEngine : PairEngine<T, 1, false, COUNT, true> {
+    using B = PairEngine<T, 1, false, COUNT, true>;
     using B::P; using B::Y; using B::L; using B::tid; using B::lane; using B::warp;
     using B::isys; using B::natoms; using B::nnode; using B::nvecs; using B::aoff; using B::noff; using B::voff;
-    using B::lv; using B::hasH; using B::hasX; using B::xrow; using B::nbw; using B::pairbad; using B::kFix;
+    using B::lv; using B::hasH; using B::hasX; using B::xrow; using B::nbw; using B::pairbad; using B::kFix; using B::kFixMax;
     using B::ngs; using B::ngc; using B::bks; using B::image_within; using B::build_candidates; using B::fix_add;
-    using B::image_excluded; using B::bbox_from_smem;
+    using B::image_excluded; using B::bbox_from_smem; using B::npair; using B::tile_mask; using B::bbmin; using B::bbmax;
     template <class X> __device__ __forceinline__ X* at(int off) { return B::template at<X>(off); }
     static constexpr int NW = T / 32;
-    unsigned long long npair = 0;      // COUNT: pair-images evaluated by this thread
-    // shifted-image pair lists of the current system (block-uniform): usable
-    // (a scratch slot, no overflow so far), built and valid, entries
-    bool listok = false, listed = false;
-    int nlist = 0, nrows = 0;
-    int cr = 0, cn = 1, par = 0;       // CL: rank in the cluster, its size, which set of sums this step uses
+    // shifted-image pair lists of the current system (block-uniform)
+    enum { LIST_NONE, LIST_QUIET, LIST_BUILT };     // QUIET: no image within cutoff + skin of the positions vp
+    bool listok = false;               // usable (a scratch slot, no overflow so far)
+    int lstate = LIST_NONE;
+    int nlist = 0;                     // entries
+    bool use_list = false;             // this step evaluates them
+    int cr = 0, cn = 1, par = 0;       // CL: rank in the cluster, its size; which set of sums (and unit counter) this step uses
 
     __device__ RelaxEngine(const Params& p, const Systems& y, char* smem, const SmemLayout& l) : B(p, y, smem, l) {
         if constexpr (CL) {
@@ -133,8 +139,10 @@ struct RelaxEngine : CtaSystem<T> {
     }
     // this step's force sums
     __device__ __forceinline__ long long* sums() { return at<long long>(L.facc) + (CL ? par * 3 * L.maxNA : 0); }
-    // flags of this CTA that the others read: [0, 1] non-finite pair force (per set of sums), [2] list slot full
-    __device__ __forceinline__ int* flags_cl() const {
+    __device__ __forceinline__ float4* gridf() { return at<float4>(L.fgrid) + (CL ? par * L.maxNA : 0); }
+    __device__ __forceinline__ float4* listf() { return at<float4>(L.flist) + (CL ? par * L.maxNA : 0); }
+    // [0, 1] a non-finite pair force (CL, per set of sums), [2, 3] units claimed (per step parity)
+    __device__ __forceinline__ int* shared_ints() const {
         __shared__ int f[4];
         return f;
     }
@@ -142,601 +150,634 @@ struct RelaxEngine : CtaSystem<T> {
     __device__ __forceinline__ bool any_cl(int k) const {
         int a = 0;
         if constexpr (CL)
-            for (int c = 0; c < cn; c++) a |= cooperative_groups::this_cluster().map_shared_rank(flags_cl(), c)[k];
+            for (int c = 0; c < cn; c++) a |= cooperative_groups::this_cluster().map_shared_rank(shared_ints(), c)[k];
         return a != 0;
     }
 
-    // arrays of the pair loops, NP atoms each
-    __device__ __forceinline__ int np() const { return 32 * L.nwords; }
-    __device__ __forceinline__ float* soa(int k) { return at<float>(L.soa) + k * np(); }
+    // pair forces beside the fixed-point sums: the small systems' whole pair sums, else
+    // without a cutoff the image rows
+    __device__ __forceinline__ bool image_row_path() const { return (P.flags & F_PBC) && !(P.Rc2 > 0.f) && !L.small; }
+    __device__ __forceinline__ bool has_listf() const { return (P.flags & F_NONBONDED) && (L.small || image_row_path()); }
 
     __device__ void load(int s) {
         B::load(s);
         listok = P.vlist != nullptr && natoms <= 4096 && P.Rc2 > 0.f && L.nimg > 0 && L.nimg <= kListMaxImages &&
                  (P.flags & F_NONBONDED);
-        listed = false;
+        lstate = LIST_NONE;
         nlist = 0;
+        use_list = false;
+        par = 0;
         __syncthreads();
         if (L.shf >= 0 && tid < L.nimg) {
-            const float3 s = image_of(image_index(tid));
-            at<float4>(L.shf)[tid] = make_float4(s.x, s.y, s.z, 0.f);
-        }
-        split_pairs((P.flags & F_PBC) && !(P.Rc2 > 0.f));
-        // padding atoms up to whole 8-atom chunks: no charge, no LJ, far away
-        const float4* spos = at<float4>(L.pos);
-        const float4* sREQ = at<float4>(L.REQ);
-        for (int a = tid; a < np(); a += T) {
-            const bool v = a < natoms;
-            const float4 p = v ? spos[a] : make_float4(1e6f, 1e6f, 1e6f, 0.f);
-            const float4 r = v ? sREQ[a] : make_float4(0.f, 0.f, 0.f, 0.f);
-            soa(0)[a] = p.x; soa(1)[a] = p.y; soa(2)[a] = p.z;
-            soa(3)[a] = r.x; soa(4)[a] = r.y; soa(5)[a] = r.z; soa(6)[a] = r.w;
+            const float3 sh = image_of(image_index(tid));
+            at<float4>(L.shf)[tid] = make_float4(sh.x, sh.y, sh.z, 0.f);
         }
         long long* facc = at<long long>(L.facc);
         for (int a = tid; a < 3 * natoms; a += T) facc[a] = 0;
-        if constexpr (CL) {
-            par = 0;
+        if constexpr (CL)
             for (int a = tid; a < 3 * natoms; a += T) facc[3 * L.maxNA + a] = 0;
-            if (tid < 4) flags_cl()[tid] = 0;
-        }
+        if (tid < 4) shared_ints()[tid] = 0;
     }
-
-    // ---- ordered pairs (i, j + shift), every atom i of the central image -----
-    // Lanes own 32 atoms i and walk the atoms j together (shared-memory
-    // broadcasts, no shuffles, no reactions), two j per packed instruction.
-    // Work: i-blocks x images x chunks of 8 j, one flat range cut into equal
-    // parts, one per warp; a warp's sum for a block goes to the fixed-point
-    // accumulators when its range leaves the block.  In the last block, when
-    // at most 16 atoms are left, 2, 4, ... lanes share an atom and take every
-    // 2nd, 4th, ... chunk.
-    int pb0, pr0, plen;          // this warp's part of the range: first block, position in it, length
-    __device__ __forceinline__ int last_lg() const {      // last block: 2^lg lanes per atom
-        const int rem = natoms - 32 * (nbw - 1);
-        return rem > 16 ? 0 : rem > 8 ? 1 : rem > 4 ? 2 : rem > 2 ? 3 : rem > 1 ? 4 : 5;
-    }
-    __device__ void split_pairs(bool all_images) {        // once per system
-        const int nim = all_images ? (2 * P.npbc[0] + 1) * (2 * P.npbc[1] + 1) * (2 * P.npbc[2] + 1) : 1;
-        const int c8 = (natoms + 7) >> 3, lg = last_lg(), cl = (c8 + (1 << lg) - 1) >> lg;
-        const int total = ((nbw - 1) * c8 + cl) * nim;
-        const int w = cr * NW + warp, nw = cn * NW;
-        const int q = (int)((long long)total * w / nw);
-        plen = (int)((long long)total * (w + 1) / nw) - q;
-        pb0 = min(q / (c8 * nim), nbw - 1);
-        pr0 = q - pb0 * c8 * nim;
-    }
-
-    template <bool HB>
-    __device__ void ordered_pairs(bool all_images, long long* facc) {
-        const int npx = all_images ? P.npbc[0] : 0, npy = all_images ? P.npbc[1] : 0, npz = all_images ? P.npbc[2] : 0;
-        const int nxi = 2 * npx + 1, nyi = 2 * npy + 1, nim = nxi * nyi * (2 * npz + 1);
-        const int central = (npz * nyi + npy) * nxi + npx;
-        const int c8 = (natoms + 7) >> 3, lg = last_lg(), cl = (c8 + (1 << lg) - 1) >> lg;
+    __device__ __forceinline__ PairC pair_consts() const {
         PairC C;
-        const bool cut = P.Rc2 > 0.f;
-        C.Rc2 = cut ? P.Rc2 : 3.0e38f;
-        C.kq = pack2(-P.kq_rc2, -P.kq_rc2); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
-        const float *X = soa(0), *Yy = soa(1), *Z = soa(2), *R = soa(3), *E = soa(4), *Q = soa(5), *H = soa(6);
-        int b = pb0, r = pr0, left = plen;                   // r: position inside the block's images x chunks
-        while (left > 0) {
-            const bool last = b == nbw - 1;
-            const int sh = last ? lg : 0, cs = last ? cl : c8;
-            const int rend = min(cs * nim, r + left);
-            left -= rend - r;
-            const int i = 32 * b + (lane & ((32 >> sh) - 1)), sub = lane >> (5 - sh);
-            const bool vi = i < natoms;
-            const int ic = vi ? i : natoms - 1;
-            const float ix = X[ic], iy = Yy[ic], iz = Z[ic];
-            PairI I;
-            I.R = pack2(R[ic], R[ic]); I.E = pack2(E[ic], E[ic]); I.Q = pack2(-Q[ic], -Q[ic]); I.H = HB ? pack2(H[ic], H[ic]) : 0;
-            const uint8_t* row = reinterpret_cast<const uint8_t*>(xrow + ic * nbw);     // byte c: chunk c of 8 atoms j
-            f32x2 fx = 0, fy = 0, fz = 0;
-            while (r < rend) {
-                const int im = all_images ? r / cs : 0;
-                int t = r - im * cs;
-                const int tend = min(cs, t + (rend - r));
-                r += tend - t;
-                float3 s = make_float3(0.f, 0.f, 0.f);
-                if (im != central) s = image_shift(lv, im % nxi - npx, (im / nxi) % nyi - npy, im / (nxi * nyi) - npz);
-                I.x = pack2(s.x - ix, s.x - ix); I.y = pack2(s.y - iy, s.y - iy); I.z = pack2(s.z - iz, s.z - iz);
-                // excluded j of chunk c (bits 0..7): the host-built rows in the
-                // central image; else i itself and its bonded neighbours there
-                auto excl = [&](int c) -> uint32_t {
-                    if (!vi || c >= c8) return 0xFFu;
-                    if (im == central) return __ldg(row + c);
-                    uint32_t m = (i >> 3) == c ? 1u << (i & 7) : 0u;
-                    if (8 * c + 8 > natoms) m |= 0xFFu << (natoms - 8 * c);
-                    if (hasX) {
-                        const int4 g = ngs(i), gc = ngc(i);
-                        if (gc.x == im && g.x >= 0 && (g.x >> 3) == c) m |= 1u << (g.x & 7);
-                        if (gc.y == im && g.y >= 0 && (g.y >> 3) == c) m |= 1u << (g.y & 7);
-                        if (gc.z == im && g.z >= 0 && (g.z >> 3) == c) m |= 1u << (g.z & 7);
-                        if (gc.w == im && g.w >= 0 && (g.w >> 3) == c) m |= 1u << (g.w & 7);
-                    }
-                    return m;
-                };
-                uint32_t mn = excl((t << sh) + sub);
-                for (; t < tend; t++) {
-                    const uint32_t m = mn;
-                    const int j0 = 8 * min((t << sh) + sub, c8 - 1);
-                    if (t + 1 < tend) mn = excl(((t + 1) << sh) + sub);
-#pragma unroll
-                    for (int k = 0; k < 8; k += 4) {
-                        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(X + j0 + k);
-                        const ulonglong2 y = *reinterpret_cast<const ulonglong2*>(Yy + j0 + k);
-                        const ulonglong2 z = *reinterpret_cast<const ulonglong2*>(Z + j0 + k);
-                        const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(R + j0 + k);
-                        const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(E + j0 + k);
-                        const ulonglong2 qq = *reinterpret_cast<const ulonglong2*>(Q + j0 + k);
-                        ulonglong2 h = make_ulonglong2(0, 0);
-                        if (HB) h = *reinterpret_cast<const ulonglong2*>(H + j0 + k);
-                        const PairJ ja = {x.x, y.x, z.x, rr.x, e.x, qq.x, h.x}, jb = {x.y, y.y, z.y, rr.y, e.y, qq.y, h.y};
-                        pair2<HB, COUNT>(ja, I, C, m & (1u << k), m & (2u << k), fx, fy, fz, npair);
-                        pair2<HB, COUNT>(jb, I, C, m & (4u << k), m & (8u << k), fx, fy, fz, npair);
-                    }
-                }
+        C.Rc2 = P.Rc2 > 0.f ? P.Rc2 : 3.0e38f;
+        C.nkq = pack2(-P.kq_rc2, -P.kq_rc2); C.m12 = pack2(-12.f, -12.f); C.m1 = pack2(-1.f, -1.f);
+        return C;
+    }
+
+    // ---- central image, two 32 x 32 tiles at a time ---------------------------
+    // Tiles of PairEngine (off_tile, diag_tile), sums in the same order: lane l owns
+    // atom i of block bi0 and one of block bi1, the atoms j of block bj0 (and bj1)
+    // rotate past it, the reactions with them.  KIND 0: both tiles have block bj0, so
+    // that a j is loaded once for both; 1: two unrelated tiles; 2: two diagonal ones.
+    // A block < 0: no second tile.
+    // Bound: the FP32 pipe (29 packed operations) and issue (about 60) a rotation step
+    // of 64 unordered pairs.
+    template <bool HB, int KIND>
+    __device__ void tile2(int bi0, int bi1, int bj0, int bj1, long long* facc) {
+        const float4* spos = at<float4>(L.pos);
+        const float4* sREQ = at<float4>(L.REQ);
+        const PairC C = pair_consts();
+        const int last = natoms - 1;
+        const int i0 = 32 * bi0 + lane, i1 = 32 * bi1 + lane;
+        const bool v0 = i0 < natoms, v1 = bi1 >= 0 && i1 < natoms;
+        const int a0 = v0 ? i0 : 0, a1 = v1 ? i1 : 0;
+        const Atom2 I = own2(spos[a0], sREQ[a0], spos[a1], sREQ[a1]);
+        // excluded j by rotation step
+        uint32_t m0 = v0 ? __ldg(xrow + i0 * nbw + bj0) : ~0u, m1 = v1 ? __ldg(xrow + i1 * nbw + (KIND == 0 ? bj0 : bj1)) : ~0u;
+        m0 = __funnelshift_r(m0, m0, lane);
+        m1 = __funnelshift_r(m1, m1, lane);
+        const int b0 = 32 * bj0, b1 = KIND == 0 ? b0 : 32 * max(bj1, 0);
+        f32x2 fx = 0, fy = 0, fz = 0, rx = 0, ry = 0, rz = 0;
+        const int nxt = (lane + 1) & 31;
+        constexpr int s0 = KIND == 2 ? 1 : 0, s1 = KIND == 2 ? 17 : 32;
+        if (KIND == 2) { m0 >>= 1; m1 >>= 1; }
+#pragma unroll 2
+        for (int s = s0; s < s1; s++) {
+            const int jl = (lane + s) & 31;
+            const int j0 = min(b0 + jl, last);
+            const float4 p0 = spos[j0], R0 = sREQ[j0];
+            Atom2 J;
+            if (KIND == 0) {
+                J = atom2(p0, R0, p0, R0);
+            } else {
+                const int j1 = min(b1 + jl, last);
+                J = atom2(p0, R0, spos[j1], sREQ[j1]);
             }
-            float3 f = make_float3(hsum2(fx), hsum2(fy), hsum2(fz));
-            for (int o = 32 >> sh; o < 32; o <<= 1) {        // lanes that share an atom
-                f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
-                f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
-                f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
+            const bool half = KIND == 2 && s == 16 && lane >= 16;
+            f32x2 dx, dy, dz;
+            bool ok0, ok1;
+            const f32x2 F = force2<HB>(J, I, C, (m0 & 1u) || half, (m1 & 1u) || half, dx, dy, dz, ok0, ok1);
+            m0 >>= 1; m1 >>= 1;
+            if (COUNT) npair += (ok0 ? 2 : 0) + (ok1 ? 2 : 0);
+            fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+            const f32x2 nF = neg2(F);
+            if (KIND == 2) {
+                const int src = (lane - s) & 31;     // the lane whose partner this lane's atoms were
+                const f32x2 gx = mul2(dx, nF), gy = mul2(dy, nF), gz = mul2(dz, nF);
+                fx = add2(fx, __shfl_sync(0xffffffffu, gx, src));
+                fy = add2(fy, __shfl_sync(0xffffffffu, gy, src));
+                fz = add2(fz, __shfl_sync(0xffffffffu, gz, src));
+            } else {
+                rx = __shfl_sync(0xffffffffu, fma2(dx, nF, rx), nxt);
+                ry = __shfl_sync(0xffffffffu, fma2(dy, nF, ry), nxt);
+                rz = __shfl_sync(0xffffffffu, fma2(dz, nF, rz), nxt);
             }
-            if (all_images) {
-                // an atom on top of an image: the force is scaled to the
-                // accumulators' range as a vector, so that its direction stays
-                const float m = fmaxf(fabsf(f.x), fmaxf(fabsf(f.y), fabsf(f.z)));
-                if (m > B::kFixMax && isfinite(m)) f = f * (B::kFixMax / m);
-            }
-            if (vi && sub == 0) fix_add(facc + 3 * i, f);
-            b++;
-            r = 0;
+        }
+        if (v0) fix_add(facc + 3 * i0, make_float3(lo2(fx), lo2(fy), lo2(fz)));
+        if (v1) fix_add(facc + 3 * i1, make_float3(hi2(fx), hi2(fy), hi2(fz)));
+        if (KIND != 2) {
+            const int j0 = b0 + lane, j1 = b1 + lane;
+            if (j0 < natoms) fix_add(facc + 3 * j0, make_float3(lo2(rx), lo2(ry), lo2(rz)));
+            if (bi1 >= 0 && j1 < natoms) fix_add(facc + 3 * j1, make_float3(hi2(rx), hi2(ry), hi2(rz)));
+        }
+    }
+    // units of tiles: doubles (2m, 2m + 1 | bj), the tiles (bj - 1, bj) of odd bj in
+    // pairs, the diagonal ones in pairs
+    __device__ __forceinline__ int double_tiles() const { return ((nbw - 1) / 2) * (nbw / 2); }
+    __device__ __forceinline__ int single_units() const { return (nbw / 2 + 1) >> 1; }
+    __device__ __forceinline__ int diag_units() const { return (nbw + 1) >> 1; }
+    template <bool HB>
+    __device__ void tile_unit(int u, long long* facc) {
+        const int nd = double_tiles(), ns = single_units();
+        if (u < nd) {
+            int bj = 2;
+            while (u >= bj / 2) { u -= bj / 2; bj++; }
+            tile2<HB, 0>(2 * u, 2 * u + 1, bj, bj, facc);
+        } else if (u < nd + ns) {
+            const int b = 4 * (u - nd);
+            const bool two = b + 3 < nbw;
+            tile2<HB, 1>(b, two ? b + 2 : -1, b + 1, two ? b + 3 : -1, facc);
+        } else {
+            const int d = 2 * (u - nd - ns), d1 = d + 1 < nbw ? d + 1 : -1;
+            tile2<HB, 2>(d, d1, d, d1, facc);
         }
     }
 
-    // ---- shifted images under a cutoff ---------------------------------------
-    // one ordered pair (scalar form of pair2)
-    template <bool HB>
-    __device__ __forceinline__ void pair1(float dx, float dy, float dz, float4 Ri, float4 Rj, bool excl, float3& f) {
-        bool ok;
-        float e;
-        const float F = pair_force<false, HB>(dx, dy, dz, Ri, Rj, excl, P.Rc2, P.kq_rc2, 0.f, true, ok, e);
-        if (COUNT && ok) npair++;
-        f.x = fmaf(dx, F, f.x); f.y = fmaf(dy, F, f.y); f.z = fmaf(dz, F, f.z);
-    }
+    // ---- shifted images -------------------------------------------------------
     // shifted image k (0 .. nimg-1, without the central one) -> image index with it, and its shift
     __device__ __forceinline__ int image_index(int k) const { return k < L.nimg / 2 ? k : k + 1; }
     __device__ __forceinline__ float3 image_of(int ipbc) const {
         const int nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
         return image_shift(lv, ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1], ipbc / (nxi * nyi) - P.npbc[2]);
     }
-
-    // Per-step candidate rows: every ordered pair (i, j + shift) with i a
-    // candidate of the mirror image and j one of the image (build_candidates),
-    // one thread per row.  The path of systems without pair lists (lists
-    // switched off, more than kListMaxImages images, a list that overflowed).
-    template <bool HB>
-    __device__ void candidate_rows(const float4* spos, const float4* sREQ, long long* facc) {
-        const int* ccnt = at<int>(L.ccnt);
-        const unsigned short* clist = at<unsigned short>(L.clist);
-        int nrows = 0;
-        for (int k = 0; k < L.nimg; k++) nrows += ccnt[L.nimg - 1 - k];
-        for (int u = cr * T + tid; u < nrows; u += cn * T) {
-            int c = u, k = 0;
-            while (c >= ccnt[L.nimg - 1 - k]) { c -= ccnt[L.nimg - 1 - k]; k++; }
-            const int i = clist[(L.nimg - 1 - k) * L.maxNA + c];
+    // some shifted image within sqrt(R2) of the box of the atoms
+    __device__ __forceinline__ bool any_image(float R2) const {
+        bool any = false;
+        const int nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
+        for (int k = 0; k < L.nimg; k++) {
             const int ipbc = image_index(k);
-            const float3 s = image_of(ipbc);
-            const float4 pi = spos[i], Ri = sREQ[i];
-            const unsigned short* Jl = clist + k * L.maxNA;
-            float3 f = make_float3(0.f, 0.f, 0.f);
-            for (int q = 0; q < ccnt[k]; q++) {
-                const int j = Jl[q];
-                const float4 pj = spos[j];
-                pair1<HB>(pj.x + s.x - pi.x, pj.y + s.y - pi.y, pj.z + s.z - pi.z, Ri, sREQ[j], image_excluded(i, j, ipbc), f);
-            }
-            fix_add(facc + 3 * i, f);
+            any |= image_within(ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1], ipbc / (nxi * nyi) - P.npbc[2], R2);
         }
+        return any;
+    }
+
+    // Without a cutoff: atoms i of unit u (64 of them, two per lane) against all atoms of
+    // every shifted image, images and atoms j in order; each atom's sum in one accumulator.
+    template <bool HB>
+    __device__ void image_row_unit(int u, float4* out) {
+        const float4* spos = at<float4>(L.pos);
+        const float4* sREQ = at<float4>(L.REQ);
+        const PairC C = pair_consts();
+        const int i0 = 64 * u + lane, i1 = i0 + 32;
+        const bool v0 = i0 < natoms, v1 = i1 < natoms;
+        const int a0 = v0 ? i0 : 0, a1 = v1 ? i1 : 0;
+        const float4 p0 = spos[a0], p1 = spos[a1];
+        Atom2 I = own2(p0, sREQ[a0], p1, sREQ[a1]);
+        const int4 g0 = ngs(a0), c0 = ngc(a0), g1 = ngs(a1), c1 = ngc(a1);
+        const int nim = (2 * P.npbc[0] + 1) * (2 * P.npbc[1] + 1) * (2 * P.npbc[2] + 1), central = nim / 2;
+        f32x2 fx = 0, fy = 0, fz = 0;
+        for (int im = 0; im < nim; im++) {
+            if (im == central) continue;
+            const float3 s = image_of(im);
+            I.x = pack2(s.x - p0.x, s.x - p1.x); I.y = pack2(s.y - p0.y, s.y - p1.y); I.z = pack2(s.z - p0.z, s.z - p1.z);
+            auto cell = [&](int c, int g) { return c == im ? g : -1; };
+            const int e0 = cell(c0.x, g0.x), e1 = cell(c0.y, g0.y), e2 = cell(c0.z, g0.z), e3 = cell(c0.w, g0.w);
+            const int h0 = cell(c1.x, g1.x), h1 = cell(c1.y, g1.y), h2 = cell(c1.z, g1.z), h3 = cell(c1.w, g1.w);
+            const bool bonds = __any_sync(0xffffffffu, max(max(max(e0, e1), max(e2, e3)), max(max(h0, h1), max(h2, h3))) >= 0);
+            auto pass = [&](auto excl) {
+#pragma unroll 2
+                for (int j = 0; j < natoms; j++) {
+                    const float4 p = spos[j], R = sREQ[j];
+                    const Atom2 J = atom2(p, R, p, R);
+                    f32x2 dx, dy, dz;
+                    bool ok0, ok1, x0, x1;
+                    excl(j, x0, x1);
+                    const f32x2 F = force2<HB>(J, I, C, x0, x1, dx, dy, dz, ok0, ok1);
+                    if (COUNT) npair += (ok0 && v0 ? 1 : 0) + (ok1 && v1 ? 1 : 0);
+                    fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+                }
+            };
+            if (!bonds) pass([&](int j, bool& x0, bool& x1) { x0 = j == i0; x1 = j == i1; });
+            else pass([&](int j, bool& x0, bool& x1) {
+                x0 = j == i0 || j == e0 || j == e1 || j == e2 || j == e3;
+                x1 = j == i1 || j == h0 || j == h1 || j == h2 || j == h3;
+            });
+        }
+        if (v0) out[i0] = make_float4(lo2(fx), lo2(fy), lo2(fz), 0.f);
+        if (v1) out[i1] = make_float4(hi2(fx), hi2(fy), hi2(fz), 0.f);
     }
 
     // Shifted-image pair lists (Verlet lists with a skin, P.vskin, 1 A by
-    // default).  Of the pairs the candidate rows of the shifted images
+    // default).  Of the pairs the candidate tiles of the shifted images
     // evaluate, only a few percent lie inside the cutoff: for a large molecule
     // the candidates of an image span its whole cross-section.  With lists,
     // the ordered pairs (i, j + shift of image k) over every shifted image k
     // closer than Rc + skin are collected once and evaluated every step (both
     // orders of a pair are listed, so no reaction is needed) until some atom
     // has moved more than skin/2 since the build (move() checks); then they are
-    // rebuilt.  One row per atom i over all images, entry j | k << 12, in the
-    // CTA's slot of global scratch; row starts in shared memory.
-    __device__ __forceinline__ unsigned short* vslot() const { return P.vlist + (size_t)blockIdx.x * P.vcap; }
+    // rebuilt.  The entries are numbered by image, then atom i, then atom j, and cut
+    // into L.runs runs of equal length; within a run the consecutive entries of an atom
+    // i have one FP32 sum.  Entry e of run v lies at word e L.runs + v of the CTA's
+    // slot of global scratch (a warp's 32 runs read whole lines), and the first entry's
+    // number of every row (image, i) behind the entries.
+    __device__ __forceinline__ uint32_t* vslot() const { return P.vlist + (size_t)blockIdx.x * P.vstride; }
+    __device__ __forceinline__ uint32_t run_start(uint32_t v) const { return (uint32_t)nlist * v / (uint32_t)L.runs; }
 
-    // pass over the listed pairs of atom i by one warp: f(pair listed here, entry) per 32 candidates
+    // pass over the listed pairs of row r by one warp: f(pair listed here, entry) per 32 candidates
     template <class F>
-    __device__ __forceinline__ void row_pass(int i, const float4* spos, float Rv2, F&& f) {
+    __device__ __forceinline__ void row_pass(int r, const float4* spos, float Rv2, F&& f) {
         const int* ccnt = at<int>(L.ccnt);
         const unsigned short* clist = at<unsigned short>(L.clist);
-        const uint32_t* words = at<uint32_t>(L.cwords);
-        const float4 pi = spos[i];
-        for (int k = 0; k < L.nimg; k++) {
-            if (!((words[(L.nimg - 1 - k) * L.nwords + (i >> 5)] >> (i & 31)) & 1u)) continue;   // i cannot reach image k
-            const int ipbc = image_index(k);
-            const float4 s = at<float4>(L.shf)[k];
-            const float qx = pi.x - s.x, qy = pi.y - s.y, qz = pi.z - s.z;
-            const unsigned short* Jl = clist + k * L.maxNA;
-            const int nJ = ccnt[k];
-            for (int j0 = 0; j0 < nJ; j0 += 32) {
-                const int j = Jl[min(j0 + lane, nJ - 1)];
-                const float4 pj = spos[j];
-                const float dx = pj.x - qx, dy = pj.y - qy, dz = pj.z - qz;
-                f(j0 + lane < nJ && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < Rv2 && !image_excluded(i, j, ipbc), j | (k << 12));
-            }
+        int k = 0;
+        while (r >= ccnt[L.nimg - 1 - k]) { r -= ccnt[L.nimg - 1 - k]; k++; }
+        const int i = clist[(L.nimg - 1 - k) * L.maxNA + r], ipbc = image_index(k);
+        const float4 pi = spos[i], s = at<float4>(L.shf)[k];
+        const float qx = pi.x - s.x, qy = pi.y - s.y, qz = pi.z - s.z;
+        const unsigned short* Jl = clist + k * L.maxNA;
+        const int nJ = ccnt[k];
+        for (int j0 = 0; j0 < nJ; j0 += 32) {
+            const int j = Jl[min(j0 + lane, nJ - 1)];
+            const float4 pj = spos[j];
+            const float dx = pj.x - qx, dy = pj.y - qy, dz = pj.z - qz;
+            f(j0 + lane < nJ && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < Rv2 && !image_excluded(i, j, ipbc),
+              (uint32_t)i | ((uint32_t)j << 12) | ((uint32_t)k << 24));
         }
     }
 
     // rebuild this system's lists from the current positions; false
     // (block-uniform) when they do not fit in the slot.  All threads; barriers.
-    __device__ bool list_build(const float4* spos) {
-        const float Rv = sqrtf(P.Rc2) + P.vskin, Rv2 = Rv * Rv;
-        bbox_from_smem();
-        bool any = false;
-        for (int k = 0; k < L.nimg; k++) {
-            const int ipbc = image_index(k), nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
-            any |= image_within(ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1], ipbc / (nxi * nyi) - P.npbc[2], Rv2);
+    __device__ bool list_build(const float4* spos, float Rv2) {
+        store_vp(spos);
+        build_candidates(Rv2);
+        const int* ccnt = at<int>(L.ccnt);
+        uint32_t* ent = vslot();
+        uint32_t* rows = ent + P.vcap + L.runs;
+        int R = 0;
+        for (int k = 0; k < L.nimg; k++) R += ccnt[k];
+        for (int r = warp; r < R; r += NW) {                 // entries of every row
+            int c = 0;
+            row_pass(r, spos, Rv2, [&](bool in, uint32_t) { c += __popc(__ballot_sync(0xffffffffu, in)); });
+            if (lane == 0) rows[r] = c;
         }
+        __syncthreads();
+        int* tmp = at<int>(L.red);                           // exclusive sums
+        const int r0 = (int)((long long)R * tid / T), r1 = (int)((long long)R * (tid + 1) / T);
+        int c = 0;
+        for (int r = r0; r < r1; r++) c += rows[r];
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) tmp[warp] = incl;
+        __syncthreads();
+        int base = 0, total = 0;
+        for (int w = 0; w < NW; w++) {
+            if (w < warp) base += tmp[w];
+            total += tmp[w];
+        }
+        if (total > P.vcap) return false;
+        base += incl - c;
+        for (int r = r0; r < r1; r++) { const int n = rows[r]; rows[r] = base; base += n; }
+        nlist = total;
+        __syncthreads();
+        for (int r = warp; r < R; r += NW) {                 // write (CL: the runs of this CTA)
+            const uint32_t q0 = rows[r], q1 = r + 1 < R ? rows[r + 1] : (uint32_t)total;
+            if (q0 == q1) continue;
+            uint32_t at0 = q0;
+            row_pass(r, spos, Rv2, [&](bool in, uint32_t w) {
+                const uint32_t bal = __ballot_sync(0xffffffffu, in);
+                if (in) {
+                    const uint32_t q = at0 + __popc(bal & ((1u << lane) - 1u));
+                    const uint32_t v = ((q + 1) * (uint32_t)L.runs - 1) / (uint32_t)total;      // the last run that starts at or before q
+                    if (!CL || (int)(v >> 5) % cn == cr) ent[(q - run_start(v)) * L.runs + v] = w;
+                }
+                at0 += __popc(bal);
+            });
+        }
+        __syncthreads();
+        return true;
+    }
+    __device__ __forceinline__ void store_vp(const float4* spos) {
         float* vp = at<float>(L.vp);
         for (int a = tid; a < natoms; a += T) {
             const float4 p = spos[a];
             vp[a] = p.x; vp[L.maxNA + a] = p.y; vp[2 * L.maxNA + a] = p.z;
         }
-        nlist = 0;
-        if (!any) return true;
-        build_candidates(Rv2);
-        int* rst = at<int>(L.rst);
-        for (int i = warp; i < natoms; i += NW) {            // count (CL: the rows of atoms i = cr mod cn)
-            int c = 0;
-            if (!CL || i % cn == cr) row_pass(i, spos, Rv2, [&](bool in, int) { c += __popc(__ballot_sync(0xffffffffu, in)); });
-            if (lane == 0) rst[i] = c;
-        }
-        __syncthreads();
-        if (warp == 0) {                                     // row starts
-            int run = 0;
-            for (int a0 = 0; a0 < natoms; a0 += 32) {
-                const int a = a0 + lane, ce = a < natoms ? rst[a] : 0;
-                const int c = (ce + 1) & ~1;                 // rows start at whole words
-                int incl = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                if (a < natoms) rst[a] = 2 * (run + incl - c) + (ce & 1);
-                run += __shfl_sync(0xffffffffu, incl, 31);
-            }
-            if (lane == 0) rst[natoms] = 2 * run;
-        }
-        __syncthreads();
-        const int total = rst[natoms] >> 1;
-        bool full = total > P.vcap;
-        if constexpr (CL) {
-            if (tid == 0) flags_cl()[2] = full;
-            csync();
-            full = any_cl(2);
-            csync();
-        }
-        if (full) return false;
-        // rows by falling length: the rows a warp evaluates at a time are
-        // alike (their longest sets the time), atoms without a row drop out
-        unsigned short* perm = at<unsigned short>(L.perm);
-        float4* flist = at<float4>(L.flist);
-        for (int a = tid; a < natoms; a += T) {
-            const int n = (rst[a + 1] >> 2) - (rst[a] >> 2);
-            flist[a] = make_float4(0.f, 0.f, 0.f, 0.f);
-            int rank = 0;
-            for (int o = 0, p0 = 0; o < natoms; o++) {
-                const int p1 = rst[o + 1] >> 2, m = p1 - p0;
-                rank += (m > n) || (m == n && o < a);
-                p0 = p1;
-            }
-            perm[rank] = (unsigned short)a;
-        }
-        unsigned short* ent = vslot();
-        for (int i = warp; i < natoms; i += NW) {            // write
-            int at0 = rst[i] >> 1;
-            if ((rst[i + 1] >> 1) == at0) continue;
-            row_pass(i, spos, Rv2, [&](bool in, int w) {
-                const uint32_t bal = __ballot_sync(0xffffffffu, in);
-                if (in) ent[at0 + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)w;
-                at0 += __popc(bal);
-            });
-        }
-        nlist = total;
-        __syncthreads();
-        int lo = 0, hi = natoms;                             // rows that are not empty
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1, a = perm[mid];
-            if ((rst[a + 1] >> 2) > (rst[a] >> 2)) lo = mid + 1; else hi = mid;
-        }
-        nrows = lo;
-        return true;
     }
 
-    // the listed pairs: kRowLanes lanes per atom, two entries (one word) per lane
-    // and packed operation; each atom's sum goes to flist (no atomics: the row is
-    // all of the atom's listed pairs).  The entries come from L2, several hundred
-    // cycles away: four words per lane are in flight ahead of the one evaluated,
-    // and a group's next row is fetched before it evaluates this one.  Rows hold
-    // 5 to 30 entries: with four lanes fewer of them idle at the row's end and
-    // each warp closes eight rows at once (time per system-step, eight -> four
-    // lanes: 100 atoms 0.0317 -> 0.0299 us, 200: 0.0942 -> 0.0906, 330: 0.2223 ->
-    // 0.2163, 395: 0.3008 -> 0.2933); a cluster's CTA has too few rows for that
-    // (350 atoms x 37: 0.604 with eight, 0.634 with four).
-    static constexpr int kRowLanes = CL ? 8 : 4;
+    // runs 32 g .. 32 g + 31 of the listed pairs, one per lane
     template <bool HB>
-    __device__ void list_pairs(const float4* spos, const float4* sREQ, long long* facc) {
-        constexpr int G = kRowLanes, NG = T / G, RW = 32 / G;      // lanes per row, rows of the block, of a warp
-        const int* rst = at<int>(L.rst);
-        float4* flist = at<float4>(L.flist);
-        const float4* shf = at<float4>(L.shf);
-        const uint32_t* ent = reinterpret_cast<const uint32_t*>(vslot());       // two entries a word
-        const unsigned short* perm = at<unsigned short>(L.perm);
-        const int gl = lane & (G - 1);
-        PairC C;
-        C.Rc2 = P.Rc2;
-        C.kq = pack2(-P.kq_rc2, -P.kq_rc2); C.p12 = pack2(12.f, 12.f); C.m12 = pack2(-12.f, -12.f);
-        // row: atom, words, whether the last word holds one entry, first word, and
-        // this lane's first four words
-        struct Row { int i, nw, odd; const uint32_t* p; uint32_t u[4]; };
-        auto fetch = [&](int row, Row& x) {
-            x.i = row < nrows ? (int)perm[row] : 0;
-            const int a = rst[x.i];
-            x.odd = a & 1;
-            x.nw = row < nrows ? (rst[x.i + 1] >> 2) - (a >> 2) : 0;
-            x.p = ent + (a >> 2) + gl;
-#pragma unroll
-            for (int t = 0; t < 4; t++) x.u[t] = G * t + gl < x.nw ? x.p[G * t] : 0u;
-        };
-        Row nx;
-        fetch(tid / G, nx);
-        for (int i0 = 0, k = 0; i0 < nrows; i0 += NG, k++) {
-            Row w = nx;
-            // every other round the warps take their rows in reverse order
-            if (i0 + NG < nrows) fetch(i0 + NG + ((k & 1) ? tid / G : (NG - RW) - RW * warp + (lane / G)), nx);
-            const int i = w.i, n = w.nw;
-            f32x2 fx = 0, fy = 0, fz = 0;
-            if (gl < n) {
-                const float4 pi = spos[i], Ri = sREQ[i];
-                PairI I;
-                I.x = I.y = I.z = 0;
-                I.R = pack2(Ri.x, Ri.x); I.E = pack2(Ri.y, Ri.y); I.Q = pack2(-Ri.z, -Ri.z); I.H = HB ? pack2(Ri.w, Ri.w) : 0;
-#pragma unroll 1
-                for (int t = gl; t < n; t += G) {
-                    const bool one = w.odd && t + 1 == n;                  // the word's second half is no entry
-                    const unsigned c0 = w.u[0] & 0xFFFFu, c1 = one ? c0 : w.u[0] >> 16;
-                    w.u[0] = w.u[1]; w.u[1] = w.u[2]; w.u[2] = w.u[3];
-                    w.p += G;
-                    if (t + 4 * G < n) w.u[3] = w.p[3 * G];
-                    const float4 s0 = shf[c0 >> 12], s1 = shf[c1 >> 12];
-                    const float4 p0 = spos[c0 & 0xFFFu], p1 = spos[c1 & 0xFFFu], R0 = sREQ[c0 & 0xFFFu], R1 = sREQ[c1 & 0xFFFu];
-                    PairJ J;
-                    J.x = pack2(p0.x + s0.x - pi.x, p1.x + s1.x - pi.x);
-                    J.y = pack2(p0.y + s0.y - pi.y, p1.y + s1.y - pi.y);
-                    J.z = pack2(p0.z + s0.z - pi.z, p1.z + s1.z - pi.z);
-                    J.R = pack2(R0.x, R1.x); J.E = pack2(R0.y, R1.y); J.Q = pack2(R0.z, R1.z); J.H = HB ? pack2(R0.w, R1.w) : 0;
-                    pair2<HB, COUNT>(J, I, C, false, one, fx, fy, fz, npair);
-                }
-            }
-            float3 f = make_float3(hsum2(fx), hsum2(fy), hsum2(fz));
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) {
-                f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
-                f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
-                f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
-            }
-            if (CL) {
-                if (gl == 0 && n > 0) fix_add(facc + 3 * i, f);
-            } else if (gl == 0 && n > 0) {
-                auto lim = [](float x) { return fminf(fmaxf(x, -B::kFixMax), B::kFixMax) + 0.f * x; };   // as fix_add; NaN stays
-                flist[i] = make_float4(lim(f.x), lim(f.y), lim(f.z), 0.f);
-            }
-        }
-    }
-
-    // ---- bonded terms of one node, four lanes (one per neighbour slot q) ------
-    // MMFFsp3_loc::eval_atom (MMFFsp3_loc.h:250-575), the terms of eval_atom in
-    // mmff_device.cuh.  A lane evaluates the bond, pi-pi and pi-sigma terms of its
-    // neighbour and its own end of the three angles it is part of (the other
-    // end's bond vector comes by shuffle), so no force has to travel back; the
-    // force on the node is minus the sum of the four ends' (without the 1-3
-    // pair part, which acts between the ends).  A thread per node instead is
-    // some 1000 instructions of straight-line code, which the small blocks
-    // (eight per SM in different phases) mostly wait for the instruction
-    // cache to deliver, with the lanes beyond the node count idle.
-    // All lanes of the warp call it; ia: node (ok: a real one).
-    __device__ __forceinline__ float node_par(int off, const float4* g, int n4) {
-        return B::compact() ? __ldg(reinterpret_cast<const float*>(g + noff) + n4) : at<float>(off)[n4];
-    }
-    __device__ void bonded_node(int ia, bool ok) {
+    __device__ void list_unit(int g, long long* facc) {
         const float4* spos = at<float4>(L.pos);
         const float4* sREQ = at<float4>(L.REQ);
-        const int flags = P.flags, q = lane & 3, n4 = 4 * ia + q;
-        int ing = -1, cell = 0;
-        if (ok) {
-            ing = B::compact() ? __ldg(reinterpret_cast<const int*>(Y.neighs + aoff) + n4) : at<int>(L.ng)[n4];
-            cell = B::compact() ? __ldg(reinterpret_cast<const int*>(Y.neighCell + aoff) + n4) : at<int>(L.ngC)[n4];
+        const float4* shf = at<float4>(L.shf);
+        const int v = 32 * g + lane;
+        const int n = (int)(run_start(v + 1) - run_start(v));
+        if (n <= 0) return;
+        const uint32_t* ent = vslot() + v;
+        int ci = -1;
+        float3 fi = make_float3(0.f, 0.f, 0.f);
+        float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), Ri = pi;
+        uint32_t wn = ent[0], wn2 = n > 1 ? ent[L.runs] : 0;
+        for (int e = 0; e < n; e++) {
+            const uint32_t w = wn;
+            wn = wn2;
+            if (e + 2 < n) wn2 = ent[(e + 2) * L.runs];
+            const int i = (int)(w & 0xFFFu), j = (int)((w >> 12) & 0xFFFu);
+            if (i != ci) {
+                if (ci >= 0) fix_add(facc + 3 * ci, fi);
+                ci = i; fi = make_float3(0.f, 0.f, 0.f);
+                pi = spos[i]; Ri = sREQ[i];
+            }
+            const float4 s = shf[w >> 24], pj = spos[j];
+            const float dx = pj.x + s.x - pi.x, dy = pj.y + s.y - pi.y, dz = pj.z + s.z - pi.z;
+            bool ok;
+            float en;
+            const float F = pair_force<false, HB>(dx, dy, dz, Ri, sREQ[j], false, P.Rc2, P.kq_rc2, 0.f, true, ok, en);
+            if (!ok) continue;
+            if (COUNT) npair++;
+            fi.x = fmaf(dx, F, fi.x); fi.y = fmaf(dy, F, fi.y); fi.z = fmaf(dz, F, fi.z);
         }
-        // neighbour slots end at the first empty one
-        const unsigned neg = (__ballot_sync(0xffffffffu, ing < 0) >> (lane & 28)) & 0xFu;
-        const int nbn = neg ? __ffs(neg) - 1 : 4;
-        const bool v = q < nbn;
-        const float4 apar = B::npar(L.apar, Y.apars, ia);
-        const float3 pa = f3(spos[ia]), hpi = f3(spos[natoms + ia]);
-        float3 h = make_float3(0.f, 0.f, 1.f), fb = make_float3(0.f, 0.f, 0.f), f13 = fb, fpi = fb, fps = fb;
-        float il = 1.f, l = 1.f;
-        if (v) {
-            h = f3(spos[ing]) - pa;
-            // most bonds stay in the central cell: no shift, and none of the integer
-            // divisions that name the cell (with the assembly's loads side by side:
-            // 24 atoms x 16 systems 0.337 -> 0.324 us per system-step, 60 atoms
-            // 0.0159 -> 0.0155, 330: 0.214 -> 0.212)
-            if ((flags & F_PBC) && cell != ((2 * P.npbc[1] + 1) * P.npbc[2] + P.npbc[1]) * (2 * P.npbc[0] + 1) + P.npbc[0]) {
-                const float3 c = image_cell(cell, P.npbc[0], P.npbc[1], P.npbc[2]);
-                h.x += lv[0] * c.x + lv[3] * c.y + lv[6] * c.z;
-                h.y += lv[1] * c.x + lv[4] * c.y + lv[7] * c.z;
-                h.z += lv[2] * c.x + lv[5] * c.y + lv[8] * c.z;
-            }
-            const float l2 = dot3(h, h);
-            il = rsq_nr(l2);
-            l = sqrt_from(l2, il);
-            h = h * il;
-            if (ia < ing) {
-                if (flags & F_BONDS) {
-                    float fr = (l - node_par(L.bL, Y.bLs, n4)) * node_par(L.bK, Y.bKs, n4);
-                    if (flags & F_SUB_BOND_NB) {
-                        const float4 Ri = sREQ[ia], Rj = sREQ[ing];
-                        float e, F = l * ljqh<false>(l * l, Ri.x + Rj.x, Ri.y * Rj.y, Ri.z * Rj.z, fminf(Ri.w * Rj.w, 0.f), e);
-                        if ((flags & F_CLAMP_NB) && F * F > P.Fmax2NB) F = copysignf(sqrtf(P.Fmax2NB), F);
-                        fr -= F;
-                    }
-                    fb = h * -fr;
-                }
-                const float kk = node_par(L.kpp, Y.Kpp, n4);
-                if ((flags & F_PIPI) && (ing < nnode) && (kk > 1e-6f)) {
-                    const float3 h2 = f3(spos[natoms + ing]);             // evalPiAling
-                    const float c = dot3(hpi, h2), g = c < 0.f ? -kk : kk, cc = fabsf(c);
-                    fpi = fma3(hpi, -cc, h2) * g;
-                    fps = fma3(h2, -cc, hpi) * g;
-                }
-            }
-            const float ks = node_par(L.ksp, Y.Ksp, n4);
-            if ((flags & F_PISIGMA) && (ks > 1e-6f)) {                    // evalAngleCos
-                const float c = dot3(hpi, h);
-                const float g = -ks * (c - apar.w) * 2.f;
-                fpi = fpi + fma3(hpi, -c, h) * g;
-                fb = fb + fma3(h, -c, hpi) * (g * il);
-            }
+        fix_add(facc + 3 * ci, fi);
+    }
+
+    // ---- small systems (up to 64 atoms): one warp has every pair sum ----------
+    // Lane l owns atoms l and l + 32; every atom's sum is one FP32 accumulator over the
+    // images in order.  Up to 32 atoms: atoms j in order in every image.  Above: in the
+    // central image each pair once, lane l meeting the atoms of lane l + s at rotation
+    // step s, the reactions coming back by shuffle.  Two sums per packed instruction.
+    __device__ __forceinline__ void small_excl(int a, int ipbc, bool pbc, uint32_t& lo, uint32_t& hi) {
+        lo = hi = 0;
+        if (a >= natoms) { lo = hi = ~0u; return; }
+        const int4 g = ngs(a), c = ngc(a);
+        auto set = [&](int j) { if (j >= 0) { if (j < 32) lo |= 1u << j; else hi |= 1u << (j - 32); } };
+        set(a);
+        if (!pbc || c.x == ipbc) set(g.x);
+        if (!pbc || c.y == ipbc) set(g.y);
+        if (!pbc || c.z == ipbc) set(g.z);
+        if (!pbc || c.w == ipbc) set(g.w);
+    }
+    __device__ __forceinline__ void small_rows(int a, uint32_t& lo, uint32_t& hi) const {
+        if (a >= natoms) { lo = hi = ~0u; return; }
+        lo = __ldg(xrow + a * nbw);
+        hi = nbw > 1 ? __ldg(xrow + a * nbw + 1) : ~0u;
+    }
+    // central image of 33 .. 64 atoms; m: excluded atoms of the own two
+    template <bool HB>
+    __device__ __forceinline__ void small_central(const Atom2& I, const PairC& C, uint32_t m0lo, uint32_t m0hi, uint32_t m1lo,
+                                                  uint32_t m1hi, f32x2& fx, f32x2& fy, f32x2& fz) {
+        const float4* spos = at<float4>(L.pos);
+        const float4* sREQ = at<float4>(L.REQ);
+        const int last = natoms - 1;
+        const uint32_t inv_hi = natoms >= 64 ? 0u : ~((1u << (natoms - 32)) - 1u);      // slots beyond the system
+        m0hi |= inv_hi; m1hi |= inv_hi;
+        bool ok0, ok1;
+        f32x2 dx, dy, dz;
+        {   // s = 0: (A, B) of this lane
+            const int b = min(lane + 32, last);
+            const float4 p = spos[b], R = sREQ[b];
+            const f32x2 F2 = force2<HB>(atom2(p, R, p, R), I, C, (m0hi >> lane) & 1u, true, dx, dy, dz, ok0, ok1);
+            const float F = lo2(F2);
+            if (COUNT && ok0) npair += 2;
+            fx = pack2(fmaf(lo2(dx), F, lo2(fx)), fmaf(-lo2(dx), F, hi2(fx)));
+            fy = pack2(fmaf(lo2(dy), F, lo2(fy)), fmaf(-lo2(dy), F, hi2(fy)));
+            fz = pack2(fmaf(lo2(dz), F, lo2(fz)), fmaf(-lo2(dz), F, hi2(fz)));
         }
-        if (flags & F_ANGLES) {
-            const int a13 = (ok && (flags & F_EXCL13)) ? __ldg(Y.a13 + noff + ia) : 0;
-            const Cut13 cu(P);
+        m0lo = __funnelshift_r(m0lo, m0lo, lane); m0hi = __funnelshift_r(m0hi, m0hi, lane);
+        m1lo = __funnelshift_r(m1lo, m1lo, lane); m1hi = __funnelshift_r(m1hi, m1hi, lane);
 #pragma unroll 1
-            for (int d = 1; d < 4; d++) {
-                const int p = (q + d) & 3, src = (lane & 28) | p;
-                const float3 hp = make_float3(__shfl_sync(0xffffffffu, h.x, src), __shfl_sync(0xffffffffu, h.y, src),
-                                              __shfl_sync(0xffffffffu, h.z, src));
-                const float lp = __shfl_sync(0xffffffffu, l, src);
-                const int jng = __shfl_sync(0xffffffffu, ing, src), jcell = __shfl_sync(0xffffffffu, cell, src);
-                if (!v || p >= nbn) continue;
-                const float3 hs = h + hp;                                 // evalAngleCosHalf
-                // cos and sin of the half angle with their reciprocals (no division)
-                const float c2 = dot3(hs, hs) * 0.25f, s2 = fmaxf(1.f - c2 + 1e-14f, 0.f);
-                const float rc = rsq(c2), rs = rsq(s2);
-                const float fr = il * (-0.25f * apar.z * fmaf(apar.y, sqrt_from(c2, rc), -apar.x * sqrt_from(s2, rs)) * (rc * rs));
-                fb = fb + hs * fr + h * (fr * (-2.f * c2));
-                if (flags & F_SUB_ANGLE_NB) {
-                    const float3 dp = hp * lp - h * l;
-                    // x13: the pair sum skipped this central-image pair
-                    const bool x13 = ((a13 >> angle_slot(min(q, p), max(q, p))) & 1) && (!(flags & F_PBC) || cell == jcell);
-                    float e, ep;
-                    float3 fij = dp * pair13<false>(dot3(dp, dp), sREQ[ing], sREQ[jng], x13, cu.Rc2, cu.kq, cu.rc, e, ep);
-                    if (flags & F_CLAMP_NB) { const float ff = dot3(fij, fij); if (ff > P.Fmax2NB) fij = fij * sqrtf(P.Fmax2NB / ff); }
-                    f13 = f13 + fij;
-                }
+        for (int s = 1; s <= 16; s++) {
+            const int p = (lane + s) & 31, src = (lane - s) & 31;
+            const bool half = s == 16 && lane >= 16;
+            m0lo >>= 1; m0hi >>= 1; m1lo >>= 1; m1hi >>= 1;
+            const int jb = min(p + 32, last);
+            const float4 pA = spos[p], RA = sREQ[p], pB = spos[jb], RB = sREQ[jb];
+            float3 r;
+            {   // (A, A') and (B, A'); s = 16: the second is (A', B) of lane p, done there
+                const f32x2 F = force2<HB>(atom2(pA, RA, pA, RA), I, C, (m0lo & 1u) || half, (m1lo & 1u) || s == 16, dx, dy, dz, ok0, ok1);
+                if (COUNT) npair += (ok0 ? 2 : 0) + (ok1 ? 2 : 0);
+                fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+                r.x = fmaf(-hi2(dx), hi2(F), -lo2(dx) * lo2(F));
+                r.y = fmaf(-hi2(dy), hi2(F), -lo2(dy) * lo2(F));
+                r.z = fmaf(-hi2(dz), hi2(F), -lo2(dz) * lo2(F));
             }
+            fx = pack2(lo2(fx) + __shfl_sync(0xffffffffu, r.x, src), hi2(fx));
+            fy = pack2(lo2(fy) + __shfl_sync(0xffffffffu, r.y, src), hi2(fy));
+            fz = pack2(lo2(fz) + __shfl_sync(0xffffffffu, r.z, src), hi2(fz));
+            {   // (A, B') and (B, B')
+                const f32x2 F = force2<HB>(atom2(pB, RB, pB, RB), I, C, m0hi & 1u, (m1hi & 1u) || half, dx, dy, dz, ok0, ok1);
+                if (COUNT) npair += (ok0 ? 2 : 0) + (ok1 ? 2 : 0);
+                fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+                r.x = fmaf(-lo2(dx), lo2(F), -hi2(dx) * hi2(F));
+                r.y = fmaf(-lo2(dy), lo2(F), -hi2(dy) * hi2(F));
+                r.z = fmaf(-lo2(dz), lo2(F), -hi2(dz) * hi2(F));
+            }
+            fx = pack2(lo2(fx), hi2(fx) + __shfl_sync(0xffffffffu, r.x, src));
+            fy = pack2(lo2(fy), hi2(fy) + __shfl_sync(0xffffffffu, r.y, src));
+            fz = pack2(lo2(fz), hi2(fz) + __shfl_sync(0xffffffffu, r.z, src));
         }
-        // sums over the node's four lanes
-        float3 fa = fb;
+    }
+
+    template <bool HB>
+    __device__ void small_pairs(float4* out) {
+        const float4* spos = at<float4>(L.pos);
+        const float4* sREQ = at<float4>(L.REQ);
+        const PairC C = pair_consts();
+        const bool pbc = (P.flags & F_PBC) != 0, cut = P.Rc2 > 0.f, two = natoms > 32;
+        const int npx = pbc ? P.npbc[0] : 0, npy = pbc ? P.npbc[1] : 0, npz = pbc ? P.npbc[2] : 0;
+        const int a0 = lane, a1 = lane + 32, last = natoms - 1;
+        float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        if (cut && (npx | npy | npz)) {              // the atoms' box
+            for (int i = lane; i < natoms; i += 32) {
+                const float4 p = spos[i];
+                mn[0] = fminf(mn[0], p.x); mn[1] = fminf(mn[1], p.y); mn[2] = fminf(mn[2], p.z);
+                mx[0] = fmaxf(mx[0], p.x); mx[1] = fmaxf(mx[1], p.y); mx[2] = fmaxf(mx[2], p.z);
+            }
 #pragma unroll
-        for (int o = 1; o < 4; o <<= 1) {
-            fa.x += __shfl_xor_sync(0xffffffffu, fa.x, o); fa.y += __shfl_xor_sync(0xffffffffu, fa.y, o);
-            fa.z += __shfl_xor_sync(0xffffffffu, fa.z, o);
-            fpi.x += __shfl_xor_sync(0xffffffffu, fpi.x, o); fpi.y += __shfl_xor_sync(0xffffffffu, fpi.y, o);
-            fpi.z += __shfl_xor_sync(0xffffffffu, fpi.z, o);
+            for (int k = 0; k < 3; k++) { mn[k] = wmin(mn[k]); mx[k] = wmax(mx[k]); }
         }
-        if (!ok) return;
-        float4* fasm = at<float4>(L.fasm);
-        float4* fng = at<float4>(L.fng);
-        fng[n4] = make_float4(fb.x + f13.x, fb.y + f13.y, fb.z + f13.z, 0.f);
-        fng[4 * L.maxNN + n4] = make_float4(fps.x, fps.y, fps.z, 0.f);
-        if (q == 0) fasm[ia] = make_float4(-fa.x, -fa.y, -fa.z, 0.f);
-        if (q == 1) fasm[natoms + ia] = make_float4(fpi.x, fpi.y, fpi.z, 0.f);
+        const float4 q0 = spos[min(a0, last)], q1 = spos[min(a1, last)];
+        Atom2 I = own2(q0, sREQ[min(a0, last)], q1, sREQ[min(a1, last)]);
+        f32x2 fx = 0, fy = 0, fz = 0;
+        int im = 0;
+#pragma unroll 1
+        for (int iz = -npz; iz <= npz; iz++)
+#pragma unroll 1
+            for (int iy = -npy; iy <= npy; iy++)
+#pragma unroll 1
+                for (int ix = -npx; ix <= npx; ix++, im++) {
+                    const float3 s = image_shift(lv, ix, iy, iz);
+                    const bool central = (ix | iy | iz) == 0;
+                    if (cut && !central) {
+                        const float gx = fmaxf(0.f, fabsf(s.x) - (mx[0] - mn[0]));
+                        const float gy = fmaxf(0.f, fabsf(s.y) - (mx[1] - mn[1]));
+                        const float gz = fmaxf(0.f, fabsf(s.z) - (mx[2] - mn[2]));
+                        if (gx * gx + gy * gy + gz * gz >= P.Rc2) continue;   // image out of reach (uniform)
+                    }
+                    uint32_t m0lo, m0hi, m1lo, m1hi;
+                    if (central) { small_rows(a0, m0lo, m0hi); small_rows(a1, m1lo, m1hi); }
+                    else { small_excl(a0, im, pbc, m0lo, m0hi); small_excl(a1, im, pbc, m1lo, m1hi); }
+                    if (two) {
+                        if (central) {
+                            I.x = neg2(pack2(q0.x, q1.x)); I.y = neg2(pack2(q0.y, q1.y)); I.z = neg2(pack2(q0.z, q1.z));
+                            small_central<HB>(I, C, m0lo, m0hi, m1lo, m1hi, fx, fy, fz);
+                            continue;
+                        }
+                        I.x = pack2(s.x - q0.x, s.x - q1.x); I.y = pack2(s.y - q0.y, s.y - q1.y); I.z = pack2(s.z - q0.z, s.z - q1.z);
+#pragma unroll 1
+                        for (int j = 0; j < natoms; j++) {
+                            const float4 p = spos[j], R = sREQ[j];
+                            f32x2 dx, dy, dz;
+                            bool ok0, ok1;
+                            const f32x2 F = force2<HB>(atom2(p, R, p, R), I, C, m0lo & 1u, m1lo & 1u, dx, dy, dz, ok0, ok1);
+                            if (COUNT) npair += (ok0 ? 1 : 0) + (ok1 ? 1 : 0);
+                            m0lo = (m0lo >> 1) | (m0hi << 31); m0hi >>= 1;
+                            m1lo = (m1lo >> 1) | (m1hi << 31); m1hi >>= 1;
+                            fx = fma2(dx, F, fx); fy = fma2(dy, F, fy); fz = fma2(dz, F, fz);
+                        }
+                    } else {
+                        // one atom per lane: two atoms j side by side, one sum
+                        Atom2 K = I;
+                        K.x = pack2(s.x - q0.x, s.x - q0.x); K.y = pack2(s.y - q0.y, s.y - q0.y); K.z = pack2(s.z - q0.z, s.z - q0.z);
+                        K.R = pack2(lo2(I.R), lo2(I.R)); K.E = pack2(lo2(I.E), lo2(I.E)); K.Q = pack2(lo2(I.Q), lo2(I.Q)); K.H = pack2(lo2(I.H), lo2(I.H));
+                        float3 f = make_float3(lo2(fx), lo2(fy), lo2(fz));
+#pragma unroll 1
+                        for (int j = 0; j < natoms; j += 2) {
+                            const int j1 = min(j + 1, last);
+                            f32x2 dx, dy, dz;
+                            bool ok0, ok1;
+                            const f32x2 F = force2<HB>(atom2(spos[j], sREQ[j], spos[j1], sREQ[j1]), K, C, (m0lo >> j) & 1u, (m0lo >> j1) & 1u,
+                                                       dx, dy, dz, ok0, ok1);
+                            if (COUNT) npair += (ok0 ? 1 : 0) + (ok1 && j1 > j ? 1 : 0);
+                            f.x = fmaf(lo2(dx), lo2(F), f.x); f.y = fmaf(lo2(dy), lo2(F), f.y); f.z = fmaf(lo2(dz), lo2(F), f.z);
+                            if (j1 > j) { f.x = fmaf(hi2(dx), hi2(F), f.x); f.y = fmaf(hi2(dy), hi2(F), f.y); f.z = fmaf(hi2(dz), hi2(F), f.z); }
+                        }
+                        fx = pack2(f.x, 0.f); fy = pack2(f.y, 0.f); fz = pack2(f.z, 0.f);
+                    }
+                }
+        if (a0 < natoms) out[a0] = make_float4(lo2(fx), lo2(fy), lo2(fz), 0.f);
+        if (a1 < natoms) out[a1] = make_float4(hi2(fx), hi2(fy), hi2(fz), 0.f);
     }
 
     // ------------------------------------------------------------------ forces
-    template <bool HB>
-    __device__ __forceinline__ void pairs(bool pbc, long long* facc) {
-        ordered_pairs<HB>(pbc && !(P.Rc2 > 0.f), facc);
-        if (nlist > 0) list_pairs<HB>(at<float4>(L.pos), at<float4>(L.REQ), facc);
+    // bonded terms of nodes 32 u .. 32 u + 31, one per lane
+    __device__ void bonded_unit(int u) {
+        const int ia = 32 * u + lane;
+        if (ia >= nnode) return;
+        float4* fasm = at<float4>(L.fasm);
+        float4* fng = at<float4>(L.fng);
+        BondedOut o;
+        eval_atom<false>(ia, natoms, nnode, P.flags, P.Fmax2NB, at<float4>(L.pos), at<float4>(L.REQ), ngs(ia), ngc(ia),
+                         B::npar(L.apar, Y.apars, ia), B::npar(L.bL, Y.bLs, ia), B::npar(L.bK, Y.bKs, ia),
+                         B::npar(L.ksp, Y.Ksp, ia), B::npar(L.kpp, Y.Kpp, ia), lv, P.npbc[0], P.npbc[1], P.npbc[2],
+                         __ldg(Y.a13 + noff + ia), Cut13(P), o);
+        fasm[ia] = make_float4(o.fa.x, o.fa.y, o.fa.z, 0.f);
+        fasm[natoms + ia] = make_float4(o.fpi.x, o.fpi.y, o.fpi.z, 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            fng[ia * 4 + k] = make_float4(o.fbs[k].x, o.fbs[k].y, o.fbs[k].z, 0.f);
+            fng[4 * L.maxNN + ia * 4 + k] = make_float4(o.fps[k].x, o.fps[k].y, o.fps[k].z, 0.f);
+        }
     }
 
-    // moved: some atom moved more than half the list skin since the lists were
-    // built (block-uniform, from the previous step's move)
+    // GridFF samples of atoms 8 g .. 8 g + 7, four lanes each (x-slices); the four
+    // slices are added in pairs, in small systems one after another
+    __device__ void grid_unit(int g, float4* fgr) {
+        const float4* spos = at<float4>(L.pos);
+        const int i = 8 * g + (lane >> 2), a = lane & 3;
+        const bool ok = i < natoms;
+        const int ic = ok ? i : natoms - 1;
+        const float4 p = spos[ic];
+        const float3 uu = make_float3((p.x + lv[9]) * P.ginv[0], (p.y + lv[10]) * P.ginv[1], (p.z + lv[11]) * P.ginv[2]);
+        float3 e;                            // d/dy, d/dz and value of the slice
+        float4 bx, dx;
+        if (Y.gkey != nullptr)
+            e = grid_slice_cached(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, B::plq(ic), a, ok, at<unsigned>(L.key) + ic,
+                                  Y.gkey + aoff + ic, Y.gcs + (size_t)(aoff + ic) * 16, bx, dx);
+        else
+            e = grid_slice<(T >= MMFF_UNROLL_MIN_T) ? 4 : 1>(P.grid, P.gn[0], P.gn[1], P.gn[2], uu, B::plq(ic), a, bx, dx);
+        float4 r;
+        if (L.small) {
+            r = make_float4(0.f, 0.f, 0.f, 0.f);
+            const int l0 = lane & 28;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const float ex = __shfl_sync(0xffffffffu, e.x, l0 | k), ey = __shfl_sync(0xffffffffu, e.y, l0 | k);
+                const float ez = __shfl_sync(0xffffffffu, e.z, l0 | k);
+                r.x = fmaf(comp(dx, k), ez, r.x); r.y = fmaf(comp(bx, k), ex, r.y); r.z = fmaf(comp(bx, k), ey, r.z);
+            }
+        } else {
+            r = make_float4(comp(dx, a) * e.z, comp(bx, a) * e.x, comp(bx, a) * e.y, 0.f);
+#pragma unroll
+            for (int o = 2; o > 0; o >>= 1) {
+                r.x += __shfl_xor_sync(0xffffffffu, r.x, o);
+                r.y += __shfl_xor_sync(0xffffffffu, r.y, o);
+                r.z += __shfl_xor_sync(0xffffffffu, r.z, o);
+            }
+        }
+        if (ok && a == 0) fgr[i] = make_float4(r.x * P.gmi[0], r.y * P.gmi[1], r.z * P.gmi[2], 0.f);
+    }
+
+    // all units of this step, claimed by the warps in turn, the long ones first:
+    // image rows, bonded terms, pair sums of a small system, tiles, list runs, grid
+    template <bool HB>
+    __device__ void units(long long* facc) {
+        const bool nb = (P.flags & F_NONBONDED) != 0;
+        auto mine = [&](int n) { return CL ? (n - cr + cn - 1) / cn : n; };       // units cr, cr + cn, ... of n
+        const int nI = mine(nb && image_row_path() ? (natoms + 63) >> 6 : 0);
+        const int nS = nb && L.small ? 1 : 0;
+        const int nB = (nnode + 31) >> 5;
+        const int nT = mine(nb && !L.small ? double_tiles() + single_units() + diag_units() : 0);
+        const int nL = mine(use_list ? L.runs >> 5 : 0);
+        const int nG = mine((P.flags & F_GRID) ? (natoms + 7) >> 3 : 0);
+        const int e0 = nI, e1 = e0 + nS, e2 = e1 + nB, e3 = e2 + nT, e4 = e3 + nL, e5 = e4 + nG;
+        int* claim = shared_ints() + 2 + par;
+        auto global_unit = [&](int m) { return CL ? cr + cn * m : m; };
+        while (true) {
+            int u = 0;
+            if (lane == 0) u = atomicAdd(claim, 1);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if (u >= e5) break;
+            if (u < e0) image_row_unit<HB>(global_unit(u), listf());
+            else if (u < e1) small_pairs<HB>(listf());
+            else if (u < e2) bonded_unit(u - e1);
+            else if (u < e3) tile_unit<HB>(global_unit(u - e2), facc);
+            else if (u < e4) list_unit<HB>(global_unit(u - e3), facc);
+            else grid_unit(global_unit(u - e4), gridf());
+            __syncwarp();
+        }
+    }
+
+    // moved: some atom moved more than half the list skin since the positions vp
+    // (block-uniform, from the previous step's move)
     __device__ void forces(bool moved) {
         const int flags = P.flags;
         const float4* spos = at<float4>(L.pos);
-        const bool pbc = (flags & F_PBC) != 0;
         long long* facc = sums();
+        use_list = false;
         if ((flags & F_NONBONDED) && P.Rc2 > 0.f && L.nimg > 0) {
-            if (listok && (!listed || moved)) {
-                if (COUNT && tid == 0) atomicAdd(Y.counters + 3, 1ull);
-                listok = listed = list_build(spos);
-            }
-            if (!listok) {
-                nlist = 0;
+            use_list = listok && lstate == LIST_BUILT && !moved;
+            if (!use_list && !(listok && lstate == LIST_QUIET && !moved)) {
                 bbox_from_smem();
-                bool any = false;
-                for (int k = 0; k < L.nimg; k++) {
-                    const int ipbc = image_index(k), nxi = 2 * P.npbc[0] + 1, nyi = 2 * P.npbc[1] + 1;
-                    any |= image_within(ipbc % nxi - P.npbc[0], (ipbc / nxi) % nyi - P.npbc[1], ipbc / (nxi * nyi) - P.npbc[2], P.Rc2);
-                }
-                if (any) {
-                    build_candidates(P.Rc2);
-                    if (hasH) candidate_rows<true>(spos, at<float4>(L.REQ), facc);
-                    else candidate_rows<false>(spos, at<float4>(L.REQ), facc);
-                    __syncthreads();                 // the lists share the recoil slots' memory
+                if (any_image(P.Rc2)) {
+                    const float Rv = sqrtf(P.Rc2) + P.vskin, Rv2 = Rv * Rv;
+                    if (listok) {
+                        if (COUNT && tid == 0) atomicAdd(Y.counters + 3, 1ull);
+                        use_list = listok = list_build(spos, Rv2);
+                        lstate = LIST_BUILT;
+                    }
+                    if (!listok) {
+                        __syncthreads();
+                        build_candidates(P.Rc2);
+                        if (hasH) candidate_units<true>(spos, facc);
+                        else candidate_units<false>(spos, facc);
+                        __syncthreads();                 // the lists share the recoil slots' memory
+                    }
+                } else if (listok && lstate != LIST_BUILT) {
+                    // nothing in reach: no need to look again until an atom has moved
+                    const float Rv = sqrtf(P.Rc2) + P.vskin;
+                    lstate = any_image(Rv * Rv) ? LIST_NONE : LIST_QUIET;
+                    if (lstate == LIST_QUIET) store_vp(spos);
                 }
             }
-            if (COUNT && tid == 0 && listok) atomicAdd(Y.counters + 4, (unsigned long long)nlist);
+            if (COUNT && tid == 0 && use_list) atomicAdd(Y.counters + 4, (unsigned long long)nlist);
         }
-        // Bonded terms and GridFF samples in units of one warp (eight nodes, or
-        // eight atoms), dealt to the warps in turn; nothing waits between these
-        // units and the pairs.
-        float4* fgr = at<float4>(L.fgrid);
-        const int nB = (nnode + 7) >> 3, nG = (flags & F_GRID) ? (natoms + 7) >> 3 : 0;
-#pragma unroll 1
-        for (int u = warp; u < nB; u += NW) {
-            const int ia = 8 * u + (lane >> 2);
-            bonded_node(min(ia, nnode - 1), ia < nnode);
-        }
-        double d0 = 0.0;
-        if constexpr (CL) {
-#pragma unroll 1
-            for (int u = cr + cn * warp; u < nG; u += cn * NW) {
-                B::template grid_phase<false, true>(32 * u + lane, 1 << 30, fgr, d0);
-                __syncwarp();
-                const int a = 8 * u + lane;
-                if (lane < 8 && a < natoms) fix_add(facc + 3 * a, f3(fgr[a]));
-            }
-        } else {
-#pragma unroll 1
-            for (int u = (warp + NW - nB % NW) % NW; u < nG; u += NW)
-                B::template grid_phase<false, true>(32 * u + lane, 1 << 30, fgr, d0);
-        }
-        if (flags & F_NONBONDED) {
-            if (hasH) pairs<true>(pbc, facc);
-            else pairs<false>(pbc, facc);
-        }
-        // direct substrate term (getSurfMorse), one thread per atom
+        if (hasH) units<true>(facc);
+        else units<false>(facc);
+        // direct substrate term (getSurfMorse), one thread per atom (never in a cluster)
         if (flags & F_SURF) {
             __syncthreads();
+            float4* fgr = gridf();
             const float4* sR = at<float4>(L.REQ);
             for (int a = tid; a < natoms; a += T) {
                 const float4 p = spos[a];
                 const float4 r = surf_atom(P, make_float3(p.x + lv[9], p.y + lv[10], p.z + lv[11]), sR[a]);
-                const float4 g = (!CL && (flags & F_GRID)) ? fgr[a] : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 g = (flags & F_GRID) ? fgr[a] : make_float4(0.f, 0.f, 0.f, 0.f);
                 fgr[a] = make_float4(g.x + r.x, g.y + r.y, g.z + r.z, 0.f);
             }
         }
-        if (CL && pairbad) flags_cl()[par] = 1;
+        if (CL && pairbad) shared_ints()[par] = 1;
+    }
+    template <bool HB>
+    __device__ void candidate_units(const float4* spos, long long* facc) {
+        const float4* sREQ = at<float4>(L.REQ);
+        float ec = 0.f;
+        const int n = B::image_tile_count();
+        for (int u = cr * NW + warp; u < n; u += cn * NW) B::template image_tile_unit<HB>(u, spos, sREQ, facc, ec);
+        B::template image_rows<HB>(cr * T + tid, cn * T, spos, sREQ, true, facc, ec);
     }
 
     // ---------------------------------------------------------------- assemble
@@ -745,8 +786,9 @@ struct RelaxEngine : CtaSystem<T> {
     __device__ void assemble(double& vf, double& vv, double& ff, float& fmax2, bool& bad) {
         float4* fasm = at<float4>(L.fasm);
         long long* facc = sums();
-        const float4* fgr = at<float4>(L.fgrid);
-        const float4* flist = at<float4>(L.flist);
+        float4* fgr = gridf();
+        float4* flist = listf();
+        const bool with_list = has_listf(), with_grid = (P.flags & (F_GRID | F_SURF)) != 0;
         const float4* fng = at<float4>(L.fng);
         const float4* spos = at<float4>(L.pos);
         const float4* svel = B::vels();
@@ -757,9 +799,8 @@ struct RelaxEngine : CtaSystem<T> {
             float3 f = make_float3(0.f, 0.f, 0.f);
             if (pi || v < nnode) f = f3(fasm[v]);
             if (!pi) {
-                if (P.flags & (CL ? F_SURF : F_GRID | F_SURF)) f = f + f3(fgr[v]);
-                if (!CL && nlist > 0) f = f + f3(flist[v]);
                 long long s[3] = {0, 0, 0};
+                float3 b = make_float3(0.f, 0.f, 0.f), g = b;
                 if constexpr (CL) {
                     for (int c = 0; c < cn; c++) {
                         const long long* q = cooperative_groups::this_cluster().map_shared_rank(facc, c) + 3 * v;
@@ -767,13 +808,18 @@ struct RelaxEngine : CtaSystem<T> {
                     }
                     long long* z = at<long long>(L.facc) + (par ^ 1) * 3 * L.maxNA + 3 * v;
                     z[0] = 0; z[1] = 0; z[2] = 0;
+                    // (the owners of the atom's image row and grid sample)
+                    if (with_list) b = f3(cooperative_groups::this_cluster().map_shared_rank(flist, (v >> 6) % cn)[v]);
+                    if (with_grid) g = f3(cooperative_groups::this_cluster().map_shared_rank(fgr, (v >> 3) % cn)[v]);
                 } else {
                     s[0] = facc[3 * v]; s[1] = facc[3 * v + 1]; s[2] = facc[3 * v + 2];
                     facc[3 * v] = 0; facc[3 * v + 1] = 0; facc[3 * v + 2] = 0;
+                    if (with_list) b = f3(flist[v]);
+                    if (with_grid) g = f3(fgr[v]);
                 }
-                f.x += (float)s[0] * (1.f / kFix);
-                f.y += (float)s[1] * (1.f / kFix);
-                f.z += (float)s[2] * (1.f / kFix);
+                f.x = f.x + ((float)s[0] * (1.f / kFix) + b.x) + g.x;
+                f.y = f.y + ((float)s[1] * (1.f / kFix) + b.y) + g.y;
+                f.z = f.z + ((float)s[2] * (1.f / kFix) + b.z) + g.z;
             }
             const int4 bk = bks(ia);
             const int bks[4] = {bk.x, bk.y, bk.z, bk.w};
@@ -807,13 +853,10 @@ struct RelaxEngine : CtaSystem<T> {
             fmax2 = fmaxf(fmax2, (float)f2);
             bad |= !isfinite(f.x + f.y + f.z);
         }
-        if constexpr (CL) {
-            bad |= any_cl(par);
-            if (tid == 0) flags_cl()[par ^ 1] = 0;
-            par ^= 1;
-        } else {
-            bad |= pairbad;
-        }
+        if (CL) bad |= any_cl(par);
+        else bad |= pairbad;
+        if (tid == 0) { shared_ints()[par ^ 1] = 0; shared_ints()[2 + (par ^ 1)] = 0; }
+        par ^= 1;
     }
 
     // block reduction of 3 doubles + one float max (+flag); result in all threads
@@ -839,11 +882,9 @@ struct RelaxEngine : CtaSystem<T> {
     }
 
     // -------------------------------------------------------------------- move
-    // a moved atom: its copy in the pair arrays, and whether it left the
-    // neighbourhood (half the skin) of its position at the lists' build
+    // whether a moved atom left the neighbourhood (half the skin) of its position vp
     __device__ __forceinline__ bool moved_atom(int v, float3 p) {
-        soa(0)[v] = p.x; soa(1)[v] = p.y; soa(2)[v] = p.z;
-        if (!listed) return false;
+        if (lstate == LIST_NONE) return false;
         const float* vp = at<float>(L.vp);
         const float dx = p.x - vp[v], dy = p.y - vp[L.maxNA + v], dz = p.z - vp[2 * L.maxNA + v];
         return !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= 0.25f * P.vskin * P.vskin);

@@ -85,10 +85,10 @@ struct Bucket {
     SmemLayout lay, elay;          // CTA kernels: shared-memory layouts of relaxation and evaluation
     int cn = 1;                    // relaxation by clusters of cn CTAs per system (> 1), with layout clay
     SmemLayout clay;
-    // CTA relax kernels with a cutoff and a 2-D cell: scratch for the shifted-image
-    // pair lists, vcap entries per resident CTA (0: none)
-    DBuf<unsigned short> vl;
-    int vcap = 0;
+    // relax kernels with a cutoff and a 2-D cell: scratch for the shifted-image pair
+    // lists, vstride words per resident CTA for at most vcap entries (0: none)
+    DBuf<uint32_t> vl;
+    int vstride = 0, vcap = 0;
 };
 
 // autotuned launch configuration of one size class (kind -1: default_config;
@@ -305,8 +305,9 @@ int cluster_size(Bucket& B, int nimg, int dev_smem) {
     B.cn = 1;
     const int n = (int)B.sys.size();
     void* fn = relax_cluster_fn(B.T);
-    if (W.force_T || !fn || B.maxNA <= kClusterMinAtoms || 2 * W.nsys > W.nsm) return 0;
+    if (W.force_T || !fn || B.maxNA <= kClusterMinAtoms || 2 * W.nsys > W.nsm || (W.flags & F_SURF)) return 0;
     B.clay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 2);
+    B.clay.runs = B.lay.runs;
     if (B.clay.total > dev_smem || B.clay.vel < 0) return 0;
     if (set_smem_limit(fn, B.clay.total)) return -1;
     for (int c = std::min(8, W.nsm / W.nsys); c >= 2; c--) {
@@ -329,10 +330,18 @@ int config_bucket(Bucket& B, int T, int S) {
     const int nimg = W.Rcut > 0 ? shifted_images(W.flags, W.npbc) : 0;
     void* fns[3];
     B.T = T; B.S = S;
-    B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 1);
+    // the order of the pair sums goes by the system's size class alone (mmff_relax.cu)
+    const bool small = !W.force_T && B.maxNA <= 64;
+    const int runs = kClassT[std::max(0, size_class(B.maxNA) - 2)];
+    auto layout = [&](int mode) {
+        SmemLayout l = smem_layout(B.maxNA, B.maxNN, B.T, small ? 0 : nimg, mode);
+        l.small = small; l.runs = runs;
+        return l;
+    };
+    B.lay = layout(1);
     if (B.lay.total > dev_smem && B.T < kCompactMinThreads) {     // only the larger blocks leave arrays in global memory
         B.T = kCompactMinThreads;
-        B.lay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 1);
+        B.lay = layout(1);
     }
     B.smem = B.lay.total;
     fns[0] = relax_fn(B.T, false); fns[1] = relax_fn(B.T, true); fns[2] = relax_explore_fn(B.T);
@@ -361,10 +370,11 @@ int config_bucket(Bucket& B, int T, int S) {
     if (occ < 1) return fail("kernel cannot be resident (T=%d smem=%d)", B.T, B.smem);
     B.grid = std::min((int)B.sys.size(), occ * W.nsm);
     if (cluster_size(B, nimg, dev_smem)) return -1;
-    B.vcap = 0;
-    if (nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
-        B.vcap = B.maxNA * kListEntriesPerAtom;      // even: rows are read by words
-        if (B.vl.ensure((size_t)std::max(B.grid, B.cn > 1 ? (int)B.sys.size() * B.cn : 0) * B.vcap)) return -1;
+    B.vcap = B.vstride = 0;
+    if (!small && nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
+        B.vcap = B.maxNA * kListEntriesPerAtom;
+        B.vstride = B.vcap + runs + nimg * B.maxNA;
+        if (B.vl.ensure((size_t)std::max(B.grid, B.cn > 1 ? (int)B.sys.size() * B.cn : 0) * B.vstride)) return -1;
     }
     if (B.queue.ensure(B.sys.size())) return -1;
     CK(cudaMemcpy(B.queue.p, B.sys.data(), B.sys.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -583,6 +593,7 @@ void set_lists(Params& P, const Bucket& B) {
     const bool on = W.pair_lists && B.vcap > 0 && B.vl.p;
     P.vlist = on ? B.vl.p : nullptr;
     P.vcap = on ? B.vcap : 0;
+    P.vstride = B.vstride;
     P.vskin = (float)W.list_skin;
 }
 
