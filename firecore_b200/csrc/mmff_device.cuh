@@ -758,8 +758,10 @@ struct SmemLayout {
     int stage;
     // relaxation kernels only (-1 otherwise): pair forces that are no fixed-point
     // sums (flist); with pair lists: the positions they were built at (3 arrays) and
-    // the images' shifts
-    int flist, vp, shf;
+    // the images' shifts; positions and pair parameters by pairs of blocks (pj) and
+    // atom after atom (soa)
+    int flist, vp, shf, pj, soa;
+    int fbuf;                           // relaxation, few systems of up to 32 atoms: scalar pair forces [image][j][32]
     int small;                          // relaxation: pair sums and grid in the order of the small systems (mmff_relax.cu)
     int runs;                           // relaxation: runs that the pair lists are cut into
 };
@@ -790,7 +792,11 @@ constexpr int kImageTileMinThreads = 128;
 constexpr int kListMaxImages = 12;
 constexpr int kListEntriesPerAtom = 48;
 
-__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, int mode, int lvl) {
+// a relaxation's pair sums (mmff_relax.cu): the pair arrays they read, and whether some
+// are no fixed-point sums
+enum : int { PAIRS_BLOCKS = 1, PAIRS_ATOMS = 2, PAIRS_SUMS = 4 };
+
+__host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, int nimg, int mode, int lvl, int forms) {
     SmemLayout L;
     const bool relax = mode > 0;
     L.maxNA = maxNA; L.maxNN = maxNN; L.maxNV = maxNA + maxNN; L.nwarps = T / 32;
@@ -841,10 +847,13 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
         }
     }
     L.facc = take(8 * 3 * maxNA * (mode == 2 ? 2 : 1));
-    L.flist = relax ? take(16 * maxNA * (mode == 2 ? 2 : 1)) : -1;
+    L.flist = (forms & PAIRS_SUMS) && lvl < 3 ? take(16 * maxNA * (mode == 2 ? 2 : 1)) : -1;
     const bool lists = relax && nimg > 0 && nimg <= kListMaxImages;
     L.vp = lists ? take(4 * 3 * maxNA) : -1;
     L.shf = lists ? take(16 * nimg) : -1;
+    L.pj = forms & PAIRS_BLOCKS ? take(2048 * ((L.nwords + 1) / 2)) : -1;
+    L.soa = (forms & PAIRS_ATOMS) && lvl < 3 ? take(4 * 7 * 32 * L.nwords) : -1;
+    L.fbuf = -1;
     L.small = 0; L.runs = 0;
     L.total = o;
     return L;
@@ -855,13 +864,15 @@ __host__ __device__ inline SmemLayout smem_layout_(int maxNA, int maxNN, int T, 
 // force sums).  Level 0: all in
 // shared memory; 1: topology and node parameters in global memory (above);
 // 2 (relaxation, when level 1 exceeds the CTA's limit): the velocities too,
-// which only the thread that owns a vector reads and writes.
+// which only the thread that owns a vector reads and writes; 3 (when level 2
+// exceeds it): the pair forces beside the fixed-point sums, in the system's part of the
+// force output, and no pair array atom after atom.
 constexpr int kSmemMax = 227 * 1024;
-__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg, int mode) {
-    SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, mode, 0);
+__host__ __device__ inline SmemLayout smem_layout(int maxNA, int maxNN, int T, int nimg, int mode, int forms = 0) {
+    SmemLayout L = smem_layout_(maxNA, maxNN, T, nimg, mode, 0, forms);
     if (T >= kCompactMinThreads && L.total > kCompactAbove) {
-        L = smem_layout_(maxNA, maxNN, T, nimg, mode, 1);
-        if (mode == 1 && L.total > kSmemMax) L = smem_layout_(maxNA, maxNN, T, nimg, mode, 2);
+        L = smem_layout_(maxNA, maxNN, T, nimg, mode, 1, forms);
+        for (int lvl = 2; lvl <= 3 && mode == 1 && L.total > kSmemMax; lvl++) L = smem_layout_(maxNA, maxNN, T, nimg, mode, lvl, forms);
     }
     return L;
 }

@@ -39,9 +39,24 @@ __device__ __forceinline__ float3 image_shift(const float* lv, int ix, int iy, i
                        lv[2] * ix + lv[5] * iy + lv[8] * iz);
 }
 
-template <int T>
+// G: systems of a CTA, T threads each, with barriers of their own
+template <int T, int G = 1>
 struct CtaSystem {
     static_assert(T % 32 == 0, "whole warps");
+    static __device__ __forceinline__ int group() { return G == 1 ? 0 : threadIdx.x / T; }
+    static __device__ __forceinline__ void sync() {
+        if (G == 1) __syncthreads();
+        else if (T == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + group()), "n"(T) : "memory");
+    }
+    static __device__ __forceinline__ bool sync_or(int p) {
+        if (G == 1) return __syncthreads_or(p) != 0;
+        if (T == 32) return __any_sync(0xffffffffu, p) != 0;
+        int r;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                     : "=r"(r) : "r"(p), "r"(1 + group()), "n"(T) : "memory");
+        return r != 0;
+    }
     const Params& P;
     const Systems& Y;
     const SmemLayout& L;        // kernel parameter: its offsets come from the constant bank
@@ -60,7 +75,7 @@ struct CtaSystem {
 
     __device__ CtaSystem(const Params& p, const Systems& y, char* smem, const SmemLayout& l)
         : P(p), Y(y), L(l), sm(smem) {
-        tid = threadIdx.x; lane = tid & 31; warp = tid >> 5;
+        tid = G == 1 ? threadIdx.x : threadIdx.x % T; lane = tid & 31; warp = tid >> 5;
         lv = at<float>(L.sysc);
     }
     template <class X> __device__ __forceinline__ X* at(int off) { return reinterpret_cast<X*>(sm + off); }
@@ -113,8 +128,8 @@ struct CtaSystem {
                 at<int4>(L.bk)[a] = Y.bkneighs[aoff + a];
             }
         }
-        hasH = __syncthreads_or(h & 1) != 0;
-        hasX = __syncthreads_or(h & 2) != 0;
+        hasH = sync_or(h & 1);
+        hasX = sync_or(h & 2);
         if (full)
             for (int n = tid; n < nnode; n += T) {
                 at<float4>(L.apar)[n] = Y.apars[noff + n]; at<float4>(L.bL)[n] = Y.bLs[noff + n];
@@ -143,7 +158,7 @@ struct CtaSystem {
 #pragma unroll
             for (int k = 0; k < 3; k++) { red[6 * warp + k] = mn[k]; red[6 * warp + 3 + k] = mx[k]; }
         }
-        __syncthreads();
+        sync();
         float a[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, b[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
         for (int w = 0; w < L.nwarps; w++) {
 #pragma unroll
@@ -203,7 +218,7 @@ struct CtaSystem {
                         k++;
                     }
         }
-        __syncthreads();
+        sync();
         for (int k = warp; k < L.nimg; k += L.nwarps) {
             int run = 0;
             for (int w0 = 0; w0 < nw; w0 += 32) {
@@ -221,7 +236,7 @@ struct CtaSystem {
             }
             if (lane == 0) cnt[k] = run;
         }
-        __syncthreads();
+        sync();
         for (int j = tid; j < natoms; j += T) {
             const int w = j >> 5;
             const uint32_t below = (1u << (j & 31)) - 1u;
@@ -230,7 +245,7 @@ struct CtaSystem {
                 if ((m >> (j & 31)) & 1u) list[k * L.maxNA + pref[k * nw + w] + __popc(m & below)] = (unsigned short)j;
             }
         }
-        __syncthreads();
+        sync();
     }
 
     // excluded pair of the shifted image ipbc (NBFF::evalLJQs_ng4_PBC_atom,
@@ -255,9 +270,16 @@ struct CtaSystem {
         pairbad |= !isfinite(f.x + f.y + f.z);
         const float x = fminf(fmaxf(f.x, -kFixMax), kFixMax), y = fminf(fmaxf(f.y, -kFixMax), kFixMax);
         const float z = fminf(fmaxf(f.z, -kFixMax), kFixMax);
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 0), (unsigned long long)__float2ll_rn(x * kFix));
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 1), (unsigned long long)__float2ll_rn(y * kFix));
-        atomicAdd(reinterpret_cast<unsigned long long*>(a + 2), (unsigned long long)__float2ll_rn(z * kFix));
+        add64(a + 0, __float2ll_rn(x * kFix));
+        add64(a + 1, __float2ll_rn(y * kFix));
+        add64(a + 2, __float2ll_rn(z * kFix));
+    }
+    // 64-bit add in shared memory by two 32-bit ones (the hardware's; a 64-bit one is a
+    // compare-and-swap loop): whoever makes the low word wrap carries
+    static __device__ __forceinline__ void add64(long long* a, long long v) {
+        unsigned* w = reinterpret_cast<unsigned*>(a);
+        const unsigned lo = (unsigned)v, old = atomicAdd(w, lo);
+        atomicAdd(w + 1, (unsigned)((unsigned long long)v >> 32) + (old + lo < old ? 1u : 0u));
     }
 
     // bonded terms of nodes tid, tid + nt, ... by threads tid < nt; caps get a zero own-force

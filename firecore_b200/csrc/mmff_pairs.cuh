@@ -9,10 +9,10 @@ namespace mmff {
 
 // T threads, S lanes per atom on the ordered rows; ENERGY: pair energies too;
 // COUNT: counts the pair-images; TILES: long candidate lists as tiles (else rows only)
-template <int T, int S, bool ENERGY, bool COUNT = false, bool TILES = (T >= kImageTileMinThreads)>
-struct PairEngine : CtaSystem<T> {
+template <int T, int S, bool ENERGY, bool COUNT = false, bool TILES = (T >= kImageTileMinThreads), int G = 1>
+struct PairEngine : CtaSystem<T, G> {
     static_assert(32 % S == 0, "bad tile");
-    using B = CtaSystem<T>;
+    using B = CtaSystem<T, G>;
     using B::P; using B::Y; using B::L; using B::sm; using B::tid; using B::lane; using B::warp;
     using B::natoms; using B::lv; using B::hasH; using B::xrow; using B::nbw;
     using B::ngs; using B::ngc; using B::fix_add;

@@ -38,6 +38,8 @@ void* relax_fn(int T, bool count);
 void* eval_fn(int T, int S, bool energy);
 void* relax_explore_fn(int T);
 void* relax_cluster_fn(int T);
+void* relax_group_fn(int T);
+int relax_group(int T);
 void* eval_warp_fn(int apl, bool energy);
 
 }  // namespace mmff
@@ -83,6 +85,7 @@ struct Bucket {
     // evaluation: eT threads and S lanes per atom per CTA, or (eapl > 0) a warp per system
     int eT = 0, eapl = 0, esmem = 0;
     SmemLayout lay, elay;          // CTA kernels: shared-memory layouts of relaxation and evaluation
+    int group = 1, ggrid = 0;      // plain relaxation: systems per CTA (> 1: grouped kernel), its CTAs
     int cn = 1;                    // relaxation by clusters of cn CTAs per system (> 1), with layout clay
     SmemLayout clay;
     // relax kernels with a cutoff and a 2-D cell: scratch for the shifted-image pair
@@ -306,7 +309,7 @@ int cluster_size(Bucket& B, int nimg, int dev_smem) {
     const int n = (int)B.sys.size();
     void* fn = relax_cluster_fn(B.T);
     if (W.force_T || !fn || B.maxNA <= kClusterMinAtoms || 2 * W.nsys > W.nsm || (W.flags & F_SURF)) return 0;
-    B.clay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 2);
+    B.clay = smem_layout(B.maxNA, B.maxNN, B.T, nimg, 2, PAIRS_BLOCKS | (W.Rcut <= 0 && shifted_images(W.flags, W.npbc) > 0 ? PAIRS_ATOMS | PAIRS_SUMS : 0));
     B.clay.runs = B.lay.runs;
     if (B.clay.total > dev_smem || B.clay.vel < 0) return 0;
     if (set_smem_limit(fn, B.clay.total)) return -1;
@@ -316,6 +319,26 @@ int cluster_size(Bucket& B, int nimg, int dev_smem) {
         if (cudaOccupancyMaxActiveClusters(&active, fn, &l.c) != cudaSuccess) { cudaGetLastError(); continue; }
         if (active >= n) { B.cn = c; break; }
     }
+    return 0;
+}
+
+// Systems per CTA of a bucket's plain relaxation.  Up to 128 threads per system an
+// SM holds 4 to 16 systems in different phases of a step, and each scheduler's warps
+// mostly waited for the instruction cache (2 to 3 of 7 stalled warps); as one block
+// that steps together they share it (0.25).  Time per system-step, a block each /
+// grouped: 28 atoms 0.0084 -> 0.0076 us, 60: 0.0260 -> 0.0193, 100: 0.0503 -> 0.0410.  With
+// fewer systems than fill every SM's block they are better spread over the SMs.
+int group_size(Bucket& B, int dev_smem) {
+    B.group = 1;
+    const int g = relax_group(B.T);
+    void* fn = relax_group_fn(B.T);
+    if (W.force_T || !fn || B.cn > 1 || (int)B.sys.size() < g * W.nsm || g * B.smem > dev_smem) return 0;
+    if (set_smem_limit(fn, g * B.smem)) return -1;
+    int occ = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, B.T * g, g * B.smem));
+    if (occ < 1) return 0;
+    B.group = g;
+    B.ggrid = std::min(((int)B.sys.size() + g - 1) / g, occ * W.nsm);
     return 0;
 }
 
@@ -333,9 +356,14 @@ int config_bucket(Bucket& B, int T, int S) {
     // the order of the pair sums goes by the system's size class alone (mmff_relax.cu)
     const bool small = !W.force_T && B.maxNA <= 64;
     const int runs = kClassT[std::max(0, size_class(B.maxNA) - 2)];
+    const bool rows = W.Rcut <= 0 && shifted_images(W.flags, W.npbc) > 0;      // image rows, atom after atom
+    const int forms = small ? PAIRS_SUMS | (B.maxNA <= 32 ? PAIRS_ATOMS : PAIRS_BLOCKS) : PAIRS_BLOCKS | (rows ? PAIRS_ATOMS | PAIRS_SUMS : 0);
     auto layout = [&](int mode) {
-        SmemLayout l = smem_layout(B.maxNA, B.maxNN, B.T, small ? 0 : nimg, mode);
+        SmemLayout l = smem_layout(B.maxNA, B.maxNN, B.T, small ? 0 : nimg, mode, forms);
         l.small = small; l.runs = runs;
+        // few systems: all warps share the pair forces of a small one
+        const int fbytes = 4 * 32 * B.maxNA * (1 + shifted_images(W.flags, W.npbc));
+        if (small && B.maxNA <= 32 && B.T >= 128 && l.total + fbytes <= dev_smem / 2) { l.fbuf = l.total; l.total += fbytes; }
         return l;
     };
     B.lay = layout(1);
@@ -370,11 +398,12 @@ int config_bucket(Bucket& B, int T, int S) {
     if (occ < 1) return fail("kernel cannot be resident (T=%d smem=%d)", B.T, B.smem);
     B.grid = std::min((int)B.sys.size(), occ * W.nsm);
     if (cluster_size(B, nimg, dev_smem)) return -1;
+    if (group_size(B, dev_smem)) return -1;
     B.vcap = B.vstride = 0;
     if (!small && nimg > 0 && nimg <= kListMaxImages && B.maxNA <= 4096) {
         B.vcap = B.maxNA * kListEntriesPerAtom;
         B.vstride = B.vcap + runs + nimg * B.maxNA;
-        if (B.vl.ensure((size_t)std::max(B.grid, B.cn > 1 ? (int)B.sys.size() * B.cn : 0) * B.vstride)) return -1;
+        if (B.vl.ensure((size_t)std::max({B.grid, B.cn > 1 ? (int)B.sys.size() * B.cn : 0, B.group * B.ggrid}) * B.vstride)) return -1;
     }
     if (B.queue.ensure(B.sys.size())) return -1;
     CK(cudaMemcpy(B.queue.p, B.sys.data(), B.sys.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -618,6 +647,9 @@ int enqueue_relax(const Params& P) {
             void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.clay};
             ClusterLaunch l(nq * B.cn, B.T, B.clay.total, B.cn, st);
             CK(cudaLaunchKernelExC(&l.c, relax_cluster_fn(B.T), args));
+        } else if (B.group > 1 && P.md_mode != 2 && !W.count) {
+            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
+            CK(cudaLaunchKernel(relax_group_fn(B.T), dim3(B.ggrid), dim3(B.T * B.group), args, B.group * B.smem, st));
         } else {
             void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
             CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
