@@ -1,6 +1,6 @@
 // mmff_eval.cu -- one force (and energy) evaluation of every system, one CTA
-// per system (systems of more than 64 atoms, or any size with forced launch
-// shapes), and the grid sampler.
+// per system (systems of more than 64 atoms, batches of no more systems than
+// SMs, or any size with forced launch shapes), and the grid sampler.
 //
 //   phase 1  bonded terms (thread per node), non-bonded pairs (32 x 32 tiles,
 //            each unordered pair once) and the B-spline GridFF sample (4 lanes
@@ -217,7 +217,14 @@ __global__ void __launch_bounds__(T) eval_kernel(Params P, Systems Y, const int*
     // (the host passes Flim <= 0 here: eval reports unclamped forces)
     float fmax2 = 0.f;
     E.assemble(fmax2);
+    float* wm = E.template at<float>(L.red);          // largest force of the system, by warps
+    fmax2 = wmax(fmax2);
+    if (E.lane == 0) wm[E.warp] = fmax2;
     __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < T / 32; w++) fmax2 = fmaxf(fmax2, wm[w]);
+        Y.fconv[s] = sqrtf(fmax2);
+    }
     const float4* fasm = E.template at<float4>(L.fasm);
     for (int v = threadIdx.x; v < E.nvecs; v += T) Y.force[E.voff + v] = fasm[v];
     if (ENERGY) {
@@ -233,7 +240,6 @@ __global__ void __launch_bounds__(T) eval_kernel(Params P, Systems Y, const int*
         E.reduce4(x13, z0, z1, dummy, b2);
         if (threadIdx.x == 0) Y.energy[s] = make_double4(eb - x13, enb + x13, eg, eb + enb + eg);
     }
-    if (threadIdx.x == 0) Y.fconv[s] = sqrtf(fmax2);
 }
 
 // B-spline sample of n points (grid parity tests): fe = (Fx, Fy, Fz, E)
