@@ -39,6 +39,40 @@ struct Engine : PairEngine<T, S, ENERGY> {
         return par < now ? Tb : T;
     }
 
+    // pair forces of every atom as plain FP32 sums, a thread per atom over the images and
+    // atoms j in order: for systems with a force beyond the fixed-point sums' range (atoms
+    // on top of one another), whose clamped terms would lose its size and direction
+    __device__ void plain_pairs(float4* fnb, bool pbc, int central) {
+        const float4* spos = at<float4>(L.pos);
+        const float4* sREQ = at<float4>(L.REQ);
+        const int npx = pbc ? P.npbc[0] : 0, npy = pbc ? P.npbc[1] : 0, npz = pbc ? P.npbc[2] : 0;
+        const float Rc2 = P.Rc2 > 0.f ? P.Rc2 : 3.0e38f;
+        for (int i = tid; i < natoms; i += T) {
+            const float4 pi = spos[i], Ri = sREQ[i];
+            float3 f = make_float3(0.f, 0.f, 0.f);
+            int ipbc = 0;
+            for (int iz = -npz; iz <= npz; iz++) for (int iy = -npy; iy <= npy; iy++) for (int ix = -npx; ix <= npx; ix++, ipbc++) {
+                if (ipbc != central && !image_active(ix, iy, iz)) continue;
+                const float3 s = image_shift(lv, ix, iy, iz);
+                for (int j = 0; j < natoms; j++) {
+                    const bool ex = ipbc == central ? (__ldg(B::xrow + i * B::nbw + (j >> 5)) >> (j & 31)) & 1u
+                                                    : B::image_excluded(i, j, ipbc);
+                    const float4 pj = spos[j];
+                    const float dx = pj.x + s.x - pi.x, dy = pj.y + s.y - pi.y, dz = pj.z + s.z - pi.z;
+                    bool ok;
+                    float e;
+                    const float F = hasH ? pair_force<false, true>(dx, dy, dz, Ri, sREQ[j], ex, Rc2, P.kq_rc2, 0.f, true, ok, e)
+                                         : pair_force<false, false>(dx, dy, dz, Ri, sREQ[j], ex, Rc2, P.kq_rc2, 0.f, true, ok, e);
+                    f.x = fmaf(dx, F, f.x); f.y = fmaf(dy, F, f.y); f.z = fmaf(dz, F, f.z);
+                }
+            }
+            fnb[i] = make_float4(f.x, f.y, f.z, 0.f);
+        }
+    }
+    // Some term may have been clamped (2^20 eV/A): then the outermost of the atoms on top of
+    // one another has a total of that size, as nothing pushes it back; or some was not finite.
+    static constexpr float kPlainAbove = 65536.f;
+
     // ------------------------------------------------------------------ phase 1
     // returns this thread's energy contributions (only meaningful if ENERGY)
     __device__ void forces(double& Eb, double& Enb, double& Eg) {
@@ -86,9 +120,15 @@ struct Engine : PairEngine<T, S, ENERGY> {
                 if (ENERGY) Enb += (double)ec;
             }
             __syncthreads();
-            for (int a = tid; a < natoms; a += T)
-                fnb[a] = make_float4((float)facc[3 * a] * (1.f / kFix), (float)facc[3 * a + 1] * (1.f / kFix),
-                                     (float)facc[3 * a + 2] * (1.f / kFix), 0.f);
+            bool beyond = pairbad;
+            for (int a = tid; a < natoms; a += T) {
+                const float3 f = make_float3((float)facc[3 * a] * (1.f / kFix), (float)facc[3 * a + 1] * (1.f / kFix),
+                                             (float)facc[3 * a + 2] * (1.f / kFix));
+                fnb[a] = make_float4(f.x, f.y, f.z, 0.f);
+                beyond |= fmaxf(fabsf(f.x), fmaxf(fabsf(f.y), fabsf(f.z))) > kPlainAbove;
+            }
+            beyond = __syncthreads_or(beyond) != 0;
+            if (beyond) plain_pairs(fnb, pbc, central);
             // without candidate lists: the other images of the bounding-box test,
             // ordered pairs (i, j + shift), S lanes per atom
             if (!lists && any_shift) {
@@ -119,7 +159,7 @@ struct Engine : PairEngine<T, S, ENERGY> {
                         fy += __shfl_xor_sync(0xffffffffu, fy, o);
                         fz += __shfl_xor_sync(0xffffffffu, fz, o);
                     }
-                    if (i < natoms && sub == 0) {
+                    if (i < natoms && sub == 0 && !beyond) {
                         const float4 a = fnb[i];
                         fnb[i] = make_float4(a.x + fx, a.y + fy, a.z + fz, 0.f);
                     }
