@@ -342,10 +342,10 @@ int group_size(Bucket& B, int dev_smem) {
     return 0;
 }
 
-// launch configuration of a bucket whose systems are set: T threads per system,
-// S lanes per atom on the image rows of the evaluation.  Fills layouts, sizes
-// and grid; sets kernel attributes.
-int config_bucket(Bucket& B, int T, int S) {
+// launch configuration of a bucket whose systems are set: T threads per system for
+// relaxations, eT for evaluations with S lanes per atom on the image rows.  Fills
+// layouts, sizes and grid; sets kernel attributes.
+int config_bucket(Bucket& B, int T, int eT, int S) {
     int dev_smem = 0;
     CK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, W.device));
     B.maxNA = 0; B.maxNN = 0;
@@ -376,13 +376,17 @@ int config_bucket(Bucket& B, int T, int S) {
     // evaluation: one pass over the system, a warp each up to 64 atoms
     B.eapl = B.maxNA <= 32 ? 1 : B.maxNA <= 64 ? 2 : 0;
     if (W.force_T) B.eapl = 0;
-    B.eT = B.eapl ? 128 : T;
+    B.eT = B.eapl ? 128 : eT;
     if (B.eapl && W.nsys <= W.nsm) {                      // too few for a warp each to hide anything: a block each
         B.eT = 256;
         B.S = B.eapl == 1 ? 8 : 4;
         B.eapl = 0;
     }
     if (!B.eapl) B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, 0);
+    if (!B.eapl && B.elay.total > dev_smem && B.eT < kCompactMinThreads) {
+        B.eT = kCompactMinThreads;
+        B.elay = smem_layout(B.maxNA, B.maxNN, B.eT, nimg, 0);
+    }
     B.esmem = B.eapl ? 4 * warp_layout(B.maxNA, B.maxNN).per_warp : B.elay.total;
     if (B.smem > dev_smem || B.esmem > dev_smem)
         return fail("system too large for shared memory: %d B > %d B", std::max(B.smem, B.esmem), dev_smem);
@@ -602,9 +606,10 @@ int build_buckets() {
         }
         int T, S;
         default_config(k, maxNA, (int)B.sys.size(), T, S);
+        // (a tuned class: the threads of its relaxations; evaluations keep their rule)
         const Tune& tu = W.tune[k];
-        if (tu.kind >= 0 && !W.force_T && !W.force_S) { T = tuned_threads(tu); S = tu.S; }
-        if (config_bucket(B, T, S)) { B.queue.release(); B.vl.release(); return -1; }
+        const int rT = tu.kind >= 0 && !W.force_T && !W.force_S ? tuned_threads(tu) : T;
+        if (config_bucket(B, rT, T, S)) { B.queue.release(); B.vl.release(); return -1; }
         B.cls = k;
         W.buckets.push_back(std::move(B));
     }
@@ -626,6 +631,27 @@ void set_lists(Params& P, const Bucket& B) {
     P.vskin = (float)W.list_skin;
 }
 
+// one bucket's relaxation kernel: a cluster per system, blocks of several systems, or
+// a block each; systems claimed through the queue by the counter ctr
+int launch_bucket(Bucket& B, Params& P, Systems& Y, int* ctr, bool count, cudaStream_t st) {
+    const int* q = B.queue.p;
+    int nq = (int)B.sys.size();
+    set_lists(P, B);
+    const bool plain = P.md_mode != 2 && !count;
+    const bool cluster = plain && B.cn > 1;
+    void* args[] = {&P, &Y, &q, &nq, &ctr, cluster ? &B.clay : &B.lay};
+    if (cluster) {
+        ClusterLaunch l(nq * B.cn, B.T, B.clay.total, B.cn, st);
+        CK(cudaLaunchKernelExC(&l.c, relax_cluster_fn(B.T), args));
+    } else if (plain && B.group > 1) {
+        CK(cudaLaunchKernel(relax_group_fn(B.T), dim3(B.ggrid), dim3(B.T * B.group), args, B.group * B.smem, st));
+    } else {
+        void* fn = P.md_mode == 2 ? relax_explore_fn(B.T) : relax_fn(B.T, count);
+        CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
+    }
+    return 0;
+}
+
 // the launches of one relax call on the library stream: reset the work
 // counters, fork to one stream per bucket, one persistent kernel per bucket
 // (systems claimed through the bucket's queue), join
@@ -638,22 +664,7 @@ int enqueue_relax(const Params& P) {
         Bucket& B = W.buckets[b];
         cudaStream_t st = W.bstreams[b];
         CK(cudaStreamWaitEvent(st, W.evfork, 0));
-        void* fn = P.md_mode == 2 ? relax_explore_fn(B.T) : relax_fn(B.T, W.count);
-        const int* q = B.queue.p;
-        int nq = (int)B.sys.size();
-        int* ctr = W.d_counter.p + b;
-        set_lists(Pc, B);
-        if (B.cn > 1 && P.md_mode != 2 && !W.count) {
-            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.clay};
-            ClusterLaunch l(nq * B.cn, B.T, B.clay.total, B.cn, st);
-            CK(cudaLaunchKernelExC(&l.c, relax_cluster_fn(B.T), args));
-        } else if (B.group > 1 && P.md_mode != 2 && !W.count) {
-            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
-            CK(cudaLaunchKernel(relax_group_fn(B.T), dim3(B.ggrid), dim3(B.T * B.group), args, B.group * B.smem, st));
-        } else {
-            void* args[] = {&Pc, &Y, &q, &nq, &ctr, &B.lay};
-            CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, st));
-        }
+        if (launch_bucket(B, Pc, Y, W.d_counter.p + b, W.count, st)) return -1;
         if (!g_capturing) g_launches++;
     }
     for (size_t b = 0; b < W.buckets.size(); b++) {
@@ -1385,7 +1396,8 @@ int mmff_set_graph(int on) {
 
 // ---------------------------------------------------------------- autotuner
 namespace {
-// threads per system tried for a size class, with the evaluation's lanes per atom
+// threads per system tried for a size class (S: pair lanes of the report and the files,
+// which evaluations do not use)
 struct Cand { int T, S; };
 std::vector<Cand> candidates(int cls) {
     switch (cls) {
@@ -1401,7 +1413,7 @@ std::vector<Cand> candidates(int cls) {
 
 // Time every candidate launch configuration of each size class present on a
 // sample of that class's systems (nstep_probe FIRE steps, no convergence
-// exit) and keep the fastest for later relax/eval calls.  Positions,
+// exit) and keep the fastest for later relaxations.  Positions,
 // velocities and FIRE state are restored afterwards.  report (nullable):
 // 6 floats per candidate tried (class, kind, atoms per lane, threads, pair
 // lanes, microseconds per system-step; negative: not launchable).
@@ -1445,19 +1457,14 @@ int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap
             Bucket B;
             B.sys = sample;
             float us = -1.f;
-            if (config_bucket(B, c.T, c.S) == 0) {
-                void* fn = relax_fn(B.T, false);
-                const int* q = B.queue.p;
-                int nq = (int)B.sys.size();
+            if (config_bucket(B, c.T, kCompactMinThreads, 1) == 0) {
                 int* ctr = W.d_counter.p + 32;
-                set_lists(P, B);
-                void* args[] = {&P, &Y, &q, &nq, &ctr, &B.lay};
                 float ms = 0.f;
                 for (int rep = 0; rep < 2; rep++) {        // first launch warms caches and clocks
                     if (copy_state(false)) return -1;
                     CK(cudaMemsetAsync(ctr, 0, sizeof(int), W.stream));
                     CK(cudaEventRecord(W.ev0, W.stream));
-                    CK(cudaLaunchKernel(fn, dim3(B.grid), dim3(B.T), args, B.smem, W.stream));
+                    if (launch_bucket(B, P, Y, ctr, false, W.stream)) return -1;      // as relaxations will
                     g_launches++;
                     CK(cudaEventRecord(W.ev1, W.stream));
                     CK(cudaEventSynchronize(W.ev1));
