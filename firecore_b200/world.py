@@ -95,7 +95,7 @@ class World:
         time per-system latency instead of throughput)."""
         rep = np.zeros((64, 6), np.float32)
         n = _check(self.lib.mmff_autotune(int(nstep_probe), int(max_sample), _lib.ptr(rep), 64), "mmff_autotune")
-        rows = [dict(size_class=int(r[0]), kind="warp" if r[1] == 1 else "cta", atoms_per_lane=int(r[2]),
+        rows = [dict(size_class=int(r[0]), kind="cta", atoms_per_lane=int(r[2]),
                      threads=int(r[3]), pair_lanes=int(r[4]), us_per_system_step=float(r[5])) for r in rep[:min(n, 64)]]
         if path:
             self.save_tuning(path, rows)

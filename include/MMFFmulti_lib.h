@@ -59,7 +59,8 @@ int mmff_set_fire(double dt_max, double dt_min, double damp_max, double finc, do
 /* Threads per CTA (64/128/256/512) and lanes per atom in the pair sum
  * (1/2/4/8) of the CTA-per-system kernels; 0 = chosen per size bucket
  * (evaluations of large batches then run systems of <= 64 atoms one per warp,
- * relaxations of a few large systems a cluster of CTAs per system).  A non-zero
+ * relaxations of a few large systems a cluster of CTAs per system, of many small
+ * ones several systems per CTA).  A non-zero
  * thread count forces one CTA per system; the lanes per atom apply to the
  * evaluation kernels. */
 int mmff_set_launch(int threads, int pair_split);
@@ -211,7 +212,8 @@ int mmff_get_explore(int* gopt, double* minpos);
 /* Autotuner (no counterpart in the reference, which uses one fixed work-group
  * size): for each size class present (0: <= 32 atoms, 1: <= 64, 3: <= 128,
  * 4: <= 256, 5: larger), time every candidate launch configuration (threads per
- * system) on up to
+ * system; in the form that relaxations run them: a CTA or a cluster per system,
+ * or several systems per CTA) on up to
  * max_sample of its systems for nstep_probe FIRE steps and keep the fastest.
  * State is restored.  report [6 per candidate] (nullable): class, kind,
  * atoms per lane, threads, pair lanes, us per system-step (< 0: not
@@ -219,7 +221,8 @@ int mmff_get_explore(int* gopt, double* minpos);
 int mmff_autotune(int nstep_probe, int max_sample, float* report, int report_cap);
 /* Tuned configuration of size class cls: out[4] = (kind: -1 heuristic, 0 CTA
  * per system, 1 (files of earlier versions) 32 x atoms-per-lane threads per
- * system; atoms per lane; threads; pair lanes of the evaluation). */
+ * system; atoms per lane; threads of relaxations; pair lanes, kept for the
+ * files' format).  Evaluations have a rule of their own. */
 int mmff_get_tuning(int cls, int* out);
 int mmff_set_tuning(int cls, int kind, int apl, int threads, int pair_split);
 

@@ -341,8 +341,8 @@ def test_position_springs_vs_oracle(world, golden):
 @pytest.mark.parametrize("threads", [0, 64])
 def test_bond_constraints_vs_oracle(world, golden, threads):
     """Distance / angle constraints (FireCore's Constrains, constrains.h) in both
-    relax engines (threads 0: the warp-per-system kernel for these 24-atom
-    systems; 64: the CTA kernel), with three atoms per system held by position
+    forms of the pair sums (threads 0: one warp's, for these 24-atom
+    systems; 64: tiles), with three atoms per system held by position
     springs so that every system converges: relaxed geometries match the FP64
     oracle with the same constraints (the oracle's are pinned to FireCore's
     run_no_omp in test_oracle_golden.py), and eval reports forces without them."""
